@@ -1,4 +1,4 @@
-// Prefill-side quantized-weight linear (M > 32 tokens): a dense contraction on the 5th-generation
+// Prefill-side quantized-weight linear: a dense contraction on the 5th-generation
 // tensor cores (tcgen05.mma, accumulators in TMEM).
 //
 // One CTA computes a tile of 128 or 256 output features x up to 256 tokens over the whole K range.

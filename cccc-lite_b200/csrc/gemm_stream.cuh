@@ -494,12 +494,15 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
 // ---- host side -----------------------------------------------------------------------------------------
 static inline bool sk_al16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-inline bool stream_supported(int w_type, const void* blk, unsigned int N, unsigned int M, unsigned int K, unsigned int ldw, unsigned int ldx)
+// What the streaming kernels ask of a linear besides its token count.
+inline bool stream_layout(int w_type, const void* blk, unsigned int N, unsigned int M, unsigned int K, unsigned int ldw, unsigned int ldx)
 {
-    if (M == 0 || M > 128 || N == 0 || K == 0 || (K % SK_SLICE_ELEMS) != 0 || (ldx % 8) != 0) { return false; }
+    if (M == 0 || N == 0 || K == 0 || (K % SK_SLICE_ELEMS) != 0 || (ldx % 8) != 0) { return false; }
     if (w_type == DT_FP4) { return blk != nullptr && sk_al16(blk) && (ldw % 256) == 0; }    // 16-byte rows of scales
     return (ldw % 16) == 0;
 }
+
+constexpr unsigned int kStreamNarrowTokens = 128;    // accumulator columns of this kernel; more tokens: gemm_stream_wide.cuh
 
 // k slices per tile: the largest power of two (clusters of 3, 5, 6 or 7 CTAs did not all become resident together
 // and ran as two waves) that keeps all CTAs within ONE wave of two per SM, with a margin for SMs whose cluster
@@ -595,11 +598,11 @@ static int launch_stream_t(const void* X, unsigned int ldx, StreamParams& sp, in
     return launch_stream_bn<WT, SCALED, 128>(X, ldx, sp, feature_tiles, device, stream, pdl);
 }
 
-// One launch for up to PF_MAX_GROUP linears that share X; items as for launch_prefill.  -2: not taken.
-static int launch_stream(int w_type, const GemvParams* items, unsigned int count, int device, int sm_count, cudaStream_t stream, bool pdl)
+// The launch parameters of up to PF_MAX_GROUP linears that share X; items as for launch_prefill.  False: not taken.
+static bool stream_params(int w_type, const GemvParams* items, unsigned int count, StreamParams* out, bool* scaled_out)
 {
-    if (count == 0 || count > (unsigned)PF_MAX_GROUP) { return -2; }
-    StreamParams sp;
+    if (count == 0 || count > (unsigned)PF_MAX_GROUP) { return false; }
+    StreamParams& sp = *out;
     memset(&sp, 0, sizeof(sp));
     sp.n_seg = count;
     sp.status = items[0].status;
@@ -609,11 +612,11 @@ static int launch_stream(int w_type, const GemvParams* items, unsigned int count
     bool all_pow2 = true;
     for (unsigned int j = 0; j < count; j++)
     {
-        if (!stream_supported(w_type, items[j].blk, items[j].N, items[j].M, items[j].K, items[j].ldw, items[j].ldx)) { return -2; }
-        if (!sk_al16(items[j].W)) { return -2; }
+        if (!stream_layout(w_type, items[j].blk, items[j].N, items[j].M, items[j].K, items[j].ldw, items[j].ldx)) { return false; }
+        if (!sk_al16(items[j].W)) { return false; }
         all_pow2 = all_pow2 && pf_is_pow2_scale(items[j].w_scale);
     }
-    if (!sk_al16(items[0].X)) { return -2; }
+    if (!sk_al16(items[0].X)) { return false; }
     const bool scaled = w_type != DT_FP4 && !all_pow2;
     for (unsigned int j = 0; j < count; j++)
     {
@@ -630,6 +633,16 @@ static int launch_stream(int w_type, const GemvParams* items, unsigned int count
         g.w_scale = scaled ? items[j].w_scale : 1.0f;
         g.post_scale = (w_type == DT_FP4 || scaled) ? 1.0f : items[j].w_scale;
     }
+    *scaled_out = scaled;
+    return true;
+}
+
+// One launch for up to PF_MAX_GROUP linears that share X (up to kStreamNarrowTokens tokens).  -2: not taken.
+static int launch_stream(int w_type, const GemvParams* items, unsigned int count, int device, int sm_count, cudaStream_t stream, bool pdl)
+{
+    StreamParams sp;
+    bool scaled = false;
+    if (count == 0 || items[0].M > kStreamNarrowTokens || !stream_params(w_type, items, count, &sp, &scaled)) { return -2; }
     const void* X = items[0].X;
     const unsigned int ldx = items[0].ldx;
     if (w_type == DT_FP4) { return launch_stream_t<DT_FP4, false>(X, ldx, sp, device, sm_count, stream, pdl); }

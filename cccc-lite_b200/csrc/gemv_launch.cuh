@@ -8,6 +8,7 @@
 #include "tensor_map.cuh"
 #include "prefill_launch.cuh"
 #include "gemm_stream.cuh"
+#include "gemm_stream_wide.cuh"
 #include "gemm_native.cuh"
 #include "gemm_native_fp4.cuh"
 
@@ -281,13 +282,29 @@ static int plan_for(int w_type, const void* W, const void* blk, const void* X, c
 {
     (void)Y;
     const int base = plan_base(w_type, W, blk, X, N, M, K, ldw, ldx, ldy_m, ldy_n);
-    if (base != PLAN_PLAIN && M >= kStreamMinTokens && M <= kStreamMaxTokens && stream_supported(w_type, blk, N, M, K, ldw, ldx))
+    if (base != PLAN_PLAIN && M >= kStreamMinTokens && M <= kStreamMaxTokens && stream_layout(w_type, blk, N, M, K, ldw, ldx))
     {
         return PLAN_STREAM;
     }
     return base;
 }
 
+
+// More than kStreamNarrowTokens tokens: the wide streaming kernel, or the prefill kernel?  flags bits 8-10 = 7 take the former
+// wherever it accepts the shape, a tile shape or bit 11 the latter.
+static bool want_wide(unsigned int flags, int w_type, const GemvParams* items, unsigned int count, int device, int sm_count)
+{
+    const unsigned int variant = (flags >> 8) & 7u;
+    if (items[0].M <= kStreamNarrowTokens || (flags & kFlagNoStream) != 0 || (variant != 0 && variant != kVariantStream)) { return false; }
+    unsigned int pair_tiles = 0, n_total = 0;
+    for (unsigned int j = 0; j < count; j++)
+    {
+        if (!stream_layout(w_type, items[j].blk, items[j].N, items[j].M, items[j].K, items[j].ldw, items[j].ldx)) { return false; }
+        pair_tiles += (items[j].N + 2 * SK_BM - 1) / (2 * SK_BM);
+        n_total += items[j].N;
+    }
+    return variant == kVariantStream || sw_preferred(pair_tiles, n_total, items[0].M, items[0].K, device, sm_count);
+}
 
 // The whole entry: argument checks done by the caller; picks the kernel and launches it on
 // `st`.  Returns the C-ABI code (0 ok, 1 CUDA error, -1 bad argument).
@@ -370,6 +387,11 @@ static int run_linear_wq(const GemvScratch* ws, int w_type, const void* W, const
     }
     if (plan == PLAN_PREFILL)
     {
+        if (!decode_only && want_wide(flags, w_type, &p, 1, ws->device, ws->sm_count))
+        {
+            const int r = launch_stream_wide(w_type, &p, 1, ws->device, st, pdl);
+            if (r != -2) { return r; }
+        }
         const int r = launch_prefill(w_type, &p, 1, ws->device, ws->sm_count, (int)((flags >> 8) & 7u), st);
         if (r != -2) { return r; }
         plan = PLAN_PLAIN;
@@ -565,6 +587,11 @@ static int run_linear_wq_group(const GemvScratch* ws, int w_type, unsigned int c
             q.alpha = items[j].alpha;
             q.beta = items[j].beta;
             q.out_f32 = (flags & 4u) ? 1u : ((flags & 8u) ? 2u : 0u);
+        }
+        if (want_wide(flags, w_type, ps, count, ws->device, ws->sm_count))
+        {
+            const int w = launch_stream_wide(w_type, ps, count, ws->device, st, (flags & 1u) != 0);
+            if (w != -2) { return w; }
         }
         const int r = launch_prefill(w_type, ps, count, ws->device, ws->sm_count, (int)((flags >> 8) & 7u), st);
         if (r != -2) { return r; }

@@ -30,7 +30,8 @@ enum PrefillVariant : int
 // (each weight is converted once per 512 tokens, each CTA stages half of the activations, five and
 // four stages deep); with fewer tiles the 256 x 256 pair tile (two CTAs per SM) wins, and when even
 // that leaves most SMs idle the 128 x 128 one-CTA tile gives the most CTAs.  The k loop of a CTA
-// costs about 0.55 us per 64-wide k block whatever the tile, so small problems are bound by K alone.
+// costs about 0.55 us per 64-wide k block whatever the tile, so small problems are bound by K alone.  (Where K is a whole number
+// of 256 the dispatcher comes here for the 512-token pair tile only; everything else goes to gemm_stream_wide.cuh.)
 static int pf_pick_variant(int w_type, unsigned int N, unsigned int M, unsigned int K, int sm_count)
 {
     (void)w_type;

@@ -81,11 +81,12 @@ C_EXPORT void cuda_clear_last_error(void);
  * is added: Y = bf16( bf16(alpha * W x) + beta * Y ), which with beta = 1 is the reference's linear
  * followed by its residual add (two BF16 tensors, scripts/convert_weights.py:562, :582).
  * bits 8-10 = kernel choice for tests and tuning (0 = chosen by shape: the decode kernel up to 8 tokens,
- * the streaming tensor-core kernel from 9 to 128 tokens where K % 256 == 0, the prefill kernel above;
+ * the streaming tensor-core kernel from 9 to 128 tokens where K % 256 == 0, above that its wide form on CTA pairs or
+ * the prefill kernel, whichever is estimated the faster;
  * 1-3 = the prefill kernel with one CTA per tile: 128 features x 128 tokens, 128 x 256, 256 x 256;
  * 4-6 = with CTA pairs: 256 x 256, 512 features x 256 tokens, 256 x 512 - the six tile shapes give the same
- * result bit for bit; 7 = the streaming kernel wherever it accepts the shape, i.e. from 1 token).
- * bit 11 = never the streaming kernel (the decode kernel up to 32 tokens, the prefill kernel above).
+ * result bit for bit; 7 = the streaming kernel, above 128 tokens its wide form, wherever it accepts the shape).
+ * bit 11 = never the streaming kernels (the decode kernel up to 32 tokens, the prefill kernel above).
  * bit 12 = the native-operand kernel wherever it accepts the shape (FP8 up to 32 tokens with a power-of-two
  * inv_scale and K % 128 == 0; FP4 up to 32 tokens with K % 256 == 0): the quantised weights go from HBM through
  * shared memory into tcgen05.mma (kind::f8f6f4, kind::mxf4nvf4 with the block scales) unchanged, the BF16
