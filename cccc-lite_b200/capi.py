@@ -91,6 +91,7 @@ SYMBOLS["cuda_rope_bf16"] = (_i, [_vp, _vp, _vp, _vp, _u, _u, _u, _u, _vp, _u])
 SYMBOLS["cuda_embed_bf16"] = (_i, [_vp, _vp, _vp, _u, _u, _u, _vp, _u])
 SYMBOLS["cuda_swiglu_bf16"] = (_i, [_vp, _vp, _vp, _u, _u, _u, _u, _u, _vp, _u])
 SYMBOLS["cuda_attn_decode_bf16"] = (_i, [C.POINTER(AttnDecode), _vp, _u])
+SYMBOLS["cuda_attn_append_bf16"] = (_i, [C.POINTER(AttnDecode), _vp, _u])
 
 
 
@@ -370,6 +371,11 @@ def make_attn_decode(*, q, k, v, k_cache, v_cache, pos, out, cos_tab, sin_tab, B
 
 def attn_decode_bf16(desc, stream=None, flags: int = 0) -> int:
     return lib().cuda_attn_decode_bf16(C.byref(desc), _stream(stream), flags)
+
+
+def attn_append_bf16(desc, stream=None, flags: int = 0) -> int:
+    """Norm and rotation of q (into desc.out) and k, k and v appended, for any number of tokens."""
+    return lib().cuda_attn_append_bf16(C.byref(desc), _stream(stream), flags)
 
 
 class DecodeProgram:

@@ -171,6 +171,71 @@ __global__ void __launch_bounds__(kTeam, (G <= 4 ? 2 : 1)) attn_decode_kernel(co
     cluster.sync();    // the other splits keep their shared memory alive until split 0 has read it
 }
 
+// ---- q/k norm, RoPE and cache append of many tokens ----------------------------------------------------
+// One warp per (token, head); heads 0 .. H-1 are queries, then Hkv keys, then Hkv values.  Lane l holds the elements l, l + 32,
+// ..: a rotation's two elements meet in one lane, and the squares are added in the order of team_sum_squares, so that a row
+// has the bits that the decode kernel's prologue gives it.  Bound by HBM: a prompt's projections are read once, its queries and
+// cache rows written once.
+template <int HD>
+__global__ void __launch_bounds__(256) attn_append_kernel(const AttnDecodeParams p)
+{
+    constexpr int N = HD / 32, HALF = N / 2;
+    const unsigned int lane = threadIdx.x & 31u, head = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const unsigned int b = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (head >= p.H + 2 * p.Hkv) { return; }
+    const int pos_i = p.pos[b];
+    const unsigned int pos = pos_i < 0 ? 0u : (unsigned int)pos_i;
+    const bool is_q = head < p.H, is_v = head >= p.H + p.Hkv;
+    const unsigned int kvh = is_v ? head - p.H - p.Hkv : head - p.H;
+    const uint16_t* src = is_q ? p.q + (size_t)b * p.ldq + (size_t)head * HD : (is_v ? p.v + (size_t)b * p.ldv : p.k + (size_t)b * p.ldk) + (size_t)kvh * HD;
+    uint16_t* dst;
+    if (is_q) { dst = p.out + (size_t)b * p.ldo + (size_t)head * HD; }
+    else
+    {
+        if (pos >= p.T_max) { return; }
+        dst = (is_v ? p.v_cache : p.k_cache) + (attn_cache_row(p, b, kvh) + pos) * HD;
+    }
+    if (is_v)
+    {
+#pragma unroll
+        for (int i = 0; i < N; i++) { dst[lane + 32 * i] = src[lane + 32 * i]; }
+        return;
+    }
+    float x[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) { x[i] = bf16_bits_to_float(src[lane + 32 * i]); }
+    const uint16_t* w = is_q ? p.q_norm : p.k_norm;
+    if (w != nullptr)
+    {
+        float sq[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) { sq[i] = __fmul_rn(x[i], x[i]); }
+#pragma unroll
+        for (int h = N / 2; h > 0; h >>= 1)
+        {
+#pragma unroll
+            for (int i = 0; i < h; i++) { sq[i] += sq[i + h]; }
+        }
+        float sum = sq[0];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) { sum += __shfl_down_sync(0xFFFFFFFFu, sum, o); }
+        const float invstd = rms_invstd(__shfl_sync(0xFFFFFFFFu, sum, 0), HD, p.eps);
+#pragma unroll
+        for (int i = 0; i < N; i++) { x[i] = rms_apply(x[i], invstd, bf16_bits_to_float(w[lane + 32 * i])); }
+    }
+    const uint16_t *c = p.cos_tab + (size_t)pos * (HD / 2), *s = p.sin_tab + (size_t)pos * (HD / 2);
+#pragma unroll
+    for (int i = 0; i < HALF; i++)
+    {
+        float yl, yr;
+        rope_pair(x[i], x[i + HALF], bf16_bits_to_float(c[lane + 32 * i]), bf16_bits_to_float(s[lane + 32 * i]), yl, yr);
+        dst[lane + 32 * i] = bf16_bits(yl);
+        dst[lane + 32 * (i + HALF)] = bf16_bits(yr);
+    }
+}
+
 static unsigned int attn_ts_cap(unsigned int T_max, unsigned int S) { return (((T_max + S - 1) / S) + 31u) & ~31u; }
 
 template <int G, int HD>
@@ -343,12 +408,11 @@ C_EXPORT int cuda_swiglu_bf16(const void* gate, const void* up, void* out, unsig
         (const uint16_t*)gate, (const uint16_t*)up, (uint16_t*)out, cols, ld_gate, ld_up, ld_out);
 }
 
-C_EXPORT int cuda_attn_decode_bf16(const cuda_attn_decode* a, void* stream, unsigned int flags)
+// The descriptor's checks and its kernel form.  0: ok, p is filled.
+static int attn_params(const cuda_attn_decode* a, AttnDecodeParams* out)
 {
-    if (!a) { return -1; }
-    if (a->B == 0 || a->H == 0) { return 0; }
     if (!a->q || !a->k || !a->v || !a->cos_tab || !a->sin_tab || !a->k_cache || !a->v_cache || !a->pos || !a->out) { return -1; }
-    if (a->Hkv == 0 || (a->H % a->Hkv) != 0 || a->T_max == 0 || a->B > 65535u || a->Hkv > 65535u) { return -1; }
+    if (a->Hkv == 0 || (a->H % a->Hkv) != 0 || a->T_max == 0 || a->Hkv > 65535u) { return -1; }
     auto misaligned = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) != 0; };
     if ((a->ldq % 8) != 0 || (a->ldk % 8) != 0 || (a->ldv % 8) != 0 || misaligned(a->q) || misaligned(a->k) || misaligned(a->v)
         || misaligned(a->k_cache) || misaligned(a->v_cache) || misaligned(a->cos_tab) || misaligned(a->sin_tab)
@@ -356,9 +420,7 @@ C_EXPORT int cuda_attn_decode_bf16(const cuda_attn_decode* a, void* stream, unsi
     {
         return -1;
     }
-    const DeviceFacts* f = device_facts();
-    if (!f) { return 1; }
-    AttnDecodeParams p;
+    AttnDecodeParams& p = *out;
     p.q = (const uint16_t*)a->q;
     p.k = (const uint16_t*)a->k;
     p.v = (const uint16_t*)a->v;
@@ -381,6 +443,33 @@ C_EXPORT int cuda_attn_decode_bf16(const cuda_attn_decode* a, void* stream, unsi
     p.T_max = a->T_max;
     p.eps = a->epsilon;
     p.scale = 1.0f / sqrtf(a->dk > 0.f ? a->dk : (float)a->head_dim);
+    return 0;
+}
+
+C_EXPORT int cuda_attn_append_bf16(const cuda_attn_decode* a, void* stream, unsigned int flags)
+{
+    if (!a) { return -1; }
+    if (a->B == 0 || a->H == 0) { return 0; }
+    AttnDecodeParams p;
+    const int rc = attn_params(a, &p);
+    if (rc != 0) { return rc; }
+    const dim3 grid(a->B, (a->H + 2 * a->Hkv + 7) / 8);
+    if (grid.y > 65535u) { return -1; }
+    const bool pdl = (flags & 1u) != 0;
+    if (a->head_dim == 128) { return launch_simple("attn_append_bf16", attn_append_kernel<128>, grid, dim3(256), 0, (cudaStream_t)stream, pdl, p); }
+    if (a->head_dim == 64) { return launch_simple("attn_append_bf16", attn_append_kernel<64>, grid, dim3(256), 0, (cudaStream_t)stream, pdl, p); }
+    return -1;
+}
+
+C_EXPORT int cuda_attn_decode_bf16(const cuda_attn_decode* a, void* stream, unsigned int flags)
+{
+    if (!a) { return -1; }
+    if (a->B == 0 || a->H == 0) { return 0; }
+    AttnDecodeParams p;
+    const int rc = attn_params(a, &p);
+    if (rc != 0 || a->B > 65535u) { return -1; }
+    const DeviceFacts* f = device_facts();
+    if (!f) { return 1; }
     const unsigned int G = a->H / a->Hkv;
     const bool pdl = (flags & 1u) != 0;
     cudaStream_t st = (cudaStream_t)stream;

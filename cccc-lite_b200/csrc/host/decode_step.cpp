@@ -1,5 +1,6 @@
 #include "decode_step.h"
 
+#include "../../../include/cccc_b200_decoder.h"
 #include "../../../include/cccc_cuda_b200.h"
 
 #include <algorithm>
@@ -220,6 +221,7 @@ DecodeStep::~DecodeStep()
     for (void* p : owned_) { gpu_->free(p); }
     if (h_ids_) { cudaFreeHost(h_ids_); }
     if (h_logits_) { cudaFreeHost(h_logits_); }
+    if (h_meta_) { cudaFreeHost(h_meta_); }
 }
 
 void* DecodeStep::dmalloc(size_t bytes)
@@ -485,6 +487,34 @@ bool DecodeStep::loadTensors(const BinFile& file, std::string* err)
 
 void DecodeStep::resetCache() { cache_.clear(); }
 
+// A linear of a group: features from `out` on, rows of `ld` elements.
+static cuda_wq_linear member(const void* w, const void* s, float inv, int n, uint16_t* out, int k, int ld)
+{
+    cuda_wq_linear g = {};
+    g.W = w;
+    g.blk_scales = s;
+    g.Y = out;
+    g.inv_scale = inv;
+    g.alpha = 1.0f;
+    g.N_out = (unsigned int)n;
+    g.ldw = (unsigned int)k;
+    g.ldy_m = (unsigned int)ld;
+    g.ldy_n = 1;
+    return g;
+}
+
+void DecodeStep::groupQkv(const Layer& L, uint16_t* out, cuda_wq_linear* g) const
+{
+    const Linear* l[3] = { &L.q, &L.k, &L.v };
+    for (int j = 0; j < 3; out += l[j]->n, j++) { g[j] = member(l[j]->w, l[j]->s, l[j]->inv, l[j]->n, out, cfg_.hidden, qkv_ld_); }
+}
+
+void DecodeStep::groupGateUp(const Layer& L, uint16_t* out, cuda_wq_linear* g) const
+{
+    g[0] = member(L.gate.w, L.gate.s, L.gate.inv, ffn_loc_, out, cfg_.hidden, 2 * ffn_loc_);
+    g[1] = member(L.up.w, L.up.s, L.up.inv, ffn_loc_, out + ffn_loc_, cfg_.hidden, 2 * ffn_loc_);
+}
+
 int DecodeStep::issue(int M, cudaStream_t st)
 {
     const unsigned int PDL = 1u, RES = 8u;
@@ -513,43 +543,15 @@ int DecodeStep::issue(int M, cudaStream_t st)
     {
         const Layer& L = layers_[i];
         norm(L.attn_norm, pending);
-        cuda_wq_linear g[3] = {};
-        const Linear* qkv[3] = { &L.q, &L.k, &L.v };
-        unsigned int off = 0;
-        for (int j = 0; j < 3; j++)
-        {
-            g[j].W = qkv[j]->w;
-            g[j].blk_scales = qkv[j]->s;
-            g[j].Y = qkv_ + off;
-            g[j].inv_scale = qkv[j]->inv;
-            g[j].alpha = 1.0f;
-            g[j].beta = 0.0f;
-            g[j].N_out = qkv[j]->n;
-            g[j].ldw = hid;
-            g[j].ldy_m = qkv_ld_;
-            g[j].ldy_n = 1;
-            off += qkv[j]->n;
-        }
+        cuda_wq_linear g[3];
+        groupQkv(L, qkv_, g);
         ok(cuda_gemm_wq_bf16_group(wt, 3, g, xn_, M, hid, hid, st, PDL));
         cuda_attn_decode a = attnArgs(i, M);
         ok(cuda_attn_decode_bf16(&a, st, PDL));
         row_linear(L.o, att_);
         norm(L.ffn_norm, tp);
-        cuda_wq_linear u[2] = {};
-        const Linear* gu[2] = { &L.gate, &L.up };
-        for (int j = 0; j < 2; j++)
-        {
-            u[j].W = gu[j]->w;
-            u[j].blk_scales = gu[j]->s;
-            u[j].Y = gu_ + (size_t)j * ffn_loc_;
-            u[j].inv_scale = gu[j]->inv;
-            u[j].alpha = 1.0f;
-            u[j].beta = 0.0f;
-            u[j].N_out = ffn_loc_;
-            u[j].ldw = hid;
-            u[j].ldy_m = 2 * ffn_loc_;
-            u[j].ldy_n = 1;
-        }
+        cuda_wq_linear u[2];
+        groupGateUp(L, gu_, u);
         ok(cuda_gemm_wq_bf16_group(wt, 2, u, xn_, M, hid, hid, st, PDL));
         ok(cuda_swiglu_bf16(gu_, gu_ + ffn_loc_, h_, M, ffn_loc_, 2 * ffn_loc_, 2 * ffn_loc_, ffn_loc_, st, PDL));
         row_linear(L.down, h_);
@@ -587,6 +589,157 @@ cuda_attn_decode DecodeStep::attnArgs(size_t layer, int M) const
     a.epsilon = cfg_.eps;
     a.dk = 0.f;
     return a;
+}
+
+bool DecodeStep::reservePrompts(int tokens)
+{
+    prompt_cap_ = 0;
+    if (world_ != 1 || tokens <= 0 || (cfg_.head_dim != 64 && cfg_.head_dim != 128)) { return false; }
+    gpu_->setAsCurrent();
+    const size_t T = (size_t)tokens, meta = (size_t)(4 * tokens + 4 * max_batch_) * 4, work = cuda_b200_attention_work_bytes((unsigned int)cfg_.head_dim);
+    const size_t owned = owned_.size();
+    px_ = (uint16_t*)dmalloc(T * cfg_.hidden * 2);
+    pxn_ = (uint16_t*)dmalloc(T * cfg_.hidden * 2);
+    pqkv_ = (uint16_t*)dmalloc(T * qkv_ld_ * 2);
+    patt_ = (uint16_t*)dmalloc(T * q_loc_ * 2);
+    pgu_ = (uint16_t*)dmalloc(T * 2 * ffn_loc_ * 2);
+    ph_ = (uint16_t*)dmalloc(T * ffn_loc_ * 2);
+    d_meta_ = (int*)dmalloc(meta);
+    attn_work_ = dmalloc(work);
+    const bool all = px_ && pxn_ && pqkv_ && patt_ && pgu_ && ph_ && d_meta_ && attn_work_;
+    if (!all || (!h_meta_ && cudaMallocHost((void**)&h_meta_, meta) != cudaSuccess) || cudaMemset(attn_work_, 0, work) != cudaSuccess)
+    {
+        cudaGetLastError();    // no room: what was taken goes back, prompts go through the decode step
+        while (owned_.size() > owned)
+        {
+            gpu_->free(owned_.back());
+            owned_.pop_back();
+        }
+        return false;
+    }
+    cudaDeviceSynchronize();
+    prompt_cap_ = tokens;
+    return true;
+}
+
+int DecodeStep::prompt(const std::vector<PromptEntry>& entries, const std::vector<int>& want, int* next_ids, uint16_t* logits)
+{
+    const unsigned int PDL = 1u, RES = 8u;
+    int tokens = 0, max_n = 0, max_len = 0;
+    for (const auto& e : entries)
+    {
+        tokens += e.n;
+        max_n = std::max(max_n, e.n);
+        max_len = std::max(max_len, e.pos + e.n);
+    }
+    if (tokens == 0) { return 0; }
+    if (tokens > prompt_cap_ || (int)entries.size() > max_batch_ || (int)want.size() > tokens) { return -1; }
+    gpu_->setAsCurrent();
+    cudaStream_t st = gpu_->stream();
+    // per token: id, position, slot, entry; per entry: slot, position, first token, tokens
+    const int C = prompt_cap_, B = max_batch_;
+    int *ids = h_meta_, *pos = ids + C, *slot = pos + C, *owner = slot + C, *e_slot = owner + C, *e_pos = e_slot + B, *e_start = e_pos + B, *e_n = e_start + B;
+    int at = 0;
+    for (size_t e = 0; e < entries.size(); e++)
+    {
+        const PromptEntry& E = entries[e];
+        e_slot[e] = E.slot;
+        e_pos[e] = E.pos;
+        e_start[e] = at;
+        e_n[e] = E.n;
+        for (int i = 0; i < E.n; i++, at++)
+        {
+            ids[at] = E.tokens[i];
+            pos[at] = E.pos + i;
+            slot[at] = E.slot;
+            owner[at] = (int)e;
+        }
+    }
+    if (cudaMemcpyAsync(d_meta_, h_meta_, (size_t)(4 * C + 4 * B) * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) { return 1; }
+    auto dev = [&](const int* host) { return d_meta_ + (host - h_meta_); };
+    cuda_b200_batch batch = {};
+    batch.slot = dev(e_slot);
+    batch.pos = dev(e_pos);
+    batch.start = dev(e_start);
+    batch.n = dev(e_n);
+    batch.token_entry = dev(owner);
+    batch.entries = (unsigned int)entries.size();
+    batch.tokens = (unsigned int)tokens;
+    batch.max_n = (unsigned int)max_n;
+    batch.max_len = (unsigned int)max_len;
+    const int wt = (int)wt_;
+    const unsigned int hid = (unsigned int)cfg_.hidden, M = (unsigned int)tokens;
+    int n = 0, bad = 0;
+    auto ok = [&](int rc) {
+        if (rc != 0) { bad++; }
+        n++;
+    };
+    auto row_linear = [&](const Linear& L, const uint16_t* src) {
+        ok(cuda_gemm_wq_bf16(wt, L.w, L.s, L.inv, src, px_, hid, M, L.k, L.k, L.k, hid, 1, 1.0f, 1.0f, st, PDL | RES));
+    };
+    ok(cuda_embed_bf16(dev(ids), emb_, px_, hid, M, cfg_.vocab, st, 0));
+    for (size_t i = 0; i < layers_.size(); i++)
+    {
+        const Layer& L = layers_[i];
+        ok(cuda_rms_norm_bf16(px_, nullptr, nullptr, pxn_, L.attn_norm, M, hid, cfg_.eps, st, PDL));
+        cuda_wq_linear g[3];
+        groupQkv(L, pqkv_, g);
+        ok(cuda_gemm_wq_bf16_group(wt, 3, g, pxn_, M, hid, hid, st, PDL));
+        cuda_attn_decode a = attnArgs(i, tokens);
+        a.q = pqkv_;
+        a.k = pqkv_ + q_loc_;
+        a.v = pqkv_ + q_loc_ + kv_loc_;
+        a.out = pqkv_;
+        a.ldo = (unsigned int)qkv_ld_;
+        a.pos = dev(pos);
+        a.slot = dev(slot);
+        ok(cuda_attn_append_bf16(&a, st, PDL));
+        cuda_b200_attention t = {};
+        t.qkvg = pqkv_;
+        t.out = patt_;
+        t.k_cache = cache_.k((int)i);
+        t.v_cache = cache_.v((int)i);
+        t.work = attn_work_;
+        t.ld = (unsigned int)qkv_ld_;
+        t.ldo = (unsigned int)q_loc_;
+        t.H = (unsigned int)H_;
+        t.Hkv = (unsigned int)Hkv_;
+        t.dim = t.vdim = (unsigned int)cfg_.head_dim;
+        t.k_ld = (unsigned int)cache_.kLd((int)i);
+        t.v_ld = (unsigned int)cache_.vLd((int)i);
+        t.T_max = (unsigned int)cache_.rows();
+        t.slots = (unsigned int)cache_.slots();
+        t.no_append = 1;
+        t.scale = 1.0f / std::sqrt((float)cfg_.head_dim);
+        ok(cuda_b200_attention_rows((int)BFLOAT16, &t, &batch, st, PDL, 0));
+        row_linear(L.o, patt_);
+        ok(cuda_rms_norm_bf16(px_, nullptr, nullptr, pxn_, L.ffn_norm, M, hid, cfg_.eps, st, PDL));
+        cuda_wq_linear u[2];
+        groupGateUp(L, pgu_, u);
+        ok(cuda_gemm_wq_bf16_group(wt, 2, u, pxn_, M, hid, hid, st, PDL));
+        ok(cuda_swiglu_bf16(pgu_, pgu_ + ffn_loc_, ph_, M, ffn_loc_, 2 * ffn_loc_, 2 * ffn_loc_, ffn_loc_, st, PDL));
+        row_linear(L.down, ph_);
+    }
+    // the wanted rows, a decode batch at a time: gathered, normalised, through the head
+    for (size_t w0 = 0; w0 < want.size() && !bad; w0 += (size_t)max_batch_)
+    {
+        const int rows = (int)std::min((size_t)max_batch_, want.size() - w0);
+        for (int i = 0; i < rows; i++) { h_ids_[i] = want[w0 + i]; }
+        cudaMemcpyAsync(d_ids_, h_ids_, (size_t)rows * 4, cudaMemcpyHostToDevice, st);
+        ok(cuda_embed_bf16(d_ids_, px_, x_, hid, rows, M, st, 0));
+        ok(cuda_rms_norm_bf16(x_, nullptr, nullptr, xn_, final_norm_, rows, hid, cfg_.eps, st, PDL));
+        ok(cuda_gemm_wq_bf16(wt, lm_head_.w, lm_head_.s, lm_head_.inv, xn_, logits_, vocab_loc_, rows, hid, hid, hid, vocab_loc_, 1, 1.0f, 0.0f, st, PDL));
+        ok(cuda_argmax_bf16(logits_, rows, vocab_loc_, vocab_loc_, d_ids_, d_best_, st));
+        cudaMemcpyAsync(h_out_, d_ids_, (size_t)rows * 4, cudaMemcpyDeviceToHost, st);
+        if (logits) { cudaMemcpyAsync(h_logits_, logits_, (size_t)rows * vocab_loc_ * 2, cudaMemcpyDeviceToHost, st); }
+        if (cudaStreamSynchronize(st) != cudaSuccess) { return 1; }
+        if (logits) { std::memcpy(logits + w0 * vocab_loc_, h_logits_, (size_t)rows * vocab_loc_ * 2); }
+        for (int i = 0; i < rows && next_ids; i++) { next_ids[w0 + i] = h_out_[i]; }
+    }
+    last_launches_ = n;
+    if (cudaStreamSynchronize(st) != cudaSuccess) { return 1; }    // the pinned arrays are reused by the next pass
+    if (cuda_check_error("prompt") != 0 || cuda_b200_decoder_check("prompt") != 0) { return 1; }
+    return bad ? 1 : 0;
 }
 
 bool DecodeStep::buildProgram()

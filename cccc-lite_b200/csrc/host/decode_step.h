@@ -92,6 +92,20 @@ public:
     // rank); logits_host (nullable) receives this rank's shard of the BF16 logits, [M][vocab / world].
     // slots (nullable): the cache slot of each sequence; without it sequence i has slot i.
     int step(const int* token_ids, const int* positions, int M, int* next_ids, float* best_logits, uint16_t* logits_host, const int* slots = nullptr);
+    // New tokens of one sequence, which continue row `pos` of cache slot `slot`.
+    struct PromptEntry
+    {
+        int slot, pos, n;
+        const int* tokens;
+    };
+    // Room for passes of up to `tokens` prompt tokens (one GPU).  False: not taken or no memory; step() then serves prompts
+    // token by token.
+    bool reservePrompts(int tokens);
+    int promptTokens() const { return prompt_cap_; }
+    // All tokens of the entries (at most promptTokens() together) at once: linears over all rows, causal attention over the
+    // caches.  want: flat indexes of tokens whose arg-max (next_ids, nullable) and BF16 logits (logits, nullable,
+    // [want][vocab]) are asked for.
+    int prompt(const std::vector<PromptEntry>& entries, const std::vector<int>& want, int* next_ids, uint16_t* logits);
     KvCache& cache() { return cache_; }
     void resetCache();
     // One sequence, one GPU: run steps through the recorded decode program (one persistent kernel) when it takes the model.
@@ -133,6 +147,8 @@ private:
     bool loadLinear(const BinFile& f, const std::string& name, int N, int K, char kind, Linear* out, std::string* err);
     bool loadBf16(const BinFile& f, const std::string& name, size_t n, uint16_t** out, bool required, std::string* err);
     int issue(int M, cudaStream_t st);
+    void groupQkv(const Layer& L, uint16_t* out, cuda_wq_linear* g) const;
+    void groupGateUp(const Layer& L, uint16_t* out, cuda_wq_linear* g) const;
     cuda_attn_decode attnArgs(size_t layer, int M) const;
     bool buildProgram();
     void* dmalloc(size_t bytes);
@@ -162,6 +178,11 @@ private:
     bool use_program_ = false;
     size_t weight_bytes_ = 0;
     int launches_per_step_ = 0;
+    // prompts: activations of a pass, its index arrays (pinned and on the device, one block), scratch of the attention
+    int prompt_cap_ = 0;
+    uint16_t *px_ = nullptr, *pxn_ = nullptr, *pqkv_ = nullptr, *patt_ = nullptr, *pgu_ = nullptr, *ph_ = nullptr;
+    int *h_meta_ = nullptr, *d_meta_ = nullptr;
+    void* attn_work_ = nullptr;
 };
 
 }    // namespace cccc

@@ -1,8 +1,8 @@
 // The quantised cccc LLM (DecodeStep) behind the LanguageModel interface, for the registry, the scheduler and the command
 // line.  config.json: {"architecture": "cccc-llm", "hidden", "n_heads", "n_kv_heads", "head_dim", "ffn", "vocab", "layers",
 // "rope_theta", "eps", "qk_norm", and optionally "weights" (container file, default model.bin) and "weight_data_type"
-// ("fp8_e4m3", "fp8_e5m2", "fp4_e2m1": quantise while loading)}.  Prompts go through the decode step token by token, as the
-// generation loop of this model always did; sequences that decode together share a step.
+// ("fp8_e4m3", "fp8_e5m2", "fp4_e2m1": quantise while loading)}.  Prompts run in passes of many tokens (DecodeStep::prompt);
+// sequences that decode together share a step.
 #include "decode_step.h"
 #include "language_model.h"
 
@@ -45,7 +45,9 @@ public:
         if (!f.open(path)) { return fail(err, "cannot open '" + path + "'"); }
         vocab_ = m.vocab;
         batch_ = std::min(o.max_sequences, 32);
-        return step_.load(&gpu_, f, m, batch_, nullptr, 0, err);
+        if (!step_.load(&gpu_, f, m, batch_, nullptr, 0, err)) { return false; }
+        step_.reservePrompts(std::max(1, std::min(o.max_step_tokens, kMostPromptTokens)));
+        return true;
     }
     int vocab() const override { return vocab_; }
     KvCache& cache() override { return step_.cache(); }
@@ -64,6 +66,7 @@ public:
             wanted += entries[e].want.size();
             longest = std::max(longest, entries[e].tokens.size());
         }
+        if (longest > 1 && step_.promptTokens() > 0) { return prompts(entries, first, logits, choice); }
         std::vector<uint16_t> row(logits ? (size_t)batch_ * vocab_ : 0);
         for (size_t i = 0; i < longest; i++)    // the i-th tokens of all entries that have one
         {
@@ -90,11 +93,7 @@ public:
                 {
                     if (E.want[w] != (int)i) { continue; }
                     if (choice) { choice[first[owner[k]] + w] = next[k]; }
-                    for (int v = 0; logits && v < vocab_; v++)
-                    {
-                        const uint32_t u = (uint32_t)row[k * vocab_ + v] << 16;
-                        std::memcpy(logits + (first[owner[k]] + w) * vocab_ + v, &u, 4);
-                    }
+                    if (logits) { widen(row.data() + k * vocab_, logits + (first[owner[k]] + w) * vocab_); }
                 }
             }
         }
@@ -102,6 +101,61 @@ public:
     }
 
 private:
+    static constexpr int kMostPromptTokens = 2048;    // of a pass: more bring the linears nothing, and cost memory
+
+    // Passes of up to promptTokens() tokens; a long entry goes on in the next one.  first[e]: the place of entry e's results.
+    int prompts(const std::vector<StepEntry>& entries, const std::vector<size_t>& first, float* logits, int* choice)
+    {
+        std::vector<size_t> done(entries.size(), 0);
+        for (;;)
+        {
+            std::vector<DecodeStep::PromptEntry> pass;
+            std::vector<size_t> count(entries.size(), 0);
+            std::vector<int> want;
+            std::vector<size_t> place;
+            size_t at = 0;
+            for (size_t e = 0; e < entries.size(); e++)
+            {
+                const StepEntry& E = entries[e];
+                count[e] = std::min((size_t)step_.promptTokens() - at, E.tokens.size() - done[e]);
+                if (count[e] == 0) { continue; }
+                pass.push_back({ E.slot, cache().length(E.slot), (int)count[e], E.tokens.data() + done[e] });
+                for (size_t w = 0; w < E.want.size(); w++)
+                {
+                    const size_t t = (size_t)E.want[w];
+                    if (t < done[e] || t >= done[e] + count[e]) { continue; }
+                    want.push_back((int)(at + t - done[e]));
+                    place.push_back(first[e] + w);
+                }
+                at += count[e];
+            }
+            if (at == 0) { return 0; }
+            std::vector<uint16_t> rows(logits ? want.size() * vocab_ : 0);
+            std::vector<int> next(want.size());
+            if (step_.prompt(pass, want, next.data(), logits ? rows.data() : nullptr) != 0) { return 1; }
+            launches_ += step_.lastLaunches();
+            for (size_t i = 0; i < want.size(); i++)
+            {
+                if (choice) { choice[place[i]] = next[i]; }
+                if (logits) { widen(rows.data() + i * vocab_, logits + place[i] * vocab_); }
+            }
+            for (size_t e = 0; e < entries.size(); e++)
+            {
+                done[e] += count[e];
+                if (count[e]) { cache().setLength(entries[e].slot, cache().length(entries[e].slot) + (int)count[e]); }
+            }
+        }
+    }
+
+    void widen(const uint16_t* row, float* out) const
+    {
+        for (int v = 0; v < vocab_; v++)
+        {
+            const uint32_t u = (uint32_t)row[v] << 16;
+            std::memcpy(out + v, &u, 4);
+        }
+    }
+
     static bool fail(std::string* err, const std::string& what)
     {
         if (err) { *err = what; }

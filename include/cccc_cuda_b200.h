@@ -327,6 +327,11 @@ typedef struct cuda_attn_decode
 } cuda_attn_decode;
 C_EXPORT int cuda_attn_decode_bf16(const cuda_attn_decode* a, void* stream, unsigned int flags);
 
+/* The part of cuda_attn_decode_bf16 that comes before the scores, for any number of tokens (B of them, each with its pos and
+ * slot; several may belong to one sequence): norm and rotation of q and k with the same bits, k and v appended.  The rotated
+ * queries go to `out` ([B] rows of H*head_dim, stride ldo), which may be q itself.  head_dim 64 or 128. */
+C_EXPORT int cuda_attn_append_bf16(const cuda_attn_decode* a, void* stream, unsigned int flags);
+
 /* ---- additions: a whole decode step as one kernel ------------------------------------------- */
 
 /* No counterpart in the reference (it issues about 40 ops per layer, each followed by a device
