@@ -157,7 +157,7 @@ C_EXPORT int cuda_gemm_w8a8_bf16(const void* W, float w_inv_scale, const void* X
         return 1;
     }
     const W8A8Member m = { W, Y, w_inv_scale, alpha, beta, N_out, ldw, ldy_m, ldy_n };
-    return launch_w8a8(&ws->scratch, &m, 1, X, act_scale, M_tokens, K, ldx, (cudaStream_t)stream, flags, false, false, (flags >> 8) & 3u);
+    return launch_w8a8(&ws->scratch, &m, 1, X, act_scale, M_tokens, K, ldx, (cudaStream_t)stream, flags, false, false, (flags >> 8) & 7u);
 }
 
 C_EXPORT int cuda_gemm_w8a8_bf16_group(unsigned int count, const cuda_wq_linear* linears, const void* X, float act_scale, unsigned int M_tokens,
@@ -178,7 +178,7 @@ C_EXPORT int cuda_gemm_w8a8_bf16_group(unsigned int count, const cuda_wq_linear*
         m[j] = { linears[j].W, linears[j].Y, linears[j].inv_scale, linears[j].alpha, linears[j].beta, linears[j].N_out, linears[j].ldw,
             linears[j].ldy_m, linears[j].ldy_n };
     }
-    return launch_w8a8(&ws->scratch, m, count, X, act_scale, M_tokens, K, ldx, (cudaStream_t)stream, flags, false, false, (flags >> 8) & 3u);
+    return launch_w8a8(&ws->scratch, m, count, X, act_scale, M_tokens, K, ldx, (cudaStream_t)stream, flags, false, false, (flags >> 8) & 7u);
 }
 
 C_EXPORT int cuda_gemm_fp8_fp8(const void* W, float w_inv_scale, const void* X_fp8, float x_inv_scale, void* Y, int y_type, unsigned int N_out,
@@ -195,7 +195,7 @@ C_EXPORT int cuda_gemm_fp8_fp8(const void* W, float w_inv_scale, const void* X_f
         return 1;
     }
     const W8A8Member m = { W, Y, w_inv_scale, alpha, beta, N_out, ldw, ldy_m, ldy_n };
-    return launch_w8a8(&ws->scratch, &m, 1, X_fp8, x_inv_scale, M_tokens, K, ldx, (cudaStream_t)stream, flags & 1u, true, y_type == DT_E4M3, (flags >> 8) & 3u);
+    return launch_w8a8(&ws->scratch, &m, 1, X_fp8, x_inv_scale, M_tokens, K, ldx, (cudaStream_t)stream, flags & 1u, true, y_type == DT_E4M3, (flags >> 8) & 7u);
 }
 
 C_EXPORT int cuda_bf16_to_fp8e4m3_dynamic(const void* src, void* dst_fp8, unsigned int n, void* d_absmax_tmp, void* d_inv_scale_out)
@@ -207,7 +207,7 @@ C_EXPORT int cuda_bf16_to_fp8e4m3_dynamic(const void* src, void* dst_fp8, unsign
     count_launch();
     absmax_bf16_rows_kernel<<<dim3(gx > 1024u ? 1024u : gx, 1), 256>>>((const uint16_t*)src, n, n, 1, (float*)d_absmax_tmp);
     count_launch();
-    quantise_activations_kernel<<<dim3(gx, 1), 256>>>((const uint16_t*)src, n, n, 1, (uint8_t*)dst_fp8, n, (const float*)d_absmax_tmp, 0.f, 0.f,
+    quantise_activations_kernel<<<dim3(gx, 1), 256>>>((const uint16_t*)src, n, n, 1, (uint8_t*)dst_fp8, n, (const float*)d_absmax_tmp, 1u, 0.f, 0.f,
         (float*)d_inv_scale_out, 1, false, false);
     return report_launch("bf162fp8e4m3_dynamic");
 }

@@ -2,17 +2,24 @@
 // the reference selects with act_data_type = FP8_E4M3 (cccc/cublas_real.h:619-666: quantise the BF16 activations, static
 // scale or dynamic absmax, then a cublasLt FP8 x FP8 matmul with both scales).  Here the quantised activations are one
 // E4M3 row per token of the native-operand FP8 kernel (gemm_native.cuh, PIECES = 1): both operands go into
-// tcgen05.mma kind::f8f6f4 as they are.  More than 32 tokens run on CTA pairs (gemm_w8a8_pair.cuh).
+// tcgen05.mma kind::f8f6f4 as they are.  More than 32 tokens run with k slices (gemm_w8a8_split.cuh) or on CTA pairs
+// (gemm_w8a8_pair.cuh).
 #pragma once
 
 #include "gemm_native.cuh"
 #include "gemm_w8a8_pair.cuh"
+#include "gemm_w8a8_split.cuh"
 
 namespace b200
 {
 
-constexpr int W8A8_MAX_TOKENS = 32;    // up to here the streaming kernel (all SMs share the k range); above, CTA pairs
-// (the streaming kernel with 64 token columns measured slower than the pairs: 27.8 against 20 us for 4096 x 4096 at 64 tokens)
+constexpr int W8A8_MAX_TOKENS = 32;    // up to here the streaming kernel (all SMs share the k range)
+
+// More tokens: k slices, or CTA pairs?  The line depends on tokens and k alone, so that a group of linears and the separate calls
+// take the same kernel and give the same bits.  Measured (dynamic scale, pairs' best form / slices, us): up to 64 tokens the
+// slices win on every linear of a layer (gemm_w8a8_split.cuh); at 128 tokens 4096 x 4096 17.9 / 14.2 but 24576 x 4096 31.4 / 38.3
+// (192 tiles, one CTA per SM); long k has few features: 4096 x 12288 at 128 / 256 / 300 tokens 35.6 / 21.9, 43.7 / 31.4, 44.8 / 44.6.
+static inline bool w8a8_split_preferred(unsigned int M, unsigned int K) { return M <= 64 || (M <= 256 && K >= 8192); }
 
 static inline int w8a8_launch_failed()
 {
@@ -50,14 +57,29 @@ static __global__ void __launch_bounds__(256) absmax_bf16_rows_kernel(const uint
     }
 }
 
+// The largest of n (at most W8A8_MAX_BLOCKS) non-negative floats, for every thread of a block of 256.
+constexpr unsigned int W8A8_MAX_BLOCKS = 148;
+__device__ __forceinline__ float block_maximum(const float* v, unsigned int n)
+{
+    __shared__ unsigned int of_warp[8];
+    unsigned int m = threadIdx.x < n ? __float_as_uint(v[threadIdx.x]) : 0u;    // they order as their bits
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o)); }
+    if ((threadIdx.x & 31u) == 0) { of_warp[threadIdx.x >> 5] = m; }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; w++) { m = max(m, of_warp[w]); }
+    return __uint_as_float(m);
+}
+
 // BF16 -> E4M3 with the reference's encoder (float_to_e4m3, cuda_functions.cu:2551-2580).  Dynamic (fwd_static == 0):
 // scale = 448 / absmax, multiplier back = absmax / 448 (1 and 1 for an all-zero tensor), cuda_functions.cu:2640-2657;
 // static: fwd_static = 1 / act_scale, multiplier back = inv_static = act_scale (cublas_real.h:627-632).
 // Grid (column chunks, rows + padding rows): rows past `rows` are written as zeros.  inv_out[r] receives the multiplier
 // back for each of the first n_inv rows (the linear reads one per token); pass n_inv = 1 for a single word.
 static __global__ void __launch_bounds__(256) quantise_activations_kernel(const uint16_t* __restrict__ X, unsigned int ld, unsigned int cols,
-    unsigned int rows, uint8_t* __restrict__ Q, unsigned int ldq, const float* __restrict__ absmax, float fwd_static, float inv_static,
-    float* __restrict__ inv_out, unsigned int n_inv, bool pdl, bool src_is_e4m3)
+    unsigned int rows, uint8_t* __restrict__ Q, unsigned int ldq, const float* __restrict__ absmax, unsigned int n_max, float fwd_static,
+    float inv_static, float* __restrict__ inv_out, unsigned int n_inv, bool pdl, bool src_is_e4m3)
 {
     if (pdl)
     {
@@ -76,7 +98,8 @@ static __global__ void __launch_bounds__(256) quantise_activations_kernel(const 
     if (fwd_static == 0.f)
     {
         float a;
-        if (absmax) { a = *absmax; }
+        if (absmax && n_max == 1) { a = *absmax; }
+        else if (absmax) { a = block_maximum(absmax, n_max); }
         else
         {
             // a small tensor: every block that quantises finds the largest magnitude itself (eight values per load; the
@@ -116,16 +139,20 @@ static __global__ void __launch_bounds__(256) quantise_activations_kernel(const 
     Q[(size_t)r * ldq + i] = r < rows ? float_to_e4m3(bf16_bits_to_float(X[(size_t)r * ld + i]), fwd) : (uint8_t)0;
 }
 
-// The same two steps for many tokens, eight values per thread (16-byte loads, 8-byte stores; cols and ld multiples of 8,
-// aligned bases), grid-stride over the [rows][cols / 8] groups.
-static __global__ void __launch_bounds__(256) absmax_bf16_x8_kernel(const uint16_t* __restrict__ X, unsigned int ld, unsigned int cols, unsigned int rows,
-    float* __restrict__ absmax)
+// The same two steps, eight values per thread and access (16-byte loads; cols and ld multiples of 8, aligned bases).  The
+// largest magnitudes of up to W8A8_MAX_BLOCKS blocks go side by side instead of into one word by atomicMax: nothing has to be
+// cleared first, which took a memset of 1.5 us and a gap per call.
+static __global__ void __launch_bounds__(1024) absmax_bf16_x8_kernel(const uint16_t* __restrict__ X, unsigned int ld, unsigned int cols, unsigned int rows,
+    float* __restrict__ maxima, bool pdl)
 {
-    __shared__ unsigned int warp_max[8];
+    __shared__ unsigned int warp_max[32];
+    pdl_launch_dependents();    // the quantiser
+    if (pdl) { pdl_wait(); }
     const unsigned int per_row = cols / 8;
-    const unsigned long long groups = (unsigned long long)rows * per_row;
+    const unsigned long long groups = (unsigned long long)rows * per_row, step = (unsigned long long)gridDim.x * 1024;
     unsigned int m = 0;
-    for (unsigned long long j = (unsigned long long)blockIdx.x * 256 + threadIdx.x; j < groups; j += (unsigned long long)gridDim.x * 256)
+#pragma unroll 4
+    for (unsigned long long j = (unsigned long long)blockIdx.x * 1024 + threadIdx.x; j < groups; j += step)
     {
         const uint4 v = *reinterpret_cast<const uint4*>(X + (size_t)(j / per_row) * ld + (size_t)(j % per_row) * 8);
         const unsigned int w[4] = { v.x, v.y, v.z, v.w };
@@ -144,18 +171,21 @@ static __global__ void __launch_bounds__(256) absmax_bf16_x8_kernel(const uint16
     if (threadIdx.x == 0)
     {
 #pragma unroll
-        for (int w = 1; w < 8; w++) { m = max(m, warp_max[w]); }
-        atomicMax(reinterpret_cast<unsigned int*>(absmax), m << 16);
+        for (int w = 1; w < 32; w++) { m = max(m, warp_max[w]); }
+        maxima[blockIdx.x] = __uint_as_float(m << 16);
     }
 }
 
 static __global__ void __launch_bounds__(256) quantise_activations_x8_kernel(const uint16_t* __restrict__ X, unsigned int ld, unsigned int cols,
-    unsigned int rows, uint8_t* __restrict__ Q, const float* __restrict__ absmax, float fwd_static, float inv_static, float* __restrict__ inv_out)
+    unsigned int rows, uint8_t* __restrict__ Q, const float* __restrict__ maxima, unsigned int n_max, float fwd_static, float inv_static,
+    float* __restrict__ inv_out)
 {
+    pdl_launch_dependents();    // the linear: its weights do not depend on this
+    pdl_wait();
     float fwd = fwd_static, inv = inv_static;
     if (fwd_static == 0.f)
     {
-        const float a = *absmax;
+        const float a = block_maximum(maxima, n_max);
         fwd = (a > 0.f) ? (448.0f / a) : 1.0f;
         inv = (a > 0.f) ? (a / 448.0f) : 1.0f;
     }
@@ -180,13 +210,14 @@ static __global__ void __launch_bounds__(256) quantise_activations_x8_kernel(con
 }
 
 // The linear(s).  Returns the C-ABI code, -1 for what this path does not serve (K % 128 != 0, unaligned operands, more
-// than three members, a workspace that is too small for the quantised activations).  pair_fh: tile shape of the launch
-// for more than 32 tokens (0: chosen here).
+// than three members, a workspace that is too small for the quantised activations).  pair_fh: form of the launch
+// for more than 32 tokens (0: chosen here, 1 .. 3: of the pair kernels, 4: the k slices).
 // x_is_e4m3: X holds E4M3 bytes (ldx in bytes) whose multiplier back is act_scale (> 0); y_e4m3: Y receives E4M3 bytes.
 static int launch_w8a8(const GemvScratch* ws, const W8A8Member* mem, unsigned int count, const void* X, float act_scale, unsigned int M,
     unsigned int K, unsigned int ldx, cudaStream_t stream, unsigned int flags, bool x_is_e4m3 = false, bool y_e4m3 = false, unsigned int pair_fh = 0)
 {
     if (count == 0 || count > (unsigned int)PF_MAX_GROUP || M == 0 || M > 65535u || act_scale < 0.f) { return -1; }
+    if (pair_fh > 4) { pair_fh &= 3u; }
     const bool big = M > (unsigned int)W8A8_MAX_TOKENS;
     if (x_is_e4m3 && !(act_scale > 0.f)) { return -1; }
     const unsigned int bnp = big ? M : (M <= 16 ? 16u : 32u);    // rows the quantiser writes
@@ -239,34 +270,61 @@ static int launch_w8a8(const GemvScratch* ws, const W8A8Member* mem, unsigned in
     if (!ok) { return -1; }
     const bool pdl = (flags & 1u) != 0;
     const bool dynamic = act_scale == 0.f && !x_is_e4m3;
-    // dynamic scale of a small tensor: the quantiser finds the maximum itself (16-byte loads: K and ldx % 8, an aligned base)
-    const bool self_absmax = dynamic && (size_t)M * K <= 16384 && (K % 8) == 0 && (ldx % 8) == 0 && sk_al16(X);
+    const bool eights = (K % 8) == 0 && (ldx % 8) == 0 && sk_al16(X);    // 16-byte loads of X
+    // dynamic scale of a small tensor: the quantiser finds the maximum itself
+    const bool self_absmax = dynamic && !big && (size_t)M * K <= 16384 && eights;
+    // The linear behind the quantiser (`after`: that was the launch before it on the stream; it lets its successor start).
+    auto many_tokens = [&](const NativeParams& n, const uint8_t* q, unsigned int ldq, bool after) {
+        if (pair_fh == 4 || (pair_fh == 0 && w8a8_split_preferred(M, K)))
+        {
+            const int r = launch_w8a8_split(n, mem, q, ldq, ws->device, ws->sm_count, stream, after || pdl);
+            if (r != -2) { return r; }
+        }
+        return launch_w8a8_pair(n, mem, q, ldq, ws->device, ws->sm_count, pair_fh, stream);
+    };
     if (big && x_is_e4m3 && (ldx % 16) == 0 && sk_al16(X))
     {
         // E4M3 activations that TMA can read where they lie: no copy, the multiplier back goes with the launch
         np.inv_scale = nullptr;
         np.act_inv = act_scale;
-        return launch_w8a8_pair(np, mem, (const uint8_t*)X, ldx, ws->device, ws->sm_count, pair_fh, stream);
+        return many_tokens(np, (const uint8_t*)X, ldx, false);
     }
-    if (big && !x_is_e4m3 && (K % 8) == 0 && (ldx % 8) == 0 && sk_al16(X))
+    cudaLaunchAttribute after[1];
+    after[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    after[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t qc;
+    memset(&qc, 0, sizeof(qc));
+    qc.stream = stream;
+    qc.attrs = after;
+    unsigned int n_max = 1;
+    if (dynamic && !self_absmax && eights)
     {
-        // many tokens: eight values per thread, a grid that fills the GPU a few times over
-        const unsigned long long groups = (unsigned long long)M * (K / 8);
-        unsigned long long blocks = (groups + 255) / 256;
-        if (blocks > 16ull * (unsigned)ws->sm_count) { blocks = 16ull * (unsigned)ws->sm_count; }
-        if (dynamic)
-        {
-            if (cudaMemsetAsync(absmax, 0, sizeof(float), stream) != cudaSuccess) { return w8a8_launch_failed(); }
-            count_launch();
-            absmax_bf16_x8_kernel<<<(unsigned int)blocks, 256, 0, stream>>>((const uint16_t*)X, ldx, K, M, absmax);
-        }
+        const unsigned long long blocks = ((unsigned long long)M * (K / 8) + 1023) / 1024;
+        n_max = (unsigned int)(blocks < W8A8_MAX_BLOCKS ? blocks : W8A8_MAX_BLOCKS);
+        absmax = inv + 64;    // behind the multipliers of up to 32 tokens
+        qc.gridDim = dim3(n_max);
+        qc.blockDim = dim3(1024);
+        qc.numAttrs = pdl ? 1 : 0;
         count_launch();
-        quantise_activations_x8_kernel<<<(unsigned int)blocks, 256, 0, stream>>>((const uint16_t*)X, ldx, K, M, Q, absmax, dynamic ? 0.f : 1.0f / act_scale,
-            dynamic ? 0.f : act_scale, inv);
-        if (cudaPeekAtLastError() != cudaSuccess) { return w8a8_launch_failed(); }
-        return launch_w8a8_pair(np, mem, Q, K, ws->device, ws->sm_count, pair_fh, stream);
+        if (cudaLaunchKernelEx(&qc, absmax_bf16_x8_kernel, (const uint16_t*)X, ldx, K, M, absmax, pdl) != cudaSuccess) { return w8a8_launch_failed(); }
     }
-    if (dynamic && !self_absmax)
+    if (big && !x_is_e4m3 && eights)
+    {
+        // many tokens: eight values per thread, a grid that fills the GPU
+        const unsigned long long blocks = ((unsigned long long)M * (K / 8) + 255) / 256, most = 8ull * (unsigned)ws->sm_count;
+        qc.gridDim = dim3((unsigned int)(blocks < most ? blocks : most));
+        qc.blockDim = dim3(256);
+        qc.numAttrs = pdl || dynamic ? 1 : 0;    // behind the absmax kernel, which itself starts after whatever came before
+        count_launch();
+        if (cudaLaunchKernelEx(&qc, quantise_activations_x8_kernel, (const uint16_t*)X, ldx, K, M, Q, (const float*)absmax, n_max, dynamic ? 0.f : 1.0f / act_scale,
+                dynamic ? 0.f : act_scale, inv)
+            != cudaSuccess)
+        {
+            return w8a8_launch_failed();
+        }
+        return many_tokens(np, Q, K, true);
+    }
+    if (dynamic && !self_absmax && !eights)
     {
         if (cudaMemsetAsync(absmax, 0, sizeof(float), stream) != cudaSuccess) { return w8a8_launch_failed(); }
         unsigned int gx = (K + 255) / 256;
@@ -283,16 +341,16 @@ static int launch_w8a8(const GemvScratch* ws, const W8A8Member* mem, unsigned in
     cfg.attrs = attr;
     cfg.gridDim = dim3((K + 255) / 256, bnp);
     cfg.blockDim = dim3(256);
-    const bool q_pdl = pdl && (!dynamic || self_absmax);    // behind the absmax kernel the quantiser is plainly ordered
+    const bool q_pdl = dynamic && !self_absmax ? eights : pdl;    // behind absmax_bf16_rows_kernel the quantiser is plainly ordered
     cfg.numAttrs = q_pdl ? 1 : 0;
     count_launch();
-    if (cudaLaunchKernelEx(&cfg, quantise_activations_kernel, (const uint16_t*)X, ldx, K, M, Q, K, self_absmax ? (const float*)nullptr : (const float*)absmax,
+    if (cudaLaunchKernelEx(&cfg, quantise_activations_kernel, (const uint16_t*)X, ldx, K, M, Q, K, self_absmax ? (const float*)nullptr : (const float*)absmax, n_max,
             dynamic ? 0.f : 1.0f / act_scale, dynamic ? 0.f : act_scale, inv, big ? 1u : M, q_pdl, x_is_e4m3)
         != cudaSuccess)
     {
         return w8a8_launch_failed();
     }
-    if (big) { return launch_w8a8_pair(np, mem, Q, K, ws->device, ws->sm_count, pair_fh, stream); }
+    if (big) { return many_tokens(np, Q, K, q_pdl); }
     auto launch_linear = [&](auto kernel, int smem) -> int {
         static std::atomic<bool> attr_set[2][64];
         const int which = bnp == 16 ? 0 : 1;

@@ -1,0 +1,102 @@
+"""W8A8 with k slices (up to 64 tokens by default, more where k is long; flags bits 8-10 = 4 take it above 32 tokens) against the
+CPU oracle, and the rule that the result does not depend on how many CTAs share the k range."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tests._util import assert_close, capi, from_dev_u16, to_dev
+from tests.test_gpu_w8a8 import run
+
+pytestmark = pytest.mark.gpu
+
+SPLIT = 4 << 8
+
+
+# tokens at the edges of the 64- and 128-token tiles; features that end inside a tile; k of one block (three slices empty), of
+# unequal slices, and long enough that every stage is used again
+@pytest.mark.parametrize("flags", [SPLIT, SPLIT | 1])
+@pytest.mark.parametrize("act_scale", [0.0, 0.0123])
+@pytest.mark.parametrize("N,K,M", [(128, 128, 33), (5, 256, 48), (300, 640, 64), (129, 896, 65), (1000, 4096, 100), (256, 12288, 128), (2500, 1024, 129), (384, 256, 300),
+                                   (6144, 2048, 64), (20000, 512, 40), (4096, 1152, 97)])
+def test_matches_the_oracle(N, K, M, act_scale, flags):
+    W, _, w_inv, X = O.make_inputs(O.FP8_E4M3, N, K, M, seed=N + M, scaled=True)
+    y32, _, _ = O.linear_w8a8(W, w_inv, X, N, M, K, act_scale=act_scale)
+    assert_close(O.bf16_bits_to_f32(run(W, w_inv, X, act_scale, N, M, K, flags=flags)).reshape(M, N), y32, (N, K, M, act_scale))
+
+
+@pytest.mark.parametrize("M", [34, 70])
+def test_float32_strides_and_accumulate(M):
+    """float32 output: sums of 1024 products in another order than float64's, 2^-24 per addition at most; transposed output with
+    alpha and beta; rows of Y that are not 8-byte aligned."""
+    N, K = 203, 1024
+    W, _, w_inv, X = O.make_inputs(O.FP8_E4M3, N, K, M, seed=5, scaled=True)
+    y32, _, _ = O.linear_w8a8(W, w_inv, X, N, M, K)
+    Yf = run(W, w_inv, X, 0.0, N, M, K, flags=4 | SPLIT).reshape(M, N)
+    rms = np.sqrt(np.mean(np.square(y32), axis=1, keepdims=True))
+    assert np.max(np.abs(Yf - y32) / np.maximum(np.abs(y32), rms)) < 1e-5
+    rng = np.random.default_rng(4)
+    ya, _, _ = O.linear_w8a8(W, w_inv, X, N, M, K, alpha=0.25)
+    Y0 = O.f32_to_bf16_bits(rng.standard_normal((N, M + 3)).astype(np.float32))
+    got = O.bf16_bits_to_f32(run(W, w_inv, X, 0.0, N, M, K, Y0=Y0.copy(), alpha=0.25, beta=1.5, ldy_m=1, ldy_n=M + 3, flags=SPLIT)[:N * (M + 3)]).reshape(N, M + 3)
+    assert_close(got[:, :M].T.copy(), (ya.T + 1.5 * O.bf16_bits_to_f32(Y0)[:, :M]).T.copy(), "alpha beta strides")
+    assert np.array_equal(got[:, M:], O.bf16_bits_to_f32(Y0)[:, M:])
+    for ldy in (N + 1, N + 2):
+        assert_close(O.bf16_bits_to_f32(np.resize(run(W, w_inv, X, 0.0, N, M, K, ldy_m=ldy, flags=SPLIT), M * ldy)).reshape(M, ldy)[:, :N], y32, ldy)
+
+
+@pytest.mark.parametrize("K,M", [(1024, 64), (8192, 100)])
+def test_the_bits_do_not_depend_on_the_grid(K, M):
+    """The same 128 features alone (four CTAs per tile), with others in a group, and as part of a matrix whose tiles fill the GPU
+    without cutting k."""
+    import torch
+
+    c, most = capi(), 40960 if K < 4096 else 20480
+    W, _, w_inv, X = O.make_inputs(O.FP8_E4M3, most, K, M, seed=1, scaled=True)
+    W = W.reshape(most, K)
+    dX = to_dev(X)
+
+    def linear(n):
+        y = torch.zeros(M, n, dtype=torch.int16, device="cuda")
+        assert c.gemm_w8a8_bf16(to_dev(W[:n].copy()), w_inv, dX, 0.0, y, n, M, K, flags=1) == 0 and c.check_error("grid") == 0
+        return y[:, :128]
+
+    alone = linear(128)
+    for n in (6144, most):
+        assert torch.equal(linear(n), alone)
+    items = [dict(W=to_dev(W[:n].copy()), S=None, inv=w_inv, N=n, Y=torch.zeros(M, n, dtype=torch.int16, device="cuda")) for n in (128, 9000, 4096)]
+    assert c.gemm_w8a8_bf16_group(c.make_group(items, K), dX, 0.0, M, K) == 0 and c.check_error("group") == 0
+    assert torch.equal(items[0]["Y"], alone)
+
+
+@pytest.mark.parametrize("M", [20, 64])
+def test_the_largest_magnitude_is_found_wherever_it_lies(M):
+    """One scale for the tensor: every block of the search has to count."""
+    N, K = 128, 4096
+    W, _, w_inv, X0 = O.make_inputs(O.FP8_E4M3, N, K, M, seed=M, scaled=True)
+    for at in (0, 5, M * K // 2 + 8191, M * K - 1):
+        X = X0.reshape(-1).copy()
+        X[at] = O.f32_to_bf16_bits(np.array([300.0], np.float32))[0]
+        y32, _, _ = O.linear_w8a8(W, w_inv, X.reshape(X0.shape), N, M, K)
+        assert_close(O.bf16_bits_to_f32(run(W, w_inv, X.reshape(X0.shape), 0.0, N, M, K)).reshape(M, N), y32, (M, at))
+
+
+@pytest.mark.parametrize("y_type", [3, 4])
+def test_e4m3_activations_where_they_lie(y_type):
+    """cuda_gemm_fp8_fp8 at 70 tokens: no quantiser before the linear; BF16 and E4M3 output."""
+    import torch
+
+    c, N, K, M = capi(), 600, 1024, 70
+    W, _, w_inv, _ = O.make_inputs(O.FP8_E4M3, N, K, M, seed=2, scaled=True)
+    Xq = O.float_to_fp8(np.random.default_rng(0).standard_normal(M * K).astype(np.float32), O.FP8_E4M3, 32.0)
+    y = ((O.fp8_to_float(Xq, O.FP8_E4M3, 1.0).reshape(M, K).astype(np.float64) @ O.fp8_to_float(W, O.FP8_E4M3, 1.0).reshape(N, K).astype(np.float64).T)
+         * (float(np.float32(w_inv)) / 32.0)).astype(np.float32)
+    out = torch.zeros(M * N, dtype=torch.int16 if y_type == 3 else torch.uint8, device="cuda")
+    dW, dX = to_dev(W), to_dev(Xq)
+    assert c.lib().cuda_gemm_fp8_fp8(dW.data_ptr(), w_inv, dX.data_ptr(), 1 / 32, out.data_ptr(), y_type, N, M, K, K, K, N, 1, 1.0, 0.0, None, SPLIT) == 0
+    assert c.check_error("fp8 x fp8") == 0
+    if y_type == 3:
+        assert_close(O.bf16_bits_to_f32(from_dev_u16(out)).reshape(M, N), y, "bf16")
+    else:    # a code is a 6-12 % step: sums that differ in their last bits may land on either side of one
+        want = O.float_to_fp8(O.bf16_bits_to_f32(O.f32_to_bf16_bits(y)).reshape(-1), O.FP8_E4M3, 1.0)
+        diff = np.abs(out.cpu().numpy().astype(np.int16) - want.astype(np.int16))
+        assert diff.max() <= 1 and np.mean(diff != 0) < 2e-3
