@@ -37,6 +37,7 @@ SYMBOLS = {
     "cuda_fp4_blockscale_to_bf16": (_i, [_vp, _vp, _vp, _u, _u]),
     "cuda_float_to_fp4_blockscale": (_i, [_vp, _vp, _vp, _u, _u]),
     "cuda_check_error": (_i, [C.c_char_p]),
+    "cuda_b200_status": (_i, [_vp, _vp]),
     "cuda_clear_last_error": (None, []),
     "cuda_gemm_wq_bf16": (_i, [_i, _vp, _vp, _f, _vp, _vp, _u, _u, _u, _u, _u, _u, _u, _f, _f, _vp, _u]),
     "cuda_gemm_wq_bf16_static": (_i, [_i, _vp, _vp, _f, _vp, _vp, _u, _u, _u, _u, _u, _u, _u, _f, _f, _vp, _u]),

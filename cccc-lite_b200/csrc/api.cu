@@ -292,6 +292,12 @@ C_EXPORT int cuda_gemm_wq_bf16_plan(int w_type, const void* W, const void* blk_s
 
 C_EXPORT int cuda_check_error(const char* label) { return sync_and_report(label ? label : "cuda"); }
 
+C_EXPORT int cuda_b200_status(void* host, void* stream)
+{
+    unsigned int* w = cuda_b200_status_word();
+    return w && cudaMemcpyAsync(host, w, sizeof(*w), cudaMemcpyDeviceToHost, (cudaStream_t)stream) == cudaSuccess ? 0 : 1;
+}
+
 C_EXPORT void cuda_clear_last_error(void) { cudaGetLastError(); }
 
 C_EXPORT unsigned long long cuda_b200_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }

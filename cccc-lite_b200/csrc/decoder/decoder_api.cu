@@ -75,4 +75,10 @@ C_EXPORT int cuda_b200_decoder_check(const char* label)
     return 0;
 }
 
+C_EXPORT int cuda_b200_decoder_status(void* host, void* stream)
+{
+    unsigned int* w = decoder_status_word();
+    return w && cudaMemcpyAsync(host, w, sizeof(*w), cudaMemcpyDeviceToHost, (cudaStream_t)stream) == cudaSuccess ? 0 : 1;
+}
+
 C_EXPORT unsigned long long cuda_b200_decoder_launches(void) { return g_launches.load(std::memory_order_relaxed); }

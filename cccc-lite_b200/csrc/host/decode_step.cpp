@@ -379,10 +379,7 @@ bool DecodeStep::load(GpuControl* gpu, const BinFile& file, const ModelConfig& c
     }
     if (!ok) { return false; }
     // first use of the kernels allocates the library's per-device workspace: do it before any capture
-    std::vector<int> z(max_batch, 0);
-    cudaMemcpy(d_ids_, z.data(), (size_t)max_batch * 4, cudaMemcpyHostToDevice);
-    cudaMemcpy(d_pos_, z.data(), (size_t)max_batch * 4, cudaMemcpyHostToDevice);
-    cudaMemcpy(d_slot_, z.data(), (size_t)max_batch * 4, cudaMemcpyHostToDevice);
+    cudaMemset(d_ids_, 0, (size_t)max_batch * 16);
     if (tp_) { tp_->barrier(); }
     const int rc = issue(1, gpu_->stream());
     gpu_->synchronize();
@@ -460,17 +457,19 @@ bool DecodeStep::loadTensors(const BinFile& file, std::string* err)
     gu_ = (uint16_t*)dmalloc(B * 2 * ffn_loc_ * 2);
     h_ = (uint16_t*)dmalloc(B * ffn_loc_ * 2);
     logits_ = (uint16_t*)dmalloc(B * vocab_loc_ * 2);
-    d_ids_ = (int*)dmalloc(B * 4);
-    d_pos_ = (int*)dmalloc(B * 4);
-    d_slot_ = (int*)dmalloc(B * 4);
-    d_best_ = (float*)dmalloc(B * 4);
-    if (!x_ || !xn_ || !tmp_ || !qkv_ || !att_ || !gu_ || !h_ || !logits_ || !d_ids_ || !d_pos_ || !d_slot_ || !d_best_) { return fail(err, "no device memory for the step's buffers"); }
-    // one pinned block: ids in, positions in, slots in, ids out, best out
-    if (cudaMallocHost((void**)&h_ids_, B * 20) != cudaSuccess) { return fail(err, "no pinned memory"); }
+    d_ids_ = (int*)dmalloc(B * 16);    // one block, one copy each way: ids, positions, slots, best
+    d_pos_ = d_ids_ + B;
+    d_slot_ = d_pos_ + B;
+    d_best_ = (float*)(d_slot_ + B);
+    if (!x_ || !xn_ || !tmp_ || !qkv_ || !att_ || !gu_ || !h_ || !logits_ || !d_ids_) { return fail(err, "no device memory for the step's buffers"); }
+    // one pinned block: ids, positions and slots in; the device's block out; the status word
+    if (cudaMallocHost((void**)&h_ids_, B * 28 + 4) != cudaSuccess) { return fail(err, "no pinned memory"); }
+    std::memset(h_ids_, 0, B * 28 + 4);
     h_pos_ = h_ids_ + B;
     h_slot_ = h_pos_ + B;
     h_out_ = h_slot_ + B;
-    h_best_ = (float*)(h_out_ + B);
+    h_best_ = (float*)(h_out_ + 3 * B);
+    h_status_ = (unsigned int*)(h_best_ + B);
     if (cudaMallocHost((void**)&h_logits_, B * vocab_loc_ * 2) != cudaSuccess) { return fail(err, "no pinned memory for the logits"); }
     if (world_ > 1)
     {
@@ -821,6 +820,14 @@ bool DecodeStep::useProgram(bool on)
 
 int DecodeStep::step(const int* token_ids, const int* positions, int M, int* next_ids, float* best_logits, uint16_t* logits_host, const int* slots)
 {
+    int rc = launch(token_ids, positions, M, logits_host != nullptr, slots);
+    if (rc == 0) { rc = finish(next_ids, best_logits); }
+    if (rc == 0 && logits_host) { std::memcpy(logits_host, h_logits_, (size_t)M * vocab_loc_ * 2); }
+    return rc;
+}
+
+int DecodeStep::launch(const int* token_ids, const int* positions, int M, bool logits, const int* slots)
+{
     if (M < 1 || M > max_batch_) { return -1; }
     gpu_->setAsCurrent();
     cudaStream_t st = gpu_->stream();
@@ -830,9 +837,8 @@ int DecodeStep::step(const int* token_ids, const int* positions, int M, int* nex
         h_pos_[i] = positions[i];
         h_slot_[i] = slots ? slots[i] : i;
     }
-    cudaMemcpyAsync(d_ids_, h_ids_, (size_t)M * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(d_pos_, h_pos_, (size_t)M * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(d_slot_, h_slot_, (size_t)M * 4, cudaMemcpyHostToDevice, st);
+    // ids, positions and slots lie one behind the other, here and on the device
+    cudaMemcpyAsync(d_ids_, h_ids_, (size_t)max_batch_ * 12, cudaMemcpyHostToDevice, st);
     int rc = 0;
     if (use_program_ && M == 1 && program_)
     {
@@ -867,13 +873,22 @@ int DecodeStep::step(const int* token_ids, const int* positions, int M, int* nex
         rc = cudaGraphLaunch(graphs_[M], st) == cudaSuccess ? 0 : 1;
         last_launches_ = launches_per_step_;
     }
-    cudaMemcpyAsync(h_out_, d_ids_, (size_t)M * 4, cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(h_best_, d_best_, (size_t)M * 4, cudaMemcpyDeviceToHost, st);
-    if (logits_host) { cudaMemcpyAsync(h_logits_, logits_, (size_t)M * vocab_loc_ * 2, cudaMemcpyDeviceToHost, st); }
-    if (cudaStreamSynchronize(st) != cudaSuccess) { rc = 1; }
-    if (cuda_check_error("decode step") != 0) { rc = 1; }
-    if (logits_host) { std::memcpy(logits_host, h_logits_, (size_t)M * vocab_loc_ * 2); }
-    for (int i = 0; i < M; i++)
+    // the chosen ids and, behind two other arrays, their logits
+    cudaMemcpyAsync(h_out_, d_ids_, (size_t)max_batch_ * 16, cudaMemcpyDeviceToHost, st);
+    rc |= cuda_b200_status(h_status_, st);
+    if (logits) { cudaMemcpyAsync(h_logits_, logits_, (size_t)M * vocab_loc_ * 2, cudaMemcpyDeviceToHost, st); }
+    running_ = M;
+    if (rc != 0) { finish(h_out_, nullptr); }    // nothing stays under way
+    return rc;
+}
+
+int DecodeStep::finish(int* next_ids, float* best_logits)
+{
+    int rc = 0;
+    gpu_->setAsCurrent();
+    if (cudaStreamSynchronize(gpu_->stream()) != cudaSuccess) { rc = 1; }
+    if ((rc != 0 || *h_status_ != 0 || cudaPeekAtLastError() != cudaSuccess) && cuda_check_error("decode step") != 0) { rc = 1; }
+    for (int i = 0; i < running_; i++)
     {
         int id = h_out_[i] < 0 ? -1 : h_out_[i] + rank_ * vocab_loc_;
         float best = h_best_[i];

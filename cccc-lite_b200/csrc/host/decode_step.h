@@ -92,6 +92,11 @@ public:
     // rank); logits_host (nullable) receives this rank's shard of the BF16 logits, [M][vocab / world].
     // slots (nullable): the cache slot of each sequence; without it sequence i has slot i.
     int step(const int* token_ids, const int* positions, int M, int* next_ids, float* best_logits, uint16_t* logits_host, const int* slots = nullptr);
+    // The same in two halves: launch() starts the step (and the way of the logits to the host); where it returns 0, finish() waits
+    // for it, after which hostLogits() holds the [M][vocab / world] logits until the next launch.
+    int launch(const int* token_ids, const int* positions, int M, bool logits, const int* slots);
+    int finish(int* next_ids, float* best_logits);
+    const uint16_t* hostLogits() const { return h_logits_; }
     // New tokens of one sequence, which continue row `pos` of cache slot `slot`.
     struct PromptEntry
     {
@@ -165,6 +170,8 @@ private:
     int *d_ids_ = nullptr, *d_pos_ = nullptr, *d_slot_ = nullptr, *h_ids_ = nullptr, *h_pos_ = nullptr, *h_slot_ = nullptr, *h_out_ = nullptr;
     float *d_best_ = nullptr, *h_best_ = nullptr;
     uint16_t* h_logits_ = nullptr;
+    unsigned int* h_status_ = nullptr;
+    int running_ = 0;    // sequences of the step between launch() and finish()
     std::vector<Matrix> quantised_;    // tensors quantised while loading own their device memory
     int quantised_on_load_ = 0, layers_loaded_ = 0, last_launches_ = 0;
     KvCache cache_;

@@ -32,6 +32,16 @@ public:
     // a row of vocab() floats, choice (nullable) the id of the largest logit.  Returns 0; -1 for entries that cannot run
     // (a closed slot, one slot twice, a full cache, a token outside the vocabulary), nothing having run; 1 on a CUDA error.
     virtual int step(const std::vector<StepEntry>& entries, float* logits, int* choice) = 0;
+    // step() in two halves, so that a caller can make the place of the results ready while the device works: begin() checks the
+    // entries (-1: they cannot run, and there is nothing to end) and may start them; end() finishes them, with the results that
+    // begin() was told of (or null: not taken).  Nothing else may be asked of the model in between.
+    virtual int begin(std::vector<StepEntry> entries, bool logits, bool choice)
+    {
+        (void)logits, (void)choice;
+        held_ = std::move(entries);
+        return valid(held_) ? 0 : -1;
+    }
+    virtual int end(float* logits, int* choice) { return step(held_, logits, choice); }
     virtual int launchesLastStep() const { return 0; }
     virtual size_t weightBytes() const { return 0; }
     // Device time of one step in ms (the fastest of `repeat` runs of `inner` steps): `entries` sequences that hold `context`
@@ -45,6 +55,7 @@ public:
 protected:
     // The checks of step() that every model needs.
     bool valid(const std::vector<StepEntry>& entries);
+    std::vector<StepEntry> held_;    // between begin() and end()
 };
 
 struct ModelOptions

@@ -46,6 +46,11 @@ LayeredDecoder::~LayeredDecoder()
     if (h_meta_) { cudaFreeHost(h_meta_); }
     if (h_choice_) { cudaFreeHost(h_choice_); }
     if (h_logits_) { cudaFreeHost(h_logits_); }
+    if (h_status_) { cudaFreeHost(h_status_); }
+    for (cudaEvent_t e : piece_)
+    {
+        if (e) { cudaEventDestroy(e); }
+    }
 }
 
 void* LayeredDecoder::dmalloc(size_t bytes, bool zero)
@@ -306,7 +311,8 @@ bool LayeredDecoder::allocate(const ModelOptions& o, std::string* err)
     const size_t meta = 3 * T + 4 * T + 2 * windows_.size() * T;
     d_meta_ = (int*)get(meta * 4);
     ok = ok && cudaMallocHost((void**)&h_meta_, meta * 4) == cudaSuccess && cudaMallocHost((void**)&h_choice_, (size_t)want_cap_ * 4) == cudaSuccess
-        && cudaMallocHost((void**)&h_logits_, (size_t)want_cap_ * spec_.vocab * 4) == cudaSuccess;
+        && cudaMallocHost((void**)&h_logits_, (size_t)want_cap_ * spec_.vocab * 4) == cudaSuccess && cudaMallocHost((void**)&h_status_, 4) == cudaSuccess;
+    for (cudaEvent_t& e : piece_) { ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess; }
     if (!ok) { return fail(err, "no memory for the step's buffers"); }
     return true;
 }
@@ -551,39 +557,80 @@ int LayeredDecoder::issue(const Pass& p, cudaStream_t st)
     return r0.bad ? -1 : r0.n;
 }
 
-int LayeredDecoder::run(const Pass& p, float* logits, int* choice)
+// The results of the head's `rows` rows start for the host.
+void LayeredDecoder::sendResults(int rows, bool logits, bool choice)
 {
     cudaStream_t st = gpu_.stream();
+    const size_t V = (size_t)spec_.vocab;
+    if (cuda_b200_decoder_status(h_status_, st) != 0) { *h_status_ = 1; }    // not known: the step looks at the device's word
+    if (choice) { cudaMemcpyAsync(h_choice_, d_choice_, (size_t)rows * 4, cudaMemcpyDeviceToHost, st); }
+    for (int i = 0; i < kPieces && logits; i++)
+    {
+        const size_t r0 = (size_t)rows * i / kPieces, r1 = (size_t)rows * (i + 1) / kPieces;
+        if (r0 == r1) { continue; }
+        cudaMemcpy2DAsync(h_logits_ + r0 * V, V * 4, logits_ + r0 * ld_logits_, (size_t)ld_logits_ * 4, V * 4, r1 - r0, cudaMemcpyDeviceToHost, st);
+        cudaEventRecord(piece_[i], st);
+    }
+}
+
+// Row i goes to row place[i] of `logits`: a piece is copied on while the next one arrives.
+int LayeredDecoder::takeResults(int rows, const int* place, float* logits, int* choice)
+{
+    const size_t V = (size_t)spec_.vocab;
+    for (int i = 0; i < kPieces && logits; i++)
+    {
+        const size_t r0 = (size_t)rows * i / kPieces, r1 = (size_t)rows * (i + 1) / kPieces;
+        if (r0 == r1) { continue; }
+        if (cudaEventSynchronize(piece_[i]) != cudaSuccess) { return 1; }
+        for (size_t r = r0; r < r1; r++) { std::memcpy(logits + (size_t)place[r] * V, h_logits_ + r * V, V * 4); }
+    }
+    if (cudaStreamSynchronize(gpu_.stream()) != cudaSuccess) { return 1; }
+    for (int r = 0; r < rows && choice; r++) { choice[place[r]] = h_choice_[r]; }
+    return 0;
+}
+
+// Lengths up to a power of two share a graph.
+int LayeredDecoder::decodeBucket(const Pass& p, int rows)
+{
+    int len = 64;
+    while (len < p.parts[0].max_len) { len *= 2; }
+    return std::min(len, rows);
+}
+
+// Starts a decode step whose graph there is; its results (as asked for) follow it to the host.
+int LayeredDecoder::startDecode(const Pass& p, bool logits, bool choice, bool* started)
+{
+    cudaStream_t st = gpu_.stream();
+    *started = false;
+    if (!p.decode || p.wants > want_cap_) { return 0; }
+    auto it = graphs_.find({ p.entries, decodeBucket(p, cache_.rows()) });
+    if (it == graphs_.end()) { return 0; }
+    std::memcpy(h_meta_, p.host.data(), p.host.size() * 4);
+    if (cudaMemcpyAsync(d_meta_, h_meta_, p.host.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess || cudaGraphLaunch(it->second.first, st) != cudaSuccess) { return 1; }
+    last_launches_ += it->second.second;
+    sendResults(p.wants, logits, choice);
+    *started = true;
+    return 0;
+}
+
+// One pass; its i-th wanted row goes to place[i] of the results.
+int LayeredDecoder::run(const Pass& p, const std::vector<int>& place, float* logits, int* choice)
+{
+    cudaStream_t st = gpu_.stream();
+    bool started = false;
+    if (startDecode(p, logits != nullptr, choice != nullptr, &started)) { return 1; }
+    if (started) { return takeResults(p.wants, place.data(), logits, choice); }
     std::memcpy(h_meta_, p.host.data(), p.host.size() * 4);
     if (cudaMemcpyAsync(d_meta_, h_meta_, p.host.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) { return 1; }
     const unsigned long long before = cuda_b200_decoder_launches();
-    const size_t V = (size_t)spec_.vocab;
     auto fetch = [&](int row0, int rows) {
-        if (logits)
-        {
-            cudaMemcpy2DAsync(h_logits_, V * 4, logits_, (size_t)ld_logits_ * 4, V * 4, (size_t)rows, cudaMemcpyDeviceToHost, st);
-        }
-        if (choice) { cudaMemcpyAsync(h_choice_, d_choice_, (size_t)rows * 4, cudaMemcpyDeviceToHost, st); }
-        if (cudaStreamSynchronize(st) != cudaSuccess) { return false; }
-        if (logits) { std::memcpy(logits + (size_t)row0 * V, h_logits_, (size_t)rows * V * 4); }
-        if (choice) { std::memcpy(choice + row0, h_choice_, (size_t)rows * 4); }
-        return true;
+        sendResults(rows, logits != nullptr, choice != nullptr);
+        return takeResults(rows, place.data() + row0, logits, choice) == 0;
     };
     if (p.decode && p.wants <= want_cap_)
     {
-        // lengths up to a power of two share a graph
         Pass q = p;
-        int& len = q.parts[0].max_len;
-        len = 64;
-        while (len < p.parts[0].max_len) { len *= 2; }
-        len = std::min(len, cache_.rows());
-        auto it = graphs_.find({ p.entries, len });
-        if (it != graphs_.end())
-        {
-            if (cudaGraphLaunch(it->second.first, st) != cudaSuccess) { return 1; }
-            last_launches_ += it->second.second;
-            return fetch(0, p.wants) ? 0 : 1;
-        }
+        const int len = q.parts[0].max_len = decodeBucket(p, cache_.rows());
         // the first step of this shape runs launch by launch (which also loads the kernels), then the launches are recorded
         if (issue(q, st) < 0 || issueHead(q, 0, q.wants, st) < 0) { return -1; }
         const int launches = (int)(cuda_b200_decoder_launches() - before);
@@ -604,6 +651,7 @@ int LayeredDecoder::run(const Pass& p, float* logits, int* choice)
         graphs_[{ p.entries, len }] = { exec, launches };
         return 0;
     }
+    *h_status_ = 1;    // a pass without results: step() looks at the device's word
     if (issue(p, st) < 0) { return -1; }
     for (int r0 = 0; r0 < p.wants; r0 += want_cap_)
     {
@@ -616,19 +664,61 @@ int LayeredDecoder::run(const Pass& p, float* logits, int* choice)
     return cudaStreamSynchronize(st) == cudaSuccess ? 0 : 1;
 }
 
+// Where a pass' wanted rows go: in the order of the entries and of their wanted places.
+std::vector<int> LayeredDecoder::places(const Pass& p, const std::vector<StepEntry>& entries) const
+{
+    std::vector<int> first(entries.size(), 0), place;
+    for (size_t e = 1; e < entries.size(); e++) { first[e] = first[e - 1] + (int)entries[e - 1].want.size(); }
+    for (const auto& a : p.asked) { place.push_back(first[a.first] + a.second); }
+    return place;
+}
+
+void LayeredDecoder::advance(const std::vector<StepEntry>& entries, const std::vector<int>& count)
+{
+    for (size_t e = 0; e < entries.size(); e++)
+    {
+        if (count[e]) { cache_.setLength(entries[e].slot, cache_.length(entries[e].slot) + count[e]); }
+    }
+}
+
+int LayeredDecoder::begin(std::vector<StepEntry> entries, bool logits, bool choice)
+{
+    started_ = false;
+    const int rc = LanguageModel::begin(std::move(entries), logits, choice);
+    if (rc != 0 || held_.empty() || (int)held_.size() > cap_) { return rc; }
+    for (const auto& e : held_)
+    {
+        if (e.tokens.size() != 1 || e.want.size() != 1) { return 0; }
+    }
+    gpu_.setAsCurrent();
+    last_launches_ = 0;
+    held_pass_ = Pass();
+    makePass(held_, std::vector<int>(held_.size(), 0), std::vector<int>(held_.size(), 1), &held_pass_);
+    started_logits_ = logits;
+    started_choice_ = choice;
+    // a launch that fails leaves nothing started: end() runs the step anew, and says what is wrong
+    startDecode(held_pass_, logits, choice, &started_);
+    return 0;
+}
+
+int LayeredDecoder::end(float* logits, int* choice)
+{
+    if (!started_) { return step(held_, logits, choice); }
+    started_ = false;
+    gpu_.setAsCurrent();
+    if (takeResults(held_pass_.wants, places(held_pass_, held_).data(), started_logits_ ? logits : nullptr, started_choice_ ? choice : nullptr) != 0) { return 1; }
+    advance(held_, std::vector<int>(held_.size(), 1));
+    return *h_status_ == 0 && cudaPeekAtLastError() == cudaSuccess ? 0 : cuda_b200_decoder_check("decoder step");
+}
+
 int LayeredDecoder::step(const std::vector<StepEntry>& entries, float* logits, int* choice)
 {
     if (!valid(entries)) { return -1; }
     gpu_.setAsCurrent();
     last_launches_ = 0;
-    // passes of up to cap_ tokens; a long entry goes on in the next one.  Results are placed in the order asked for.
-    std::vector<int> done(entries.size(), 0), first(entries.size(), 0);
-    int wanted = 0;
-    for (size_t e = 0; e < entries.size(); e++)
-    {
-        first[e] = wanted;
-        wanted += (int)entries[e].want.size();
-    }
+    // passes of up to cap_ tokens; a long entry goes on in the next one
+    std::vector<int> done(entries.size(), 0);
+    unsigned int status = 0;
     for (;;)
     {
         std::vector<int> count(entries.size(), 0);
@@ -641,24 +731,13 @@ int LayeredDecoder::step(const std::vector<StepEntry>& entries, float* logits, i
         if (room == cap_) { break; }
         Pass p;
         makePass(entries, done, count, &p);
-        std::vector<int> place;
-        for (const auto& a : p.asked) { place.push_back(first[a.first] + a.second); }
-        std::vector<float> lg(logits && p.wants ? (size_t)p.wants * spec_.vocab : 0);
-        std::vector<int> ch(choice ? p.wants : 0);
-        const int rc = run(p, logits ? lg.data() : nullptr, choice ? ch.data() : nullptr);
+        const int rc = run(p, places(p, entries), logits, choice);
         if (rc) { return rc; }
-        for (size_t i = 0; i < place.size(); i++)
-        {
-            if (logits) { std::memcpy(logits + (size_t)place[i] * spec_.vocab, lg.data() + i * spec_.vocab, (size_t)spec_.vocab * 4); }
-            if (choice) { choice[place[i]] = ch[i]; }
-        }
-        for (size_t e = 0; e < entries.size(); e++)
-        {
-            done[e] += count[e];
-            if (count[e]) { cache_.setLength(entries[e].slot, cache_.length(entries[e].slot) + count[e]); }
-        }
+        status |= *h_status_;
+        for (size_t e = 0; e < entries.size(); e++) { done[e] += count[e]; }
+        advance(entries, count);
     }
-    return cuda_b200_decoder_check("decoder step");
+    return status == 0 && cudaPeekAtLastError() == cudaSuccess ? 0 : cuda_b200_decoder_check("decoder step");
 }
 
 float LayeredDecoder::timeStep(int entries, int tokens, int context, int inner, int repeat)
@@ -683,7 +762,7 @@ float LayeredDecoder::timeStep(int entries, int tokens, int context, int inner, 
     cudaEventCreate(&a);
     cudaEventCreate(&z);
     std::vector<int> ch((size_t)p.wants);
-    bool ok = p.wants <= want_cap_ && run(p, nullptr, ch.data()) == 0;
+    bool ok = p.wants <= want_cap_ && run(p, places(p, batch), nullptr, ch.data()) == 0;
     auto g = graphs_.end();
     if (ok && p.decode)
     {

@@ -120,6 +120,8 @@ public:
     int vocab() const override { return spec_.vocab; }
     KvCache& cache() override { return cache_; }
     int step(const std::vector<StepEntry>& entries, float* logits, int* choice) override;
+    int begin(std::vector<StepEntry> entries, bool logits, bool choice) override;
+    int end(float* logits, int* choice) override;
     int launchesLastStep() const override { return last_launches_; }
     size_t weightBytes() const override { return weight_bytes_; }
     float timeStep(int entries, int tokens, int context, int inner, int repeat) override;
@@ -218,7 +220,13 @@ private:
     cuda_b200_batch batchOf(const Pass& p, const Part& part) const;
     cuda_b200_batch wholeBatch(const Pass& p) const;
     int expandedFloor(const Pass& p, int window, std::vector<int>* floor, std::vector<int>* pos2) const;
-    int run(const Pass& p, float* logits, int* choice);
+    int run(const Pass& p, const std::vector<int>& place, float* logits, int* choice);
+    int startDecode(const Pass& p, bool logits, bool choice, bool* started);
+    void sendResults(int rows, bool logits, bool choice);
+    int takeResults(int rows, const int* place, float* logits, int* choice);
+    static int decodeBucket(const Pass& p, int rows);
+    std::vector<int> places(const Pass& p, const std::vector<StepEntry>& entries) const;
+    void advance(const std::vector<StepEntry>& entries, const std::vector<int>& count);
     size_t elem() const { return dtype_ == FLOAT ? 4 : 2; }
     int act() const { return dtype_ == FLOAT ? 0 : 3; }
 
@@ -261,6 +269,12 @@ private:
     float* h_logits_ = nullptr;
     std::map<std::pair<int, int>, std::pair<cudaGraphExec_t, int>> graphs_;    // (entries, length bucket) -> graph, launches
     int last_launches_ = 0;
+    // results on their way to the host: the rows' logits in pieces, each with an event behind it, and the status word
+    static constexpr int kPieces = 4;
+    cudaEvent_t piece_[kPieces] = {};
+    unsigned int* h_status_ = nullptr;
+    bool started_ = false, started_logits_ = false, started_choice_ = false;    // between begin() and end(): a decode step is under way
+    Pass held_pass_;
 };
 
 }    // namespace cccc

@@ -75,9 +75,10 @@ HOST_EXPORT int cccc_model_open_slot(void* m) { return ((LanguageModel*)m)->cach
 HOST_EXPORT void cccc_model_close_slot(void* m, int slot) { ((LanguageModel*)m)->cache().close(slot); }
 HOST_EXPORT int cccc_model_slot_length(void* m, int slot) { return ((LanguageModel*)m)->cache().length(slot); }
 
+namespace
+{
 // n_entries entries: slot[e], n_tokens[e] of `tokens`, n_want[e] of `want` (one entry behind the other).
-HOST_EXPORT int cccc_model_step(void* m, int n_entries, const int* slot, const int* n_tokens, const int* tokens, const int* n_want, const int* want,
-    float* logits, int* choice)
+std::vector<StepEntry> entriesOf(int n_entries, const int* slot, const int* n_tokens, const int* tokens, const int* n_want, const int* want)
 {
     std::vector<StepEntry> entries((size_t)n_entries);
     for (int e = 0; e < n_entries; e++)
@@ -88,8 +89,22 @@ HOST_EXPORT int cccc_model_step(void* m, int n_entries, const int* slot, const i
         tokens += n_tokens[e];
         want += n_want[e];
     }
-    return ((LanguageModel*)m)->step(entries, logits, choice);
+    return entries;
 }
+}    // namespace
+
+HOST_EXPORT int cccc_model_step(void* m, int n_entries, const int* slot, const int* n_tokens, const int* tokens, const int* n_want, const int* want,
+    float* logits, int* choice)
+{
+    return ((LanguageModel*)m)->step(entriesOf(n_entries, slot, n_tokens, tokens, n_want, want), logits, choice);
+}
+// The same in two halves (LanguageModel::begin, end): logits and choice of begin say whether end will take them.
+HOST_EXPORT int cccc_model_step_begin(void* m, int n_entries, const int* slot, const int* n_tokens, const int* tokens, const int* n_want, const int* want,
+    int logits, int choice)
+{
+    return ((LanguageModel*)m)->begin(entriesOf(n_entries, slot, n_tokens, tokens, n_want, want), logits != 0, choice != 0);
+}
+HOST_EXPORT int cccc_model_step_end(void* m, float* logits, int* choice) { return ((LanguageModel*)m)->end(logits, choice); }
 
 HOST_EXPORT float cccc_model_time_step(void* m, int entries, int tokens, int context, int inner, int repeat)
 {

@@ -67,37 +67,33 @@ public:
             longest = std::max(longest, entries[e].tokens.size());
         }
         if (longest > 1 && step_.promptTokens() > 0) { return prompts(entries, first, logits, choice); }
-        std::vector<uint16_t> row(logits ? (size_t)batch_ * vocab_ : 0);
-        for (size_t i = 0; i < longest; i++)    // the i-th tokens of all entries that have one
+        // one token of all entries that have one after the other; the graph of a step takes them all
+        for (size_t i = 0; i < longest; i++)
         {
-            std::vector<int> ids, pos, slot, next;
-            std::vector<size_t> owner;
-            bool any = false;
-            for (size_t e = 0; e < entries.size(); e++)
-            {
-                if (i >= entries[e].tokens.size()) { continue; }
-                ids.push_back(entries[e].tokens[i]);
-                slot.push_back(entries[e].slot);
-                pos.push_back(cache().length(entries[e].slot));
-                owner.push_back(e);
-                any = any || std::count(entries[e].want.begin(), entries[e].want.end(), (int)i);
-            }
-            next.resize(ids.size());
-            if (step_.step(ids.data(), pos.data(), (int)ids.size(), next.data(), nullptr, logits && any ? row.data() : nullptr, slot.data()) != 0) { return 1; }
-            launches_ += step_.lastLaunches();
-            for (size_t k = 0; k < owner.size(); k++)
-            {
-                const StepEntry& E = entries[owner[k]];
-                cache().setLength(E.slot, pos[k] + 1);
-                for (size_t w = 0; w < E.want.size(); w++)
-                {
-                    if (E.want[w] != (int)i) { continue; }
-                    if (choice) { choice[first[owner[k]] + w] = next[k]; }
-                    if (logits) { widen(row.data() + k * vocab_, logits + (first[owner[k]] + w) * vocab_); }
-                }
-            }
+            int rc = launch(entries, i, logits != nullptr);
+            if (rc == 0) { rc = finish(entries, i, first, logits, choice); }
+            if (rc != 0) { return 1; }
         }
         return 0;
+    }
+
+    int begin(std::vector<StepEntry> entries, bool logits, bool choice) override
+    {
+        const int rc = LanguageModel::begin(std::move(entries), logits, choice);
+        started_ = rc == 0 && !held_.empty();
+        for (const auto& e : held_) { started_ = started_ && e.tokens.size() == 1; }
+        if (!started_) { return rc; }
+        launches_ = 0;
+        started_rc_ = launch(held_, 0, logits);
+        return 0;
+    }
+    int end(float* logits, int* choice) override
+    {
+        if (!started_) { return step(held_, logits, choice); }
+        started_ = false;
+        std::vector<size_t> first(held_.size());
+        for (size_t e = 1; e < held_.size(); e++) { first[e] = first[e - 1] + held_[e - 1].want.size(); }
+        return started_rc_ == 0 && finish(held_, 0, first, logits, choice) == 0 ? 0 : 1;
     }
 
 private:
@@ -147,13 +143,48 @@ private:
         }
     }
 
-    void widen(const uint16_t* row, float* out) const
+    // The i-th tokens of the entries that have one, as one step.
+    int launch(const std::vector<StepEntry>& entries, size_t i, bool logits)
     {
-        for (int v = 0; v < vocab_; v++)
+        std::vector<int> ids, pos, slot;
+        bool any = false;
+        for (const auto& e : entries)
         {
-            const uint32_t u = (uint32_t)row[v] << 16;
-            std::memcpy(out + v, &u, 4);
+            if (i >= e.tokens.size()) { continue; }
+            ids.push_back(e.tokens[i]);
+            slot.push_back(e.slot);
+            pos.push_back(cache().length(e.slot));
+            any = any || std::count(e.want.begin(), e.want.end(), (int)i);
         }
+        return step_.launch(ids.data(), pos.data(), (int)ids.size(), logits && any, slot.data());
+    }
+    int finish(const std::vector<StepEntry>& entries, size_t i, const std::vector<size_t>& first, float* logits, int* choice)
+    {
+        std::vector<int> next(entries.size());
+        if (step_.finish(next.data(), nullptr) != 0) { return 1; }
+        launches_ += step_.lastLaunches();
+        size_t k = 0;
+        for (size_t e = 0; e < entries.size(); e++)
+        {
+            const StepEntry& E = entries[e];
+            if (i >= E.tokens.size()) { continue; }
+            cache().setLength(E.slot, cache().length(E.slot) + 1);
+            for (size_t w = 0; w < E.want.size(); w++)
+            {
+                if (E.want[w] != (int)i) { continue; }
+                if (choice) { choice[first[e] + w] = next[k]; }
+                if (logits) { widen(step_.hostLogits() + k * vocab_, logits + (first[e] + w) * vocab_); }
+            }
+            k++;
+        }
+        return 0;
+    }
+
+    // a BF16 number is the upper half of a float (vectorised: a row of logits is on the way of every step)
+    __attribute__((optimize("O3"))) void widen(const uint16_t* __restrict row, float* __restrict out) const
+    {
+        uint32_t* __restrict bits = (uint32_t* __restrict)(void*)out;
+        for (int v = 0; v < vocab_; v++) { bits[v] = (uint32_t)row[v] << 16; }
     }
 
     static bool fail(std::string* err, const std::string& what)
@@ -164,6 +195,8 @@ private:
     GpuControl gpu_;
     DecodeStep step_;
     int vocab_ = 0, batch_ = 1, launches_ = 0;
+    bool started_ = false;    // between begin() and end(): the step is under way (started_rc_ 0) or could not be started
+    int started_rc_ = 0;
 };
 
 const bool g_registered = ModelRegistry::add("cccc-llm", [](const ModelOptions& o, const Json& config, std::string* err) {

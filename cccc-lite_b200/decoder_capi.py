@@ -52,6 +52,7 @@ SYMBOLS = {
     "cuda_b200_gather_rows": (_i, [_i, _vp, _u, _vp, _vp, _u, _u, _u, _vp, _u]),
     "cuda_b200_argmax_f32": (_i, [_vp, _u, _u, _u, _vp, _vp, _vp, _u]),
     "cuda_b200_decoder_check": (_i, [C.c_char_p]),
+    "cuda_b200_decoder_status": (_i, [_vp, _vp]),
     "cuda_b200_decoder_launches": (C.c_ulonglong, []),
 }
 _lib = None

@@ -26,6 +26,8 @@ SYMBOLS = {
     "cccc_model_close_slot": (None, [_vp, _i]),
     "cccc_model_slot_length": (_i, [_vp, _i]),
     "cccc_model_step": (_i, [_vp, _i, _ip, _ip, _ip, _ip, _ip, _fp, _ip]),
+    "cccc_model_step_begin": (_i, [_vp, _i, _ip, _ip, _ip, _ip, _ip, _i, _i]),
+    "cccc_model_step_end": (_i, [_vp, _fp, _ip]),
     "cccc_model_time_step": (_f, [_vp, _i, _i, _i, _i, _i]),
     "cccc_model_generate": (_i, [_vp, _ip, _i, _ip, _f, _i, _f, _f, _ip, _i, _u, _i, _i, _ip, _i, _ip]),
     "cccc_model_generate_many": (_i, [_vp, _i, _ip, _ip, _f, _i, _f, _f, _ip, _i, _ip, _i, _u, _i, _i, _ip, _ip]),
@@ -98,12 +100,17 @@ class Model:
         """entries: (slot, tokens, want) triples.  Returns (logits, choices): a float array of wanted * vocab values and the
         ids of the largest logits, in the order of the entries and of their wanted places (None where not asked for)."""
         wanted = sum(len(w) for _, _, w in entries)
-        lg = array("f", bytes(4 * wanted * self.vocab)) if logits else None
-        ch = (C.c_int * max(1, wanted))() if choice else None
-        lp = (C.c_float * len(lg)).from_buffer(lg) if logits and wanted else None
-        rc = self.lib.cccc_model_step(self.h, len(entries), _ints(s for s, _, _ in entries), _ints(len(t) for _, t, _ in entries),
-                                      _ints(x for _, t, _ in entries for x in t), _ints(len(w) for _, _, w in entries),
-                                      _ints(x for _, _, w in entries for x in w), lp, ch)
+        lg = ch = lp = None
+        rc = self.lib.cccc_model_step_begin(self.h, len(entries), _ints(s for s, _, _ in entries), _ints(len(t) for _, t, _ in entries),
+                                            _ints(x for _, t, _ in entries for x in t), _ints(len(w) for _, _, w in entries),
+                                            _ints(x for _, _, w in entries for x in w), bool(logits and wanted), bool(choice))
+        if rc == 0:
+            try:    # the step is under way: the pages of its results are made meanwhile
+                lg = array("f", (0.0,)) * (wanted * self.vocab) if logits else None
+                ch = (C.c_int * max(1, wanted))() if choice else None
+                lp = (C.c_float * len(lg)).from_buffer(lg) if logits and wanted else None
+            finally:
+                rc = self.lib.cccc_model_step_end(self.h, lp, ch)
         if rc != 0:
             raise RuntimeError("the step's entries cannot run" if rc == -1 else "a step failed")
         return lg, (list(ch[:wanted]) if choice else None)

@@ -234,5 +234,9 @@ C_EXPORT int cuda_b200_argmax_f32(const void* logits, unsigned int rows, unsigne
 
 /* Device sync and report; the status word of this library's bounded waits is included.  0 = clean. */
 C_EXPORT int cuda_b200_decoder_check(const char* label);
+/* Enqueues a copy of the status word that decoder_check looks at to `host` (one pinned unsigned int) on `stream`: after a
+ * synchronisation with the stream, zero means that no bounded wait ran out, without another round trip to the device; anything
+ * else is for decoder_check to report and clear.  Returns 0 or 1 (CUDA error). */
+C_EXPORT int cuda_b200_decoder_status(void* host, void* stream);
 /* Kernels launched by this library in the calling process. */
 C_EXPORT unsigned long long cuda_b200_decoder_launches(void);

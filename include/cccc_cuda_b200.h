@@ -46,6 +46,11 @@ C_EXPORT int cuda_float_to_fp4_blockscale(const void* src, void* dst_nibbles, vo
  * that ran out); 0 = clean. */
 C_EXPORT int cuda_check_error(const char* label);
 
+/* Enqueues a copy of this device's status word, which cuda_check_error looks at, to `host` (one pinned unsigned int) on
+ * `stream`: after a synchronisation with the stream, zero means that no bounded wait ran out, without another round trip to the
+ * device; anything else is for cuda_check_error to report and clear.  Returns 0 or 1 (CUDA error). */
+C_EXPORT int cuda_b200_status(void* host, void* stream);
+
 /* Replaces cuda_clear_last_error, cuda_functions.h:198 (cuda_functions.cu:42-45). */
 C_EXPORT void cuda_clear_last_error(void);
 

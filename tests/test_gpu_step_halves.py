@@ -1,0 +1,55 @@
+"""A step in two halves (cccc_model_step_begin / _end, what serve.Model.step calls) against the step in one, which it has the bits
+of: decode steps that are started ahead, steps that are not (prompts, entries without wants), results that are not taken."""
+import ctypes as C
+import json
+
+import numpy as np
+import pytest
+
+from __graft_entry__ import load_package
+from oracle import fakilorn as F
+from tests.test_gpu_fakilorn import CONFIGS, tokens_for
+
+pytestmark = pytest.mark.gpu
+
+
+def ints(values):
+    values = list(values)
+    return (C.c_int * max(1, len(values)))(*values)
+
+
+def flat(entries):
+    return (len(entries), ints(s for s, _, _ in entries), ints(len(t) for _, t, _ in entries), ints(x for _, t, _ in entries for x in t),
+            ints(len(w) for _, _, w in entries), ints(x for _, _, w in entries for x in w))
+
+
+# rows of the four pieces that go to the host one after the other: fewer, as many, uneven
+@pytest.mark.parametrize("n", [1, 3, 4, 9])
+def test_the_halves_give_the_bits_of_the_whole(tmp_path, n):
+    c = CONFIGS["odd"]
+    (tmp_path / "config.json").write_text(json.dumps(c))
+    F.write_safetensors(str(tmp_path / "model.safetensors"), F.random_weights(c, seed=5))
+    serve = load_package().serve
+    a, b = (serve.Model(str(tmp_path), max_context=64, max_sequences=9) for _ in range(2))
+    V, slots = a.vocab, [(a.open_slot(), b.open_slot()) for _ in range(n)]
+    assert all(x == y for x, y in slots)
+    slots = [x for x, _ in slots][::-1]    # entries in another order than their slots
+    steps = [[(s, tokens_for(c, 3 + s, s), [2 + s, 0]) for s in slots]]
+    steps += [[(s, tokens_for(c, 1, 100 * i + s), [0]) for s in slots] for i in range(4)]
+    steps += [[(s, tokens_for(c, 1, s), [] if s % 2 else [0]) for s in slots], [(s, tokens_for(c, 1 + s % 2, s), [0]) for s in slots]]
+    for i, e in enumerate(steps):
+        wanted = sum(len(w) for _, _, w in e)
+        want, ids = np.zeros((wanted, V), np.float32), ints([0] * wanted)
+        assert a.lib.cccc_model_step(a.h, *flat(e), want.ctypes.data_as(C.POINTER(C.c_float)), ids) == 0
+        got, chosen = b.step(e, logits=i != 3, choice=i != 4)
+        assert (got is None) == (i == 3) and (got is None or np.array_equal(np.frombuffer(got, np.float32).reshape(wanted, V), want))
+        assert chosen is None if i == 4 else chosen == list(ids[:wanted])
+        assert [b.slot_length(s) for s in slots] == [a.slot_length(s) for s in slots]
+    # begun, and its results not taken: the next step does not see any of it
+    e = steps[1]
+    assert b.lib.cccc_model_step_begin(b.h, *flat(e), 1, 0) == 0 and b.lib.cccc_model_step_end(b.h, None, None) == 0
+    a.step(e)
+    assert np.array_equal(np.array(a.step(steps[2])[0]), np.array(b.step(steps[2])[0]))
+    # entries that cannot run: nothing to end
+    assert b.lib.cccc_model_step_begin(b.h, *flat([(slots[0], [c["vocab"]], [0])]), 1, 0) == -1
+    a.close(), b.close()
