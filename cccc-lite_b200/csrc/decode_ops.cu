@@ -2,7 +2,7 @@
 // RoPE, embedding gather, SwiGLU, and attention of one new token per sequence over a BF16 KV cache
 // with the q/k norms, RoPE and the cache append folded into its prologue.
 #include "common.cuh"
-#include "decode_ops.cuh"
+#include "attn_decode.cuh"
 #include "../../include/cccc_cuda_b200.h"
 
 #include <atomic>
@@ -104,73 +104,6 @@ __global__ void __launch_bounds__(256) swiglu_bf16_kernel(const uint16_t* __rest
     }
 }
 
-// ---- attention ---------------------------------------------------------------------------------------
-// Grid (S, Hkv, B), clusters of S CTAs along x: the S splits of one (sequence, kv head) exchange
-// their softmax statistics and partial outputs through distributed shared memory.
-template <int G, int HD>
-__global__ void __launch_bounds__(kTeam, (G <= 4 ? 2 : 1)) attn_decode_kernel(const AttnDecodeParams p, unsigned int ts_cap)
-{
-    extern __shared__ __align__(16) float at_smem[];
-    cg::cluster_group cluster = cg::this_cluster();
-    AttnSmem<G, HD> sm(at_smem, ts_cap);
-    uint4* ring = reinterpret_cast<uint4*>(sm.red);    // the reduction buffer is idle while the K and V passes run
-    const unsigned int tid = threadIdx.x;
-    const unsigned int S = gridDim.x, rank = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
-    pdl_launch_dependents();
-    pdl_wait();
-    const int pos_i = p.pos[b];
-    const unsigned int pos = pos_i < 0 ? 0u : (unsigned int)pos_i;
-    const unsigned int T = min(pos + 1u, p.T_max);
-    unsigned int ts = (T + S - 1) / S;
-    ts = (ts + 31u) & ~31u;
-    const unsigned int t0 = min(rank * ts, T), t1 = min(t0 + ts, T);
-    const bool owner = pos >= t0 && pos < t1;
-    attn_scores<G, HD, 4, true>(p, sm, b, kvh, t0, t1, ts_cap, pos, owner, tid, ring);    // (runs the prologue too)
-    cluster.sync();
-    attn_pv<G, HD, true>(p, sm, b, kvh, t0, t1, ts_cap, owner ? pos : 0xFFFFFFFFu, tid, [&]() {
-        // One thread per (head, split) fetches that split's (max, sum) over distributed shared memory in a single
-        // round trip; the S lanes of a head then pass their pairs to the head's first lane, which combines them in
-        // split order (the order a serial loop over the splits would use, so the bits do not depend on S's layout).
-        const unsigned int lanes = G * S;    // <= 128: G <= 8, S <= 16
-        if (tid < ((lanes + 31u) & ~31u))
-        {
-            const unsigned int g = tid / S, r = tid % S;
-            float m = -INFINITY, l = 0.f;
-            if (tid < lanes)
-            {
-                const float* ml = cluster.map_shared_rank(sm.ml, r);
-                m = ml[2 * g];
-                l = ml[2 * g + 1];
-            }
-            float gmax = -INFINITY, L = 0.f;
-            const unsigned int lane = tid & 31u, first = lane - r;    // S divides 32, so a head's lanes share a warp
-            for (unsigned int j = 0; j < S; j++) { gmax = fmaxf(gmax, __shfl_sync(0xFFFFFFFFu, m, first + j)); }
-            for (unsigned int j = 0; j < S; j++)
-            {
-                const float mj = __shfl_sync(0xFFFFFFFFu, m, first + j), lj = __shfl_sync(0xFFFFFFFFu, l, first + j);
-                if (lj > 0.f) { L += lj * __expf(mj - gmax); }
-            }
-            if (tid < lanes && r == 0)
-            {
-                sm.gl[2 * g] = gmax;
-                sm.gl[2 * g + 1] = 1.0f / L;
-            }
-        }
-    }, ring);
-    cluster.sync();
-    if (rank == 0)
-    {
-        uint16_t* o = p.out + (size_t)b * p.ldo + (size_t)kvh * G * HD;
-        for (unsigned int i = tid; i < G * HD; i += kTeam)
-        {
-            float s = 0.f;
-            for (unsigned int r = 0; r < S; r++) { s += cluster.map_shared_rank(sm.opart, r)[i]; }
-            o[i] = bf16_bits(s);
-        }
-    }
-    cluster.sync();    // the other splits keep their shared memory alive until split 0 has read it
-}
-
 // ---- q/k norm, RoPE and cache append of many tokens ----------------------------------------------------
 // One warp per (token, head); heads 0 .. H-1 are queries, then Hkv keys, then Hkv values.  Lane l holds the elements l, l + 32,
 // ..: a rotation's two elements meet in one lane, and the squares are added in the order of team_sum_squares, so that a row
@@ -236,76 +169,87 @@ __global__ void __launch_bounds__(256) attn_append_kernel(const AttnDecodeParams
     }
 }
 
-static unsigned int attn_ts_cap(unsigned int T_max, unsigned int S) { return (((T_max + S - 1) / S) + 31u) & ~31u; }
+// Splits of a (sequence, kv head), from a model fitted to measurements (4096 rows, 8 kv heads): the clusters run in rounds on the
+// slots of the GPU, three CTAs per SM in eight GPCs of whole clusters; a round of n CTAs takes 4 ns and the larger of 14 ns (a
+// CTA's own pace) and 0.08 n ns (HBM) per row of a split, and 5 us; a cluster takes 0.15 us per member to meet.  Hence as many
+// splits as still run in one round, and more rounds only where one would leave slots empty for long.  Measured (us, split
+// counts): 8 sequences 4: 35.5, 6: 30.4 (384 CTAs), 7: 45.7; 16 sequences 2: 59.0, 3: 50.8, 4: 71.3; 32 sequences 1: 103.9,
+// 2: 125.2, 3: 97.7, 5: 121.1; one sequence 8: 15.4, 16: 12.6.
+static unsigned int attn_splits(unsigned long long units, unsigned int T_max, int sm_count)
+{
+    unsigned int best = 1;
+    float least = INFINITY;
+    for (unsigned int S = 1; S <= (unsigned int)AD_MAX_SPLITS; S = S < 8 ? S + 1 : S + 8)
+    {
+        if (S > 1 && T_max / S < 64u) { break; }
+        const unsigned long long slots = (3ull * ((unsigned)sm_count / 8) / S) * S * 8;
+        const float rows = (float)((T_max + S - 1) / S);
+        if (slots == 0) { break; }
+        if (S > 8 && units * S > slots) { break; }
+        auto round = [&](unsigned long long n) { return n == 0 ? 0.f : rows * (4.f + fmaxf(14.f, 0.08f * (float)n)) + 5000.f; };
+        const float cost = (float)(units * S / slots) * round(slots) + round(units * S % slots) + 150.f * (float)S;
+        if (cost < least)
+        {
+            least = cost;
+            best = S;
+        }
+    }
+    return best;
+}
 
 template <int G, int HD>
 static int launch_attn(const AttnDecodeParams& p, int sm_count, int max_smem, cudaStream_t stream, bool pdl)
 {
+    // Caches beyond what sixteen splits with their scores as floats in shared memory could hold were never served: callers take
+    // their own path then, and still do.
+    if ((attn_smem_floats<G, HD>(((p.T_max + 15u) / 16u + 31u) & ~31u) + (G < 4 ? (4 - G) * 2048 : 0)) * sizeof(float) > (size_t)max_smem) { return -1; }
     auto kernel = attn_decode_kernel<G, HD>;
-    // Splits per (sequence, kv head): a power of two <= 16 with at least 64 rows per split.  Two CTAs share an SM, and an
-    // SM streams fastest with both (36 against 24 GB/s), so the splits grow while the CTAs still fit two per SM
-    // (measured at 4096 rows: 4 / 8 / 16 sequences 35 -> 25, 59 -> 38, 107 -> 65 us with 256 CTAs instead of 128);
-    // between one and 1.3 CTAs per SM one more doubling of a small cluster still gains (12 / 24 sequences: 95 -> 63,
-    // 120 -> 107 us), but clusters of 16 only pay while 8 would leave half the SMs empty (2 sequences: 24 us with
-    // 8 splits, 32 with 16).
-    const unsigned long long units = (unsigned long long)p.B * p.Hkv;
-    unsigned int S = 1;
-    while (S < 8 && units * S * 2 <= 2ull * (unsigned long long)sm_count && p.T_max / (S * 2) >= 64) { S *= 2; }
-    if (S == 8 && units * S * 2 <= (unsigned long long)sm_count + 20 && p.T_max / (S * 2) >= 64) { S = 16; }
-    if (S <= 2 && units * S * 10 <= 13ull * (unsigned long long)sm_count && p.T_max / (S * 2) >= 64) { S *= 2; }
-    auto smem_bytes = [](unsigned int ts_cap) { return attn_smem_floats<G, HD>(ts_cap) * sizeof(float); };
-    while (S < 16 && smem_bytes(attn_ts_cap(p.T_max, S)) > (size_t)max_smem) { S *= 2; }
-    static std::atomic<int> max_cluster{ 0 };    // largest cluster size this kernel can be scheduled with (0 = not probed)
-    for (;;)
+    unsigned int S = attn_splits((unsigned long long)p.B * p.Hkv, p.T_max, sm_count);
+    auto row_cap = [&](unsigned int splits) { return ((p.T_max + splits * AD_TILE - 1) / (splits * AD_TILE)) * AD_TILE; };
+    auto smem = [&](unsigned int splits) { return sizeof(AttnDecodeSmem<G, HD>) + (size_t)G * ad_score_row(row_cap(splits)) * 2; };
+    while (S < (unsigned int)AD_MAX_SPLITS && smem(S) > (size_t)max_smem) { S = S < 8 ? S + 1 : AD_MAX_SPLITS; }
+    // (the same value from every thread)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess
+        || (S > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
     {
-        const unsigned int ts_cap = attn_ts_cap(p.T_max, S);
-        const size_t smem = smem_bytes(ts_cap);
-        if (smem > (size_t)max_smem) { return -1; }
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess
-            || (S > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
+        return report_launch("attn_decode_bf16") ? 1 : 1;
+    }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(S, p.Hkv, p.B);
+    cfg.blockDim = dim3(AD_THREADS);
+    cfg.dynamicSmemBytes = smem(S);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    static std::atomic<int> max_cluster{ 0 };    // largest cluster this kernel can be scheduled with (0 = not probed)
+    if (S > 8 && max_cluster.load(std::memory_order_relaxed) == 0)
+    {
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1)
         {
             cudaGetLastError();
-            if (S > 8)
-            {
-                S = 8;
-                continue;
-            }
-            return report_launch("attn_decode_bf16") ? 1 : 1;
+            max_cluster.store(8, std::memory_order_relaxed);
         }
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3(S, p.Hkv, p.B);
-        cfg.blockDim = dim3(kTeam);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = S;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = pdl ? 2 : 1;
-        if (S > 8 && max_cluster.load(std::memory_order_relaxed) == 0)
-        {
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1)
-            {
-                cudaGetLastError();
-                max_cluster.store(8, std::memory_order_relaxed);
-            }
-            else { max_cluster.store(16, std::memory_order_relaxed); }
-        }
-        if (S > 8 && max_cluster.load(std::memory_order_relaxed) == 8)
-        {
-            S = 8;
-            continue;
-        }
-        count_launch();
-        if (cudaLaunchKernelEx(&cfg, kernel, p, ts_cap) != cudaSuccess) { return report_launch("attn_decode_bf16") ? 1 : 1; }
-        return 0;
+        else { max_cluster.store(16, std::memory_order_relaxed); }
     }
+    if (S > 8 && max_cluster.load(std::memory_order_relaxed) == 8)
+    {
+        S = 8;
+        if (smem(S) > (size_t)max_smem) { return -1; }
+        cfg.gridDim.x = attr[0].val.clusterDim.x = S;
+        cfg.dynamicSmemBytes = smem(S);
+    }
+    count_launch();
+    if (cudaLaunchKernelEx(&cfg, kernel, p, row_cap(S)) != cudaSuccess) { return report_launch("attn_decode_bf16") ? 1 : 1; }
+    return 0;
 }
 
 struct DeviceFacts

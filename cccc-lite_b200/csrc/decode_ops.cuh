@@ -118,21 +118,6 @@ __device__ __forceinline__ size_t attn_cache_row(const AttnDecodeParams& p, unsi
     return ((size_t)(p.slot != nullptr ? (unsigned int)p.slot[b] : b) * p.Hkv + kvh) * p.T_max;
 }
 
-constexpr int kAttnRingK = 4;     // passes of 32 rows (8 KB at head_dim 128); even: the loop consumes two per turn
-constexpr int kAttnRingV = 8;     // passes of 16 rows (4 KB at head_dim 128)
-template <int HD>
-__host__ __device__ constexpr size_t attn_ring_bytes()
-{
-    return (size_t)kTeam * 16 * ((kAttnRingK * (HD / 64)) > kAttnRingV ? (kAttnRingK * (HD / 64)) : kAttnRingV);
-}
-
-// floats of the region that serves as the K / V ring during the passes and as the cross-slot reduction buffer after them
-template <int G, int HD>
-__host__ __device__ constexpr size_t attn_red_floats()
-{
-    return (size_t)(kTeam / (HD / 8)) * G * HD > attn_ring_bytes<HD>() / 4 ? (size_t)(kTeam / (HD / 8)) * G * HD : attn_ring_bytes<HD>() / 4;
-}
-
 // Shared memory of one attention team (floats): see attn_smem_floats().
 template <int G, int HD>
 struct AttnSmem
@@ -145,7 +130,7 @@ struct AttnSmem
     float* ml;      // [G][2]    this split's max and sum of exponentials
     float* gl;      // [G][2]    the sequence's max and 1/sum
     float* opart;   // [G][HD]   this split's partial output
-    float* red;     // [kSlots2][G][HD]; the K / V ring (attn_ring_bytes) lives here while the passes run
+    float* red;     // [kSlots2][G][HD]
     float* wq;      // [HD] q-norm weights, [HD] k-norm weights, [HD/2] cos row, [HD/2] sin row
     float* sc;      // [G][ts_cap] scores, then probabilities
     __device__ AttnSmem(float* base, unsigned int ts_cap)
@@ -158,7 +143,7 @@ struct AttnSmem
         gl = ml + 2 * G;
         opart = gl + 2 * G;
         red = opart + G * HD;
-        wq = red + attn_red_floats<G, HD>();
+        wq = red + kSlots2 * G * HD;
         sc = wq + 3 * HD;
         (void)ts_cap;
     }
@@ -167,20 +152,8 @@ template <int G, int HD>
 __host__ __device__ constexpr size_t attn_smem_floats(unsigned int ts_cap)
 {
     return (size_t)G * HD + HD + (size_t)(G + 1) * HD + (size_t)(G + 1) * kTeam + 4 * G + (size_t)G * HD
-        + attn_red_floats<G, HD>() + 3 * HD + (size_t)G * ts_cap;
+        + (size_t)(kTeam / (HD / 8)) * G * HD + 3 * HD + (size_t)G * ts_cap;
 }
-
-// 16-byte asynchronous copy global -> shared that bypasses L1 (cp.async.cg); `valid` false fills zeros without
-// reading.  Each thread later reads back only what it copied itself, so cp.async.wait_group is all it needs.
-__device__ __forceinline__ void cp_async16(uint4* smem_dst, const void* gmem_src, bool valid)
-{
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-    const uint32_t bytes = valid ? 16u : 0u;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem_src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __device__ __forceinline__ void unpack8(const uint4 v, float (&f)[8])
 {
@@ -336,152 +309,16 @@ __device__ __forceinline__ void attn_scores_finish(AttnSmem<G, HD>& sm, unsigned
     team_sync();
 }
 
-// The ring form of attn_scores: K rows travel global -> shared by cp.async into a ring of kAttnRingK passes (32
-// rows each) that belongs to the threads piece by piece (every thread reads back only its own 16-byte pieces, so
-// no barrier is involved), and the copy of pass i + kAttnRingK is issued right after pass i has been consumed:
-// the DRAM latency of a pass overlaps the arithmetic of the passes before it, and no registers hold data in
-// flight.  (With registers as the buffer a pass was requested and then waited for: 32 KB in flight per team only
-// between the request and its use, 0.49 of the HBM rate at 32 sequences x 4096 rows.)
-template <int G, int HD>
-__device__ __forceinline__ void attn_scores_ring(const AttnDecodeParams& p, AttnSmem<G, HD>& sm, unsigned int b, unsigned int kvh,
-    unsigned int t0, unsigned int t1, unsigned int ts_cap, unsigned int pos, bool owner, unsigned int tid, uint4* ring)
-{
-    constexpr int CPL = HD / 64;    // 16-byte pieces per lane
-    constexpr int D = kAttnRingK;
-    const unsigned int sub = tid & 7u, slot = tid >> 3;
-    const uint16_t* Kb = p.k_cache + attn_cache_row(p, b, kvh) * HD;
-    const unsigned int n_pass = t1 > t0 ? (t1 - t0 + 31u) / 32u : 0u;
-    auto issue = [&](unsigned int pass) {
-        if (pass < n_pass)
-        {
-            const unsigned int t = t0 + pass * 32 + slot;
-            const bool valid = t < t1 && !(owner && t == pos);
-            const uint16_t* row = Kb + (size_t)(valid ? t : 0) * HD;
-#pragma unroll
-            for (int c = 0; c < CPL; c++) { cp_async16(ring + ((pass % D) * CPL + c) * kTeam + tid, reinterpret_cast<const uint4*>(row) + sub + 8 * c, valid); }
-        }
-        cp_async_commit();    // a group per pass, empty past the end, so that the wait below always counts the same
-    };
-#pragma unroll
-    for (int d = 0; d < D; d++) { issue(d); }
-    attn_prologue<G, HD>(p, sm, b, kvh, pos, owner, tid);
-    float qf[G][CPL][8];
-#pragma unroll
-    for (int g = 0; g < G; g++)
-#pragma unroll
-        for (int c = 0; c < CPL; c++)
-#pragma unroll
-            for (int e = 0; e < 8; e++) { qf[g][c][e] = sm.qs[g * HD + (sub + 8 * c) * 8 + e]; }
-    float mx[G];
-#pragma unroll
-    for (int g = 0; g < G; g++) { mx[g] = -INFINITY; }
-    // Two passes per turn of the loop: their dot-product and shuffle chains are independent and interleave.
-    for (unsigned int pass = 0; pass < n_pass; pass += 2)
-    {
-        cp_async_wait<D - 2>();    // the two oldest passes in flight have landed
-        float acc[2][G];
-#pragma unroll
-        for (int u = 0; u < 2; u++)
-        {
-            const unsigned int t = t0 + (pass + u) * 32 + slot;
-#pragma unroll
-            for (int g = 0; g < G; g++) { acc[u][g] = 0.f; }
-#pragma unroll
-            for (int c = 0; c < CPL; c++)
-            {
-                float kf[8];
-                if (owner && t == pos)
-                {
-                    // the row this call appends: taken from shared memory, not re-read from the cache
-#pragma unroll
-                    for (int e = 0; e < 8; e++) { kf[e] = sm.kn[(sub + 8 * c) * 8 + e]; }
-                }
-                else { unpack8(ring[(((pass + u) % D) * CPL + c) * kTeam + tid], kf); }
-#pragma unroll
-                for (int g = 0; g < G; g++)
-#pragma unroll
-                    for (int e = 0; e < 8; e++) { acc[u][g] = __fmaf_rn(kf[e], qf[g][c][e], acc[u][g]); }
-            }
-        }
-        issue(pass + D);    // the two slots just read are free again
-        issue(pass + D + 1);
-        // The 2 G partial sums of the eight lanes of a row are reduce-scattered: each step halves what a lane
-        // keeps and adds its partner's half (7 shuffles for 8 values where an all-reduce of each takes 24), so
-        // that lane `sub` ends with the finished sum number `sub` (mod the count) and rounds, stores and tracks
-        // the maximum of that one score only.
-        constexpr int NV = 2 * G;
-        float v[NV];
-#pragma unroll
-        for (int i = 0; i < NV; i++) { v[i] = acc[i / G][i % G]; }
-        int idx = 0;    // index of v[0] among the original NV values
-        int cnt = NV;   // compile-time after unrolling
-#pragma unroll
-        for (int step = 4; step >= 1; step >>= 1)
-        {
-            const bool upper = (sub & (unsigned)step) != 0;
-            if (cnt > 1)
-            {
-                const int half = cnt / 2;
-#pragma unroll
-                for (int i = 0; i < NV / 2; i++)
-                {
-                    if (i < half)
-                    {
-                        const float send = upper ? v[i] : v[half + i];
-                        const float recv = __shfl_xor_sync(0xFFFFFFFFu, send, step);
-                        v[i] = (upper ? v[half + i] : v[i]) + recv;
-                    }
-                }
-                idx += upper ? half : 0;
-                cnt = half;
-            }
-            else { v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], step); }
-        }
-#pragma unroll
-        for (int i = 0; i < NV / 8 + (NV < 8 ? 1 : 0); i++)
-        {
-            if (i < cnt)
-            {
-                const int which = idx + i;    // (pass parity, head)
-                const int u = which / G, g = which % G;
-                const unsigned int t = t0 + (pass + u) * 32 + slot;
-                if (t < t1)
-                {
-                    const float sc = bf16_round(__fmul_rn(p.scale, v[i]));
-                    sm.sc[g * ts_cap + (t - t0)] = sc;
-#pragma unroll
-                    for (int gg = 0; gg < G; gg++)
-                    {
-                        if (gg == g) { mx[gg] = fmaxf(mx[gg], sc); }
-                    }
-                }
-            }
-        }
-    }
-    cp_async_wait<0>();
-    team_sync();    // the ring shares its memory with sm.red, which the reductions below write
-    attn_scores_finish<G, HD>(sm, t0, t1, ts_cap, tid, mx);
-}
-
 // Prologue and scores of the rows [t0, t1) of one kv head against the G rotated queries:
 // sm.sc[g][t - t0] = bf16(scale * K[t] . q_g) (the reference's BF16 score tensor, MatrixEx.cpp:3056),
 // and this split's maximum and sum of exp(score - maximum) per head in sm.ml.  Eight lanes share a
 // row (two 16-byte pieces each for HD = 128), 32 rows per pass, UNROLL passes in flight.  The first
 // batch of K rows is requested BEFORE the prologue runs: the cache does not depend on q, so the DRAM
 // latency of the first batch and the prologue's own round trip overlap.
-template <int G, int HD, int UNROLL = (G <= 4 ? 8 : 4), bool RING = false>
+template <int G, int HD, int UNROLL = (G <= 4 ? 8 : 4)>
 __device__ __forceinline__ void attn_scores(const AttnDecodeParams& p, AttnSmem<G, HD>& sm, unsigned int b, unsigned int kvh,
-    unsigned int t0, unsigned int t1, unsigned int ts_cap, unsigned int pos, bool owner, unsigned int tid, uint4* ring = nullptr)
+    unsigned int t0, unsigned int t1, unsigned int ts_cap, unsigned int pos, bool owner, unsigned int tid)
 {
-    // RING is a compile-time choice: a kernel carries only the form it uses (the stand-alone kernel runs its code
-    // once per launch, and what bounds it at one sequence is instruction fetch)
-    if constexpr (RING)
-    {
-        attn_scores_ring<G, HD>(p, sm, b, kvh, t0, t1, ts_cap, pos, owner, tid, ring);
-        return;
-    }
-    else
-    {
     constexpr int CPL = HD / 64;    // 16-byte pieces per lane
     const unsigned int sub = tid & 7u, slot = tid >> 3;
     const uint16_t* Kb = p.k_cache + attn_cache_row(p, b, kvh) * HD;
@@ -553,7 +390,6 @@ __device__ __forceinline__ void attn_scores(const AttnDecodeParams& p, AttnSmem<
         }
     }
     attn_scores_finish<G, HD>(sm, t0, t1, ts_cap, tid, mx);
-    }
 }
 
 // Probabilities and P*V for the rows [t0, t1): p = bf16(exp(score - max) / sum) with the
@@ -561,9 +397,9 @@ __device__ __forceinline__ void attn_scores(const AttnDecodeParams& p, AttnSmem<
 // opart[g][d] = sum_t V[t][d] * p[g][t] in FP32.  HD/8 lanes share a row (16 bytes each).
 // `stats` produces the sequence-wide (max, 1/sum) into sm.gl; it runs AFTER the first batch of V
 // rows has been requested, because V does not depend on it.
-template <int G, int HD, bool RING = false, class Stats>
+template <int G, int HD, class Stats>
 __device__ __forceinline__ void attn_pv(const AttnDecodeParams& p, AttnSmem<G, HD>& sm, unsigned int b, unsigned int kvh,
-    unsigned int t0, unsigned int t1, unsigned int ts_cap, unsigned int pos_row, unsigned int tid, Stats stats, uint4* ring = nullptr)
+    unsigned int t0, unsigned int t1, unsigned int ts_cap, unsigned int pos_row, unsigned int tid, Stats stats)
 {
     constexpr int LPR = HD / 8;             // lanes per row
     constexpr int SLOTS = kTeam / LPR;      // rows per pass
@@ -571,83 +407,6 @@ __device__ __forceinline__ void attn_pv(const AttnDecodeParams& p, AttnSmem<G, H
     const unsigned int n = t1 > t0 ? t1 - t0 : 0;
     const unsigned int sub = tid % LPR, slot = tid / LPR;
     const uint16_t* Vb = p.v_cache + attn_cache_row(p, b, kvh) * HD;
-    if constexpr (RING)
-    {
-        // The ring form (see attn_scores_ring): V rows by cp.async, kAttnRingV passes of SLOTS rows in flight, the first
-        // ones requested before the statistics are exchanged.
-        constexpr int D = kAttnRingV;
-        const unsigned int n_pass = (n + SLOTS - 1) / SLOTS;
-        auto issue = [&](unsigned int pass) {
-            if (pass < n_pass)
-            {
-                const unsigned int t = t0 + pass * SLOTS + slot;
-                const bool valid = t < t1;
-                // the row this call appended comes from the projection output, not back from the cache
-                const uint16_t* vrow = t == pos_row ? p.v + (size_t)b * p.ldv + (size_t)kvh * HD : Vb + (size_t)(valid ? t : 0) * HD;
-                cp_async16(ring + (pass % D) * kTeam + tid, reinterpret_cast<const uint4*>(vrow) + sub, valid);
-            }
-            cp_async_commit();
-        };
-#pragma unroll
-        for (int d = 0; d < D; d++) { issue(d); }
-        stats();
-        team_sync();
-#pragma unroll
-        for (int g = 0; g < G; g++)
-        {
-            const float m = sm.gl[2 * g], inv = sm.gl[2 * g + 1];
-            for (unsigned int i = tid; i < n; i += kTeam)
-            {
-                sm.sc[g * ts_cap + i] = bf16_round(__fmul_rn(__expf(sm.sc[g * ts_cap + i] - m), inv));
-            }
-        }
-        team_sync();
-        float acc[G][8];
-#pragma unroll
-        for (int g = 0; g < G; g++)
-#pragma unroll
-            for (int e = 0; e < 8; e++) { acc[g][e] = 0.f; }
-        for (unsigned int pass = 0; pass < n_pass; pass += 2)
-        {
-            cp_async_wait<D - 2>();
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-            {
-                const unsigned int t = t0 + (pass + u) * SLOTS + slot;
-                if (t < t1)
-                {
-                    float vf[8];
-                    unpack8(ring[((pass + u) % D) * kTeam + tid], vf);
-#pragma unroll
-                    for (int g = 0; g < G; g++)
-                    {
-                        const float pr = sm.sc[g * ts_cap + (t - t0)];
-#pragma unroll
-                        for (int e = 0; e < 8; e++) { acc[g][e] = __fmaf_rn(vf[e], pr, acc[g][e]); }
-                    }
-                }
-            }
-            issue(pass + D);
-            issue(pass + D + 1);
-        }
-        cp_async_wait<0>();
-        team_sync();    // every thread has read its last ring slot before sm.red (the same memory) is written
-#pragma unroll
-        for (int g = 0; g < G; g++)
-#pragma unroll
-            for (int e = 0; e < 8; e++) { sm.red[(slot * G + g) * HD + sub * 8 + e] = acc[g][e]; }
-        team_sync();
-        for (unsigned int i = tid; i < G * HD; i += kTeam)
-        {
-            float sacc = 0.f;
-            for (int sl = 0; sl < SLOTS; sl++) { sacc += sm.red[sl * G * HD + i]; }
-            sm.opart[i] = sacc;
-        }
-        team_sync();
-        return;
-    }
-    else
-    {
     uint4 vv[UNROLL];
     auto fetch = [&](unsigned int tb) {
 #pragma unroll
@@ -710,7 +469,6 @@ __device__ __forceinline__ void attn_pv(const AttnDecodeParams& p, AttnSmem<G, H
         sm.opart[i] = s;
     }
     team_sync();
-    }
 }
 
 }    // namespace b200
