@@ -8,7 +8,13 @@
 // for is permuted in turn, and undone when the result is stored.  The next tile's keys are requested as soon as the scores
 // are out, its values as soon as the value product is.  Softmax weights enter the value product as the sum of two BF16 numbers.
 // Decoding steps (one token per sequence) are fused: the CTA whose split holds the new position brings its key to unit
-// RMS, mixes its value and appends both; every CTA brings its own queries to unit RMS.
+// RMS, mixes its value and appends both (and takes them from shared memory itself); every CTA brings its own queries to unit RMS.
+// The splits of a unit are one cluster: each CTA stores its statistics and its share of everyone's outputs into the others' shared
+// memory, one barrier, and the shares are summed where they lie.  (Partial results through global memory, summed by the last CTA
+// to arrive at a counter, took four more round trips to L2 of a chain that is all latency at a few hundred rows: 8 sequences
+// of 250 rows, 4 kv heads, 17 us behind the projections, now 8.4.)
+#include <cooperative_groups.h>
+
 #include "attention_mma.cuh"
 
 namespace b200
@@ -42,20 +48,33 @@ __device__ __forceinline__ void mma_bf16_top(float& c0, float& c1, uint32_t a0, 
         : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// grid (splits, Hkv * row_tiles, entries)
+constexpr unsigned int kDirectSplits = 16;    // one cluster
+
+template <int DK, int DV, int RT>
+struct DirectMeet
+{
+    float om[AS_WARPS][RT * DV];
+    float ml[AS_WARPS][RT][2];                 // a warp's maximum (log2) and sum of every row
+    float recv_ml[kDirectSplits][RT][2];       // a split's
+    float recv[RT * DV + kDirectSplits];       // [split][outputs that this CTA finishes]
+    __nv_bfloat16 kn[DK], vn[DV];              // the new row (fused)
+};
+
+// grid (splits, Hkv * row_tiles, entries), clusters along x
 template <int DK, int DV, int NR>    // NR: row groups of eight (1 or 2)
 __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 2) attention_direct_kernel(const AttnParams p)
 {
     constexpr int RT = 8 * NR, KB = DK / 64, C = DV / 8, VR = C / 2;    // VR: registers of a value row per lane
-    __shared__ float om[AS_WARPS * RT * DV];
-    __shared__ SplitMeet meet;
+    __shared__ __align__(16) DirectMeet<DK, DV, RT> meet;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     grid_dependency_launch();
     grid_dependency_wait();
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const unsigned int split = blockIdx.x, kvh = blockIdx.y % p.Hkv, rt = blockIdx.y / p.Hkv, e = p.e0 + blockIdx.z;
     const unsigned int n = (unsigned int)p.n[e], start = (unsigned int)p.start[e], pos = (unsigned int)p.pos[e], r0 = rt * RT;
     const unsigned int rows = n * p.G;
-    if (r0 >= rows) { return; }
+    if (r0 >= rows) { return; }    // the whole cluster
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");    // met before the first store into a peer
     const __nv_bfloat16* qkvg = (const __nv_bfloat16*)p.qkvg;
     const size_t seq = ((size_t)p.slot[e] * p.Hkv + kvh) * p.T_max;
     __nv_bfloat16* K = (__nv_bfloat16*)p.k_cache + seq * p.k_ld;
@@ -67,8 +86,9 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
     const unsigned int tiles = (T + 15) / 16, per = (tiles - begin + p.splits - 1) / p.splits;
     const unsigned int tile0 = min(begin + split * per, tiles), tile1 = min(tile0 + per, tiles);
 
+    const bool owner = p.fused && pos < p.T_max && pos / 16 >= tile0 && pos / 16 < tile1;
     uint32_t k[2][KB][8], v[4][VR];
-    auto load_k = [&](unsigned int tile) {
+    auto load_k = [&](unsigned int tile, unsigned int skip) {
 #pragma unroll
         for (int i = 0; i < 2; i++)
         {
@@ -77,16 +97,16 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
             for (int b = 0; b < KB; b++)
             {
                 const unsigned int d = b * 64 + t * 16;
-                ldg32(K + (size_t)key * p.k_ld + d, k[i][b], tile < tile1 && key < T && d < p.k_ld);
+                ldg32(K + (size_t)key * p.k_ld + d, k[i][b], tile < tile1 && key < T && d < p.k_ld && key != skip);
             }
         }
     };
-    auto load_v = [&](unsigned int tile) {
+    auto load_v = [&](unsigned int tile, unsigned int skip) {
 #pragma unroll
         for (int i = 0; i < 4; i++)
         {
             const unsigned int key = tile * 16 + 2 * t + (i & 1) + (i >> 1) * 8, d = g * C;
-            const bool ok = tile < tile1 && key < T && d < p.v_ld;
+            const bool ok = tile < tile1 && key < T && d < p.v_ld && key != skip;
             if constexpr (VR == 8) { ldg32(V + (size_t)key * p.v_ld + d, v[i], ok); }
             else { ldg16(V + (size_t)key * p.v_ld + d, v[i], ok); }
         }
@@ -102,17 +122,22 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
             if (lane * 128 < vl && (tile + 1) * 16 <= T) { asm volatile("prefetch.global.L2 [%0];" ::"l"(vp)); }
         }
     };
-    // the step's own row is in the cache only after the append below
-    const bool owner = p.fused && pos < p.T_max && pos / 16 >= tile0 && pos / 16 < tile1;
-    const bool late = owner && tile0 + warp == pos / 16;
-    if (!late)
-    {
-        load_k(tile0 + warp);
-        load_v(tile0 + warp);
-    }
+    // the step's own row is in the cache only after the append below: a first tile takes it from shared memory
+    load_k(tile0 + warp, owner ? pos : 0xFFFFFFFFu);
+    load_v(tile0 + warp, owner ? pos : 0xFFFFFFFFu);
     prefetch(tile0 + warp + AS_WARPS);
     prefetch(tile0 + warp + 2 * AS_WARPS);
-    // (every row tile of the unit writes the same values: its own reads come after them)
+    const bool wide_q = (p.dim % 16) == 0 && (p.q_ld % 16) == 0;
+    auto q_row = [&](unsigned int r) { return qkvg + (size_t)(start + r / p.G) * p.ld + (size_t)(kvh * p.G + r % p.G) * p.q_ld; };
+    uint32_t raw[NR][KB][8];
+#pragma unroll
+    for (int h = 0; h < NR; h++)
+    {
+        const unsigned int r = r0 + g + 8 * h;
+#pragma unroll
+        for (int b = 0; b < KB; b++) { ldg32(q_row(r < rows ? r : 0) + b * 64 + t * 16, raw[h][b], wide_q && r < rows && b * 64 + t * 16 < p.dim); }
+    }
+    // (every row tile of the unit writes the same values)
     if (owner)
     {
         const __nv_bfloat16* x = qkvg + (size_t)start * p.ld;
@@ -130,27 +155,55 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
                 }
                 inv = 1.0f / sqrtf(warp_sum(sq) / (float)p.dim + p.eps);
             }
-            for (unsigned int d = lane; d < p.dim; d += 32) { K[(size_t)pos * p.k_ld + d] = __float2bfloat16_rn(__bfloat162float(src[d]) * inv); }
+            for (unsigned int d = lane; d < DK; d += 32)
+            {
+                const __nv_bfloat16 x = __float2bfloat16_rn(d < p.dim ? __bfloat162float(src[d]) * inv : 0.f);
+                meet.kn[d] = x;
+                if (d < p.dim) { K[(size_t)pos * p.k_ld + d] = x; }
+            }
         }
         else if (warp == 1)
         {
             const __nv_bfloat16* src = x + p.v_off + (size_t)kvh * p.vdim;
             __nv_bfloat16* first = p.v_mix ? (__nv_bfloat16*)p.v_first + (size_t)start * p.v_first_ld + (size_t)kvh * p.vdim : nullptr;
-            for (unsigned int d = lane; d < p.vdim; d += 32)
+            for (unsigned int d = lane; d < DV; d += 32)
             {
-                float v = __bfloat162float(src[d]);
-                if (p.v_mix == 1) { first[d] = src[d]; }
-                else if (p.v_mix == 2) { v = (1.0f - p.lambda) * v + p.lambda * __bfloat162float(first[d]); }
-                V[(size_t)pos * p.v_ld + d] = __float2bfloat16_rn(v);
+                float v = d < p.vdim ? __bfloat162float(src[d]) : 0.f;
+                if (d < p.vdim && p.v_mix == 1) { first[d] = src[d]; }
+                else if (d < p.vdim && p.v_mix == 2) { v = (1.0f - p.lambda) * v + p.lambda * __bfloat162float(first[d]); }
+                const __nv_bfloat16 x = __float2bfloat16_rn(v);
+                meet.vn[d] = x;
+                if (d < p.vdim) { V[(size_t)pos * p.v_ld + d] = x; }
             }
         }
         __syncthreads();
     }
 
-    if (late)
+    if (owner && tile0 + warp == pos / 16)
     {
-        load_k(tile0 + warp);
-        load_v(tile0 + warp);
+        const unsigned int at = pos % 16;
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+        {
+            if (at == i * 8 + g)
+            {
+#pragma unroll
+                for (int b = 0; b < KB; b++)
+                {
+#pragma unroll
+                    for (int x = 0; x < 8; x++) { k[i][b][x] = reinterpret_cast<const uint32_t*>(meet.kn + b * 64 + t * 16)[x]; }
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+        {
+            if (at == 2 * t + (i & 1) + (i >> 1) * 8)
+            {
+#pragma unroll
+                for (int x = 0; x < VR; x++) { v[i][x] = reinterpret_cast<const uint32_t*>(meet.vn + g * C)[x]; }
+            }
+        }
     }
 
     // queries: the same permuted element order as the keys
@@ -161,8 +214,7 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
     {
         const unsigned int r = r0 + g + 8 * h;
         const bool ok = r < rows;
-        const unsigned int rr = ok ? r : 0;
-        const __nv_bfloat16* src = qkvg + (size_t)(start + rr / p.G) * p.ld + (size_t)(kvh * p.G + rr % p.G) * p.q_ld;
+        const __nv_bfloat16* src = q_row(ok ? r : 0);
         low[h] = first_key(p, e, pos + r / p.G + 1);
         lim[h] = min(pos + r / p.G + 1, T);
         float f[KB][16], sq = 0.f;
@@ -170,15 +222,13 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
         for (int b = 0; b < KB; b++)
         {
             const unsigned int d0 = b * 64 + t * 16;
-            if ((p.dim % 16) == 0 && (p.q_ld % 16) == 0)
+            if (wide_q)
             {
-                uint32_t x[8];
-                ldg32(src + d0, x, ok && d0 < p.dim);
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                 {
-                    f[b][2 * j] = __uint_as_float(x[j] << 16);
-                    f[b][2 * j + 1] = __uint_as_float(x[j] & 0xFFFF0000u);
+                    f[b][2 * j] = __uint_as_float(raw[h][b][j] << 16);
+                    f[b][2 * j + 1] = __uint_as_float(raw[h][b][j] & 0xFFFF0000u);
                 }
             }
             else
@@ -241,7 +291,7 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
                 }
             }
         }
-        load_k(tile + AS_WARPS);
+        load_k(tile + AS_WARPS, 0xFFFFFFFFu);
         prefetch(tile + 3 * AS_WARPS);
         const bool masked = (tile + 1) * 16 > first_lim || tile * 16 < last_low;
         uint32_t hi[2 * NR], lo[2 * NR];    // [key half][row group]
@@ -303,7 +353,7 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
                 mma_bf16_16816(o[j], lo[0], lo[NR - 1], lo[NR], lo[2 * NR - 1], b0, b1);
             }
         }
-        load_v(tile + AS_WARPS);
+        load_v(tile + AS_WARPS, 0xFFFFFFFFu);
     }
     // n index 2t (+ 1) of fragment j is column (2t (+ 1)) * C + j
 #pragma unroll
@@ -311,7 +361,7 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
     {
         l[h] += __shfl_xor_sync(0xFFFFFFFFu, l[h], 1);
         l[h] += __shfl_xor_sync(0xFFFFFFFFu, l[h], 2);
-        float* dst = om + (warp * RT + g + 8 * h) * DV + 2 * t * C;
+        float* dst = meet.om[warp] + (g + 8 * h) * DV + 2 * t * C;
 #pragma unroll
         for (int j = 0; j < C; j++)
         {
@@ -324,15 +374,84 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
             meet.ml[warp][g + 8 * h][1] = l[h];
         }
     }
-    split_finish<DV, RT>(p, meet, om, qkvg, e, start, kvh, rt, r0, rows);
+    __syncthreads();
+
+    // ---- warps -> CTA -> the CTA of the cluster that finishes the output ----
+    const unsigned int tid = threadIdx.x, S = p.splits, live = min((unsigned int)RT, rows - r0), outputs = live * p.vdim, share = (outputs + S - 1) / S;
+    auto top = [](const float (*ml)[RT][2], unsigned int n, unsigned int r) {
+        float m = -INFINITY;
+        for (unsigned int i = 0; i < n; i++) { m = fmaxf(m, ml[i][r][0]); }
+        return m;
+    };
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");    // every CTA of the cluster runs
+    for (unsigned int i = tid; i < live * S; i += 32 * AS_WARPS)
+    {
+        const unsigned int r = i % live;
+        const float mr = top(meet.ml, AS_WARPS, r), base = mr == -INFINITY ? 0.f : mr;
+        float lr = 0.f;
+#pragma unroll
+        for (int w = 0; w < AS_WARPS; w++) { lr += exp2f(meet.ml[w][r][0] - base) * meet.ml[w][r][1]; }
+        float* to = cluster.map_shared_rank(&meet.recv_ml[split][r][0], i / live);
+        to[0] = mr;
+        to[1] = lr;
+    }
+    for (unsigned int j = tid; j < outputs; j += 32 * AS_WARPS)
+    {
+        const unsigned int r = j / p.vdim, d = j % p.vdim, to = j / share;
+        const float mr = top(meet.ml, AS_WARPS, r), base = mr == -INFINITY ? 0.f : mr;
+        float x = 0.f;
+#pragma unroll
+        for (int w = 0; w < AS_WARPS; w++) { x += exp2f(meet.ml[w][r][0] - base) * meet.om[w][r * DV + d]; }
+        *cluster.map_shared_rank(&meet.recv[split * share + (j - to * share)], to) = x;
+    }
+    cluster.sync();
+    const unsigned int first = split * share, count = first < outputs ? min(share, outputs - first) : 0u;
+    for (unsigned int i = tid; i < count; i += 32 * AS_WARPS)
+    {
+        const unsigned int r = (first + i) / p.vdim, d = (first + i) % p.vdim;
+        const float mr = top(meet.recv_ml, S, r);
+        float lr = 0.f, x = 0.f;
+        for (unsigned int c = 0; c < S; c++)
+        {
+            const float w = exp2f(meet.recv_ml[c][r][0] - mr);
+            lr += w * meet.recv_ml[c][r][1];
+            x += w * meet.recv[c * share + i];
+        }
+        if (p.sink != nullptr) { lr += exp2f(p.sink[kvh * p.G + (r0 + r) % p.G] * 1.44269504088896341f - mr); }
+        attention_store(p, qkvg, start, kvh, r0 + r, d, x / lr);
+    }
 }
 
 template <int DK, int DV>
 static int run_direct(const AttnParams& p, unsigned int entries, unsigned int nr, cudaStream_t stream, bool pdl)
 {
     const dim3 grid(p.splits, p.Hkv * p.row_tiles, entries);
-    return nr == 1 ? launch_kernel("attention_direct", attention_direct_kernel<DK, DV, 1>, grid, dim3(32 * AS_WARPS), 0, stream, pdl, p)
-                   : launch_kernel("attention_direct", attention_direct_kernel<DK, DV, 2>, grid, dim3(32 * AS_WARPS), 0, stream, pdl, p);
+    return nr == 1 ? launch_cluster("attention_direct", attention_direct_kernel<DK, DV, 1>, grid, dim3(32 * AS_WARPS), 0, p.splits, stream, pdl, p)
+                   : launch_cluster("attention_direct", attention_direct_kernel<DK, DV, 2>, grid, dim3(32 * AS_WARPS), 0, p.splits, stream, pdl, p);
+}
+
+// Splits of a unit, from a model fitted to the like kernel of the quantised models (attn_splits of decode_ops.cu, with its
+// measurements): clusters run in rounds on the slots of the GPU; a round of n CTAs takes 4 ns and the larger of 14 ns (a CTA's own
+// pace) and 0.08 n ns (HBM) per row of a split, and 5 us, and 5 more for a second one; a cluster takes 0.15 us per member to meet.
+static unsigned int direct_splits(unsigned long long units, unsigned int len, int sm_count, unsigned int ctas_per_sm)
+{
+    unsigned int best = 1;
+    float least = INFINITY;
+    for (unsigned int S = 1; S <= kDirectSplits; S = S < 8 ? S + 1 : S + 8)
+    {
+        if (S > 1 && len / S < 64u) { break; }
+        const unsigned long long slots = ((unsigned long long)ctas_per_sm * ((unsigned)sm_count / 8) / S) * S * 8;
+        if (slots == 0 || (S > 8 && units * S > (unsigned long long)sm_count)) { break; }
+        const float rows = (float)((len + S - 1) / S);
+        auto round = [&](unsigned long long n) { return n == 0 ? 0.f : rows * (4.f + fmaxf(14.f, 0.08f * (float)n)) + 5000.f; };
+        const float cost = (float)(units * S / slots) * round(slots) + round(units * S % slots) + 150.f * (float)S + (units * S > slots ? 5000.f : 0.f);
+        if (cost < least)
+        {
+            least = cost;
+            best = S;
+        }
+    }
+    return best;
 }
 
 int launch_attention_direct(const AttnParams& p0, unsigned int entries, unsigned int max_n, unsigned int max_len, cudaStream_t stream, bool pdl)
@@ -343,7 +462,10 @@ int launch_attention_direct(const AttnParams& p0, unsigned int entries, unsigned
     const unsigned int nr = max_n * p.G <= 8 ? 1 : 2;
     p.row_tiles = (max_n * p.G + 8 * nr - 1) / (8 * nr);
     if ((unsigned long long)p.Hkv * p.row_tiles > 65535ull) { return -1; }
-    if (!plan_splits(p, entries, max_n, max_len, nr == 1 && (p.dim <= 64 || p.vdim <= 64) ? 3 : 2)) { return 1; }
+    const DecoderDevice* dev = decoder_device();
+    if (!dev) { return 1; }
+    if (p.window != 0 && max_len > p.window + max_n) { max_len = p.window + max_n; }
+    p.splits = direct_splits((unsigned long long)entries * p.Hkv * p.row_tiles, max_len, dev->sm_count, nr == 1 && (p.dim <= 64 || p.vdim <= 64) ? 3 : 2);
     if (p.dim <= 64) { return p.vdim <= 64 ? run_direct<64, 64>(p, entries, nr, stream, pdl) : run_direct<64, 128>(p, entries, nr, stream, pdl); }
     return p.vdim <= 64 ? run_direct<128, 64>(p, entries, nr, stream, pdl) : run_direct<128, 128>(p, entries, nr, stream, pdl);
 }
