@@ -2,7 +2,7 @@
 // the reference selects with act_data_type = FP8_E4M3 (cccc/cublas_real.h:619-666: quantise the BF16 activations, static
 // scale or dynamic absmax, then a cublasLt FP8 x FP8 matmul with both scales).  Here the quantised activations are one
 // E4M3 row per token of the native-operand FP8 kernel (gemm_native.cuh, PIECES = 1): both operands go into
-// tcgen05.mma kind::f8f6f4 as they are.  More than 32 tokens run with k slices (gemm_w8a8_split.cuh) or on CTA pairs
+// tcgen05.mma kind::f8f6f4 as they are.  More tokens (24 and up) run with k slices (gemm_w8a8_split.cuh) or on CTA pairs
 // (gemm_w8a8_pair.cuh).
 #pragma once
 
@@ -13,7 +13,13 @@
 namespace b200
 {
 
-constexpr int W8A8_MAX_TOKENS = 32;    // up to here the streaming kernel (all SMs share the k range)
+constexpr int W8A8_MAX_TOKENS = 32;    // what the streaming kernel takes (all SMs share the k range)
+
+// Do k slices take what the streaming kernel would?  From 24 tokens on they are as fast or faster on every linear of a layer and on
+// a head (dynamic, streaming / slices, us: 4096 x 4096 at 24 / 32 tokens 16.6 / 10.7, 17.7 / 11.0; 24576 x 4096 24.7 / 24.3,
+// 25.5 / 23.8; 4096 x 12288 22.9 / 17.8, 24.3 / 18.4; 151936 x 4096 107.9 / 104.3, 109.9 / 105.8); at 17 tokens 24576 x 4096 takes
+// 24.0 / 26.0, at 16 151936 x 4096 106.4 / 122.3.  Small tensors keep the quantiser that finds the maximum itself.
+static inline bool w8a8_split_early(unsigned int M, unsigned int K) { return M >= 24 && (size_t)M * K > 16384; }
 
 // More tokens: k slices, or CTA pairs?  The line depends on tokens and k alone, so that a group of linears and the separate calls
 // take the same kernel and give the same bits.  Measured (dynamic scale, pairs' best form / slices, us): up to 64 tokens the
@@ -211,14 +217,14 @@ static __global__ void __launch_bounds__(256) quantise_activations_x8_kernel(con
 
 // The linear(s).  Returns the C-ABI code, -1 for what this path does not serve (K % 128 != 0, unaligned operands, more
 // than three members, a workspace that is too small for the quantised activations).  pair_fh: form of the launch
-// for more than 32 tokens (0: chosen here, 1 .. 3: of the pair kernels, 4: the k slices).
+// for many tokens (0: chosen here, 1 .. 3: of the pair kernels, 4: the k slices).
 // x_is_e4m3: X holds E4M3 bytes (ldx in bytes) whose multiplier back is act_scale (> 0); y_e4m3: Y receives E4M3 bytes.
 static int launch_w8a8(const GemvScratch* ws, const W8A8Member* mem, unsigned int count, const void* X, float act_scale, unsigned int M,
     unsigned int K, unsigned int ldx, cudaStream_t stream, unsigned int flags, bool x_is_e4m3 = false, bool y_e4m3 = false, unsigned int pair_fh = 0)
 {
     if (count == 0 || count > (unsigned int)PF_MAX_GROUP || M == 0 || M > 65535u || act_scale < 0.f) { return -1; }
     if (pair_fh > 4) { pair_fh &= 3u; }
-    const bool big = M > (unsigned int)W8A8_MAX_TOKENS;
+    const bool big = M > (unsigned int)W8A8_MAX_TOKENS || pair_fh == 4 || (pair_fh == 0 && w8a8_split_early(M, K));
     if (x_is_e4m3 && !(act_scale > 0.f)) { return -1; }
     const unsigned int bnp = big ? M : (M <= 16 ? 16u : 32u);    // rows the quantiser writes
     NativeParams np;

@@ -1,4 +1,4 @@
-// W8A8 linear for a few dozen tokens and more than the streaming kernel's 32: E4M3 weights x E4M3 activations (tcgen05.mma
+// W8A8 linear for two dozen tokens and more: E4M3 weights x E4M3 activations (tcgen05.mma
 // kind::f8f6f4), a CTA per 128 output features and k slice.
 //
 // At these sizes the weights are the work: 4096 x 4096 is 16 MB, 2.6 us of HBM, whatever the 64 tokens cost.  The CTA pairs of

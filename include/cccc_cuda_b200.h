@@ -133,7 +133,7 @@ C_EXPORT int cuda_gemm_wq_bf16_group(int w_type, unsigned int count, const cuda_
  *   act_scale == 0: dynamic, one absmax over the whole [M_tokens, K] tensor, q = e4m3(x * 448 / absmax), multiplier back
  *                   absmax / 448 (cccc-cuda/cuda_functions.cu:2611-2669);
  * and Y = alpha * w_inv_scale * multiplier * (W . q) + beta * Y (BF16, or float32 with flags bit 2; bit 3 and bit 0 as
- * cuda_gemm_wq_bf16).  Both operands go into tcgen05.mma kind::f8f6f4 unchanged: up to 32 tokens in a kernel that
+ * cuda_gemm_wq_bf16).  Both operands go into tcgen05.mma kind::f8f6f4 unchanged: up to 23 tokens in a kernel that
  * streams the weights once over all SMs, above that with k slices as clusters (flags bits 8-10 = 4 force that form for
  * tests) or on CTA pairs (cta_group::2; 256- or 512-feature tiles, or a persistent form whose epilogue overlaps the next
  * tile; bits 8-9 = 1 / 2 / 3 force one of them, 0 lets the shape decide).  Needs K % 128 == 0, ldw % 16 == 0, ldx % 8 == 0, 16-byte aligned W and X, at most 65535 tokens

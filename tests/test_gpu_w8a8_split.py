@@ -1,4 +1,4 @@
-"""W8A8 with k slices (up to 64 tokens by default, more where k is long; flags bits 8-10 = 4 take it above 32 tokens) against the
+"""W8A8 with k slices (24 to 64 tokens by default, more where k is long; flags bits 8-10 = 4 take it at any count) against the
 CPU oracle, and the rule that the result does not depend on how many CTAs share the k range."""
 import numpy as np
 import pytest
@@ -22,6 +22,15 @@ def test_matches_the_oracle(N, K, M, act_scale, flags):
     W, _, w_inv, X = O.make_inputs(O.FP8_E4M3, N, K, M, seed=N + M, scaled=True)
     y32, _, _ = O.linear_w8a8(W, w_inv, X, N, M, K, act_scale=act_scale)
     assert_close(O.bf16_bits_to_f32(run(W, w_inv, X, act_scale, N, M, K, flags=flags)).reshape(M, N), y32, (N, K, M, act_scale))
+
+
+# the line at 24 tokens, and at 16384 activations (below, the quantiser finds the maximum itself and the streaming kernel runs)
+@pytest.mark.parametrize("act_scale", [0.0, 0.0123])
+@pytest.mark.parametrize("N,K,M", [(1000, 1024, 23), (1000, 1024, 24), (640, 4096, 31), (300, 640, 25), (300, 768, 25), (129, 512, 32), (129, 640, 32)])
+def test_the_line_below_32_tokens(N, K, M, act_scale):
+    W, _, w_inv, X = O.make_inputs(O.FP8_E4M3, N, K, M, seed=N + M, scaled=True)
+    y32, _, _ = O.linear_w8a8(W, w_inv, X, N, M, K, act_scale=act_scale)
+    assert_close(O.bf16_bits_to_f32(run(W, w_inv, X, act_scale, N, M, K)).reshape(M, N), y32, (N, K, M, act_scale))
 
 
 @pytest.mark.parametrize("M", [34, 70])
