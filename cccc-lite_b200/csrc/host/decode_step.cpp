@@ -379,9 +379,10 @@ bool DecodeStep::load(GpuControl* gpu, const BinFile& file, const ModelConfig& c
     }
     if (!ok) { return false; }
     // first use of the kernels allocates the library's per-device workspace: do it before any capture
-    cudaMemset(d_ids_, 0, (size_t)max_batch * 16);
+    // (the step's stream does not wait for the default stream: its zeros are written on it)
+    const bool cleared = cudaMemsetAsync(d_ids_, 0, (size_t)max_batch * 16, gpu_->stream()) == cudaSuccess;
     if (tp_) { tp_->barrier(); }
-    const int rc = issue(1, gpu_->stream());
+    const int rc = cleared ? issue(1, gpu_->stream()) : -1;
     gpu_->synchronize();
     const bool stepped = rc >= 0 && cuda_check_error("decode step warm-up") == 0;
     launches_per_step_ = rc;
@@ -480,7 +481,8 @@ bool DecodeStep::loadTensors(const BinFile& file, std::string* err)
         if (tp_->nMax() < (unsigned int)(B * cfg.hidden)) { return fail(err, "the exchange areas are smaller than max_batch * hidden"); }
     }
     graphs_.assign(max_batch + 1, nullptr);
-    gpu_->synchronize();
+    // The default stream's copies and the zeros above end before anything runs on the step's own stream, which is not ordered behind it.
+    if (cudaDeviceSynchronize() != cudaSuccess) { return fail(err, "a CUDA error while loading"); }
     return true;
 }
 
