@@ -34,14 +34,16 @@ public:
     virtual int step(const std::vector<StepEntry>& entries, float* logits, int* choice) = 0;
     // step() in two halves, so that a caller can make the place of the results ready while the device works: begin() checks the
     // entries (-1: they cannot run, and there is nothing to end) and may start them; end() finishes them, with the results that
-    // begin() was told of (or null: not taken).  Nothing else may be asked of the model in between.
+    // begin() was told of (or null: not taken; what begin() was not told of stays as it is).  Nothing else may be asked of the
+    // model in between.
     virtual int begin(std::vector<StepEntry> entries, bool logits, bool choice)
     {
-        (void)logits, (void)choice;
         held_ = std::move(entries);
+        held_logits_ = logits;
+        held_choice_ = choice;
         return valid(held_) ? 0 : -1;
     }
-    virtual int end(float* logits, int* choice) { return step(held_, logits, choice); }
+    virtual int end(float* logits, int* choice) { return step(held_, held_logits_ ? logits : nullptr, held_choice_ ? choice : nullptr); }
     virtual int launchesLastStep() const { return 0; }
     virtual size_t weightBytes() const { return 0; }
     // Device time of one step in ms (the fastest of `repeat` runs of `inner` steps): `entries` sequences that hold `context`
@@ -55,7 +57,8 @@ public:
 protected:
     // The checks of step() that every model needs.
     bool valid(const std::vector<StepEntry>& entries);
-    std::vector<StepEntry> held_;    // between begin() and end()
+    std::vector<StepEntry> held_;    // between begin() and end(), with the results that begin() was told of
+    bool held_logits_ = false, held_choice_ = false;
 };
 
 struct ModelOptions

@@ -694,8 +694,6 @@ int LayeredDecoder::begin(std::vector<StepEntry> entries, bool logits, bool choi
     last_launches_ = 0;
     held_pass_ = Pass();
     makePass(held_, std::vector<int>(held_.size(), 0), std::vector<int>(held_.size(), 1), &held_pass_);
-    started_logits_ = logits;
-    started_choice_ = choice;
     // a launch that fails leaves nothing started: end() runs the step anew, and says what is wrong
     startDecode(held_pass_, logits, choice, &started_);
     return 0;
@@ -703,10 +701,10 @@ int LayeredDecoder::begin(std::vector<StepEntry> entries, bool logits, bool choi
 
 int LayeredDecoder::end(float* logits, int* choice)
 {
-    if (!started_) { return step(held_, logits, choice); }
+    if (!started_) { return LanguageModel::end(logits, choice); }
     started_ = false;
     gpu_.setAsCurrent();
-    if (takeResults(held_pass_.wants, places(held_pass_, held_).data(), started_logits_ ? logits : nullptr, started_choice_ ? choice : nullptr) != 0) { return 1; }
+    if (takeResults(held_pass_.wants, places(held_pass_, held_).data(), held_logits_ ? logits : nullptr, held_choice_ ? choice : nullptr) != 0) { return 1; }
     advance(held_, std::vector<int>(held_.size(), 1));
     return *h_status_ == 0 && cudaPeekAtLastError() == cudaSuccess ? 0 : cuda_b200_decoder_check("decoder step");
 }

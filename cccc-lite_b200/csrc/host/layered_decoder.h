@@ -273,7 +273,7 @@ private:
     static constexpr int kPieces = 4;
     cudaEvent_t piece_[kPieces] = {};
     unsigned int* h_status_ = nullptr;
-    bool started_ = false, started_logits_ = false, started_choice_ = false;    // between begin() and end(): a decode step is under way
+    bool started_ = false;    // between begin() and end(): a decode step is under way
     Pass held_pass_;
 };
 

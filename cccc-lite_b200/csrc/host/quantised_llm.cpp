@@ -89,8 +89,10 @@ public:
     }
     int end(float* logits, int* choice) override
     {
-        if (!started_) { return step(held_, logits, choice); }
+        if (!started_) { return LanguageModel::end(logits, choice); }
         started_ = false;
+        logits = held_logits_ ? logits : nullptr;
+        choice = held_choice_ ? choice : nullptr;
         std::vector<size_t> first(held_.size());
         for (size_t e = 1; e < held_.size(); e++) { first[e] = first[e - 1] + held_[e - 1].want.size(); }
         return started_rc_ == 0 && finish(held_, 0, first, logits, choice) == 0 ? 0 : 1;

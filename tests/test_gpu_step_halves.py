@@ -9,6 +9,7 @@ import pytest
 from __graft_entry__ import load_package
 from oracle import fakilorn as F
 from tests.test_gpu_fakilorn import CONFIGS, tokens_for
+from tests.test_gpu_prompt import folder  # noqa: F401 (a fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -52,4 +53,25 @@ def test_the_halves_give_the_bits_of_the_whole(tmp_path, n):
     assert np.array_equal(np.array(a.step(steps[2])[0]), np.array(b.step(steps[2])[0]))
     # entries that cannot run: nothing to end
     assert b.lib.cccc_model_step_begin(b.h, *flat([(slots[0], [c["vocab"]], [0])]), 1, 0) == -1
+    a.close(), b.close()
+
+
+def test_the_halves_of_the_quantised_model(folder):  # noqa: F811
+    serve = load_package().serve
+    d, cfg = folder
+    a, b = (serve.Model(d, max_context=64, max_sequences=3) for _ in range(2))
+    rng = np.random.default_rng(3)
+    slots = [(a.open_slot(), b.open_slot())[0] for _ in range(3)]
+    token = lambda n=1: [int(t) for t in rng.integers(0, cfg.vocab, n)]
+    steps = [[(s, token(5 + s), [0, 4]) for s in slots], [(s, token(), [0]) for s in slots], [(s, token(), [] if s else [0]) for s in slots], [(slots[1], token(2), [1, 0])],
+             [(s, token(), [0]) for s in slots[::-1]], [(s, token(), [0]) for s in slots]]
+    for i, e in enumerate(steps):
+        wanted = sum(len(w) for _, _, w in e)
+        want, got, ids = np.zeros((wanted, cfg.vocab), np.float32), np.full((wanted, cfg.vocab), -1, np.float32), [ints([-1] * wanted) for _ in range(2)]
+        pointer = lambda x: x.ctypes.data_as(C.POINTER(C.c_float))
+        assert a.lib.cccc_model_step(a.h, *flat(e), pointer(want), ids[0]) == 0
+        assert b.lib.cccc_model_step_begin(b.h, *flat(e), i != 4, i != 3) == 0 and b.lib.cccc_model_step_end(b.h, pointer(got), ids[1]) == 0
+        assert np.array_equal(got, want) if i != 4 else (got == -1).all()
+        assert list(ids[1]) == (list(ids[0]) if i != 3 else [-1] * wanted)
+        assert [b.slot_length(s) for s in slots] == [a.slot_length(s) for s in slots]
     a.close(), b.close()

@@ -88,3 +88,20 @@ ok &= np.array_equal(rows(lg), expected([200, 3])) and ch == [200, 3] and [m.slo
 print(json.dumps(dict(seen(), ok=bool(ok))))
 """)
     assert s["ok"] and s["wild"] == 0 and s["prompt"] == LAYERS
+
+
+def test_the_halves_of_a_step_give_what_begin_was_told_of(run):
+    s = run("""
+m = serve.Model(FOLDER, max_context=32, max_sequences=3)
+a = m.open_slot()
+ints = lambda *v: (C.c_int * max(1, len(v)))(*v)
+def halves(tokens, want, logits, choice):
+    lg, ch = np.full((len(want), m.vocab), -1, np.float32), ints(*[-1] * len(want))
+    assert m.lib.cccc_model_step_begin(m.h, 1, ints(a), ints(len(tokens)), ints(*tokens), ints(len(want)), ints(*want), logits, choice) == 0
+    assert m.lib.cccc_model_step_end(m.h, lg.ctypes.data_as(C.POINTER(C.c_float)), ch) == 0
+    e = [tokens[w] for w in want]
+    return bool(np.array_equal(lg, expected(e)) if logits else (lg == -1).all()), list(ch) == (e if choice else [-1] * len(want))
+out = [halves(t, w, lg, ch) for t, w in (([9], [0]), ([4, 8], [1, 0])) for lg, ch in ((1, 1), (0, 1), (1, 0), (0, 0))]
+print(json.dumps(out))
+""")
+    assert s == [[True, True]] * 8
