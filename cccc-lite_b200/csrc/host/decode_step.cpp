@@ -634,7 +634,11 @@ int DecodeStep::prompt(const std::vector<PromptEntry>& entries, const std::vecto
         max_len = std::max(max_len, e.pos + e.n);
     }
     if (tokens == 0) { return 0; }
-    if (tokens > prompt_cap_ || (int)entries.size() > max_batch_ || (int)want.size() > tokens) { return -1; }
+    if (tokens > prompt_cap_ || (int)entries.size() > max_batch_) { return -1; }
+    for (int w : want)
+    {
+        if (w < 0 || w >= tokens) { return -1; }    // (a place may be wanted several times)
+    }
     gpu_->setAsCurrent();
     cudaStream_t st = gpu_->stream();
     // per token: id, position, slot, entry; per entry: slot, position, first token, tokens

@@ -105,3 +105,15 @@ out = [halves(t, w, lg, ch) for t, w in (([9], [0]), ([4, 8], [1, 0])) for lg, c
 print(json.dumps(out))
 """)
     assert s == [[True, True]] * 8
+
+
+def test_places_wanted_several_times_in_a_step_of_several_passes(run):
+    s = run("""
+m = serve.Model(FOLDER, max_context=64, max_sequences=2, max_step_tokens=8)
+a, b = m.open_slot(), m.open_slot()
+tokens, want = list(range(20, 30)), [9] * 7 + [0, 9, 3]       # the second pass has two tokens and eight wants
+lg, ch = m.step([(b, [100], [0]), (a, tokens, want)], choice=True)
+e = [100] + [tokens[w] for w in want]
+print(json.dumps([bool(np.array_equal(rows(lg), expected(e))), ch == e, m.slot_length(a)]))
+""")
+    assert s == [True, True, 10]
