@@ -7,6 +7,7 @@ from __future__ import annotations
 import ctypes as C
 import importlib.util
 import json
+import mmap
 import os
 from array import array
 
@@ -61,6 +62,14 @@ def _ints(values):
     return (C.c_int * max(1, len(values)))(*values)
 
 
+def _reserve(size):
+    """Address space for `size` bytes whose pages are not made yet."""
+    try:
+        return mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+    except (OSError, OverflowError) as e:
+        raise MemoryError("no memory for %d bytes of logits" % size) from e
+
+
 def _sampler(sampler):
     s = dict(temperature=0.0, top_k=0, top_p=1.0, repetition_penalty=1.0, banned_ids=())
     s.update(sampler or {})
@@ -98,16 +107,21 @@ class Model:
 
     def step(self, entries, logits=True, choice=False):
         """entries: (slot, tokens, want) triples.  Returns (logits, choices): a float array of wanted * vocab values and the
-        ids of the largest logits, in the order of the entries and of their wanted places (None where not asked for)."""
+        ids of the largest logits, in the order of the entries and of their wanted places (None where not asked for).  Where there is
+        no memory for them nothing runs."""
         wanted = sum(len(w) for _, _, w in entries)
-        lg = ch = lp = None
+        ch = (C.c_int * max(1, wanted))() if choice else None
+        lg = lp = None
+        # The pages of the logits are made while the step is under way, the room for them is taken before it begins.
+        room = _reserve(4 * wanted * self.vocab) if logits and wanted else None
         rc = self.lib.cccc_model_step_begin(self.h, len(entries), _ints(s for s, _, _ in entries), _ints(len(t) for _, t, _ in entries),
                                             _ints(x for _, t, _ in entries for x in t), _ints(len(w) for _, _, w in entries),
                                             _ints(x for _, _, w in entries for x in w), bool(logits and wanted), bool(choice))
         if rc == 0:
-            try:    # the step is under way: the pages of its results are made meanwhile
+            try:
+                if room is not None:
+                    room.close()
                 lg = array("f", (0.0,)) * (wanted * self.vocab) if logits else None
-                ch = (C.c_int * max(1, wanted))() if choice else None
                 lp = (C.c_float * len(lg)).from_buffer(lg) if logits and wanted else None
             finally:
                 rc = self.lib.cccc_model_step_end(self.h, lp, ch)

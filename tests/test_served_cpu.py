@@ -117,3 +117,24 @@ e = [100] + [tokens[w] for w in want]
 print(json.dumps([bool(np.array_equal(rows(lg), expected(e))), ch == e, m.slot_length(a)]))
 """)
     assert s == [True, True, 10]
+
+
+@pytest.mark.parametrize("vocab", [1 << 46, 1 << 62])    # beyond the address space, beyond what a size can say
+def test_a_step_without_memory_for_its_logits_has_not_run(vocab):
+    class Lib:
+        begun = 0
+
+        def cccc_model_step_begin(self, *_):
+            self.begun += 1
+            return 0
+
+        def cccc_model_step_end(self, *_):
+            return 0
+
+    serve = load_package().serve
+    m = serve.Model.__new__(serve.Model)
+    m.lib, m.h, m.vocab = Lib(), None, vocab
+    with pytest.raises(MemoryError):
+        m.step([(0, [1], [0])], choice=True)
+    assert m.lib.begun == 0
+    assert m.step([(0, [1], [0])], logits=False, choice=True) == (None, [0]) and m.lib.begun == 1
