@@ -68,7 +68,7 @@ struct ModelOptions
     DataType dtype = BFLOAT16;      // FLOAT: everything in true 32-bit
     int max_context = 4096;         // rows of a cache slot
     int max_sequences = 1;          // cache slots
-    int max_step_tokens = 4096;     // tokens one pass runs; longer steps run in several
+    int max_step_tokens = 4096;     // tokens one pass runs; longer steps run in several.  Activations of such a pass are held from load on.
     bool noise_weights = false;     // config.json only: seeded random weights
 };
 

@@ -46,7 +46,8 @@ public:
         vocab_ = m.vocab;
         batch_ = std::min(o.max_sequences, 32);
         if (!step_.load(&gpu_, f, m, batch_, nullptr, 0, err)) { return false; }
-        step_.reservePrompts(std::max(1, std::min(o.max_step_tokens, kMostPromptTokens)));
+        // a step never has more tokens than the cache has rows
+        step_.reservePrompts((int)std::max<long long>(1, std::min<long long>({ o.max_step_tokens, kMostPromptTokens, (long long)o.max_context * batch_ })));
         return true;
     }
     int vocab() const override { return vocab_; }

@@ -138,3 +138,13 @@ def test_a_step_without_memory_for_its_logits_has_not_run(vocab):
         m.step([(0, [1], [0])], choice=True)
     assert m.lib.begun == 0
     assert m.step([(0, [1], [0])], logits=False, choice=True) == (None, [0]) and m.lib.begun == 1
+
+
+def test_prompts_hold_no_more_than_a_step_can_have(run):
+    bytes_at = [run("""
+m = serve.Model(FOLDER, max_context=16, max_sequences=3, max_step_tokens=%d)
+a = m.open_slot()
+assert np.array_equal(rows(m.step([(a, [1] * 16, [15])])[0]), expected([1]))
+print(json.dumps(seen()))
+""" % n)["bytes"] for n in (32, 48, 4096)]
+    assert bytes_at[0] < bytes_at[1] == bytes_at[2]
