@@ -47,7 +47,8 @@ public:
         batch_ = std::min(o.max_sequences, 32);
         if (!step_.load(&gpu_, f, m, batch_, nullptr, 0, err)) { return false; }
         // a step never has more tokens than the cache has rows
-        step_.reservePrompts((int)std::max<long long>(1, std::min<long long>({ o.max_step_tokens, kMostPromptTokens, (long long)o.max_context * batch_ })));
+        const long long most = std::min<long long>({ o.max_step_tokens, kMostPromptTokens, (long long)o.max_context * batch_ });
+        if (most > 1) { step_.reservePrompts((int)most); }
         return true;
     }
     int vocab() const override { return vocab_; }
@@ -60,14 +61,18 @@ public:
         if (!valid(entries)) { return -1; }
         launches_ = 0;
         std::vector<size_t> first(entries.size());
-        size_t wanted = 0, longest = 0;
+        size_t wanted = 0, longest = 0, tokens = 0;
         for (size_t e = 0; e < entries.size(); e++)
         {
             first[e] = wanted;
             wanted += entries[e].want.size();
             longest = std::max(longest, entries[e].tokens.size());
+            tokens += entries[e].tokens.size();
         }
-        if (longest > 1 && step_.promptTokens() > 0) { return prompts(entries, first, logits, choice); }
+        // Either way a pass reads the weights once, and a decode step is one graph: many tokens at once only where that takes fewer.
+        // (Passes of one token never do, passes of two do not for two sequences.)
+        const size_t cap = (size_t)step_.promptTokens();
+        if (cap > 0 && (tokens + cap - 1) / cap < longest) { return prompts(entries, first, logits, choice); }
         // one token of all entries that have one after the other; the graph of a step takes them all
         for (size_t i = 0; i < longest; i++)
         {

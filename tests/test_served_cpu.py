@@ -148,3 +148,19 @@ assert np.array_equal(rows(m.step([(a, [1] * 16, [15])])[0]), expected([1]))
 print(json.dumps(seen()))
 """ % n)["bytes"] for n in (32, 48, 4096)]
     assert bytes_at[0] < bytes_at[1] == bytes_at[2]
+
+
+# (tokens of the sequences, tokens of a pass) -> passes, or 0: decode steps, one for each place of the longest sequence
+@pytest.mark.parametrize("lengths,cap,passes", [((10,), 1, 0), ((10,), 2, 5), ((10, 10), 2, 0), ((10, 9), 2, 0), ((10, 7), 2, 9), ((1, 2), 4096, 1), ((8, 8, 8), 3, 0)])
+def test_prompts_run_in_passes_where_that_takes_fewer(run, lengths, cap, passes):
+    s = run("""
+lengths, cap = %r
+m = serve.Model(FOLDER, max_context=16, max_sequences=3, max_step_tokens=cap)
+before = seen()
+e = [(m.open_slot(), [10 * i + j for j in range(n)], [0, n - 1]) if n > 1 else (m.open_slot(), [10 * i], [0]) for i, n in enumerate(lengths)]
+lg, ch = m.step(e, choice=True)
+want = [t[w] for _, t, ws in e for w in ws]
+ok = ch == want and np.array_equal(rows(lg), expected(want)) and [m.slot_length(x) for x, _, _ in e] == list(lengths)
+print(json.dumps(dict(ok=bool(ok), **{n: seen()[n] - before[n] for n in ("decode", "prompt", "wild")})))
+""" % ((lengths, cap),))
+    assert s == dict(ok=True, decode=0 if passes else LAYERS * max(lengths), prompt=LAYERS * passes, wild=0)
