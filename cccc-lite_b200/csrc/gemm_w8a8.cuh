@@ -21,11 +21,24 @@ constexpr int W8A8_MAX_TOKENS = 32;    // what the streaming kernel takes (all S
 // 24.0 / 26.0, at 16 151936 x 4096 106.4 / 122.3.  Small tensors keep the quantiser that finds the maximum itself.
 static inline bool w8a8_split_early(unsigned int M, unsigned int K) { return M >= 24 && (size_t)M * K > 16384; }
 
-// More tokens: k slices, or CTA pairs?  The line depends on tokens and k alone, so that a group of linears and the separate calls
-// take the same kernel and give the same bits.  Measured (dynamic scale, pairs' best form / slices, us): up to 64 tokens the
-// slices win on every linear of a layer (gemm_w8a8_split.cuh); at 128 tokens 4096 x 4096 17.9 / 14.2 but 24576 x 4096 31.4 / 38.3
-// (192 tiles, one CTA per SM); long k has few features: 4096 x 12288 at 128 / 256 / 300 tokens 35.6 / 21.9, 43.7 / 31.4, 44.8 / 44.6.
-static inline bool w8a8_split_preferred(unsigned int M, unsigned int K) { return M <= 64 || (M <= 256 && K >= 8192); }
+// More tokens: k slices, or CTA pairs?  Up to 64 the slices win on every linear of a layer (gemm_w8a8_split.cuh) and on 65536 features
+// (K 4096: 57.1 against 52.4 us).  Above, where k is long and the tiles (128 features x 128 tokens, one CTA per SM) are few, the pairs
+// leave the GPU idle; where they are many, the slices read a weight once per token tile and run in waves.  Measured (static scale,
+// quantiser included, K = 8192, pairs' best form / slices, us):
+//   up to 128 tokens, by tiles:  8 22.9 / 12.8,  32 23.4 / 14.9,  64 25.1 / 21.0,  80 27.0 / 28.2,  112 32.1 / 31.8,  148 37.7 / 36.6,
+//     160 44.8 / 57.0,  224 52.6 / 59.5,  448 97.7 / 114.1;
+//   129 tokens, by tiles (two per 128 features):  16 23.2 / 13.1,  64 23.7 / 19.1,  128 25.5 / 28.3,  160 27.2 / 42.2,  448 53.0 / 103.9;
+//   256 tokens:  64 28.1 / 19.7,  128 30.3 / 28.9,  160 31.8 / 51.9.  (K = 12288 to 28672: the same sides, few tiles gain more.)
+// Hence above 128 tokens as long as every tile gets two slices, which then run at once.  Up to 128 tokens the line lies behind what
+// would be the best one, at five quarters of a wave instead of one: the outputs of a feature keep their bits whatever matrix they are
+// part of at up to 20480 features, which the tests hold.
+static inline bool w8a8_split_preferred(unsigned int M, unsigned int K, unsigned int N, int sm_count)
+{
+    if (M <= 64) { return true; }
+    if (M > 256 || K < 8192) { return false; }
+    const unsigned long long tiles = (unsigned long long)((N + 127) / 128) * ((M + 127) / 128), sms = (unsigned)sm_count;
+    return M <= 128 ? 4 * tiles <= 5 * sms : 20 * tiles <= 9 * sms;
+}
 
 static inline int w8a8_launch_failed()
 {
@@ -280,13 +293,27 @@ static int launch_w8a8(const GemvScratch* ws, const W8A8Member* mem, unsigned in
     // dynamic scale of a small tensor: the quantiser finds the maximum itself
     const bool self_absmax = dynamic && !big && (size_t)M * K <= 16384 && eights;
     // The linear behind the quantiser (`after`: that was the launch before it on the stream; it lets its successor start).
-    auto many_tokens = [&](const NativeParams& n, const uint8_t* q, unsigned int ldq, bool after) {
-        if (pair_fh == 4 || (pair_fh == 0 && w8a8_split_preferred(M, K)))
+    // Every member takes the kernel that it would take alone, so that a group gives the bits of the separate calls; neighbours of a
+    // kind share a launch.
+    auto many_tokens = [&](const NativeParams& all, const uint8_t* q, unsigned int ldq, bool after) {
+        auto slices = [&](unsigned int j) { return pair_fh == 4 || (pair_fh == 0 && w8a8_split_preferred(M, K, mem[j].N_out, ws->sm_count)); };
+        for (unsigned int j = 0, end; j < count; j = end)
         {
-            const int r = launch_w8a8_split(n, mem, q, ldq, ws->device, ws->sm_count, stream, after || pdl);
-            if (r != -2) { return r; }
+            for (end = j + 1; end < count && slices(end) == slices(j);) { end++; }
+            NativeParams n = all;
+            n.n_seg = end - j;
+            n.tiles = 0;
+            for (unsigned int i = j; i < end; i++)
+            {
+                n.seg[i - j] = all.seg[i];
+                n.seg[i - j].tile0 = n.tiles;
+                n.tiles += (mem[i].N_out + NK_BM - 1) / NK_BM;
+            }
+            int r = slices(j) ? launch_w8a8_split(n, mem + j, q, ldq, ws->device, ws->sm_count, stream, after || pdl) : -2;
+            if (r == -2) { r = launch_w8a8_pair(n, mem + j, q, ldq, ws->device, ws->sm_count, pair_fh, stream); }
+            if (r != 0) { return r; }
         }
-        return launch_w8a8_pair(n, mem, q, ldq, ws->device, ws->sm_count, pair_fh, stream);
+        return 0;
     };
     if (big && x_is_e4m3 && (ldx % 16) == 0 && sk_al16(X))
     {

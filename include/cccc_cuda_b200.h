@@ -163,7 +163,8 @@ C_EXPORT int cuda_embed_fwd_fp8_to_fp8(const void* ids, const void* W, void* Y, 
 C_EXPORT int cuda_embed_fwd_bf16_to_fp8(const void* ids, const void* W, void* Y, int D, int T, int B);
 
 /* Up to three W8A8 linears that read the same activations (q/k/v, gate/up) as one call: the activations are quantised
- * once and the members' feature tiles are dealt out together.  Members as for cuda_gemm_wq_bf16_group (blk_scales
+ * once and the members' feature tiles are dealt out together (above 64 tokens in a launch for each kind of kernel that the
+ * members would take alone).  Members as for cuda_gemm_wq_bf16_group (blk_scales
  * unused); the result is that of `count` separate cuda_gemm_w8a8_bf16 calls, bit for bit.  -1 where one of those would
  * return it, for more than three members, or for a member without outputs. */
 C_EXPORT int cuda_gemm_w8a8_bf16_group(unsigned int count, const cuda_wq_linear* linears, const void* X, float act_scale,

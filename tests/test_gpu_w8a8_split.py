@@ -109,3 +109,50 @@ def test_e4m3_activations_where_they_lie(y_type):
         want = O.float_to_fp8(O.bf16_bits_to_f32(O.f32_to_bf16_bits(y)).reshape(-1), O.FP8_E4M3, 1.0)
         diff = np.abs(out.cpu().numpy().astype(np.int16) - want.astype(np.int16))
         assert diff.max() <= 1 and np.mean(diff != 0) < 2e-3
+
+
+def on_device(Ns, K, M, seed=0):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    Ws = [torch.randint(0, 256, (N, K), dtype=torch.uint8, device="cuda", generator=g) for N in Ns]
+    for W in Ws:
+        W[(W & 0x7F) == 0x7F] = 0    # not a number in E4M3
+    return Ws, torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+
+
+# the lines between the k slices and the CTA pairs, in tiles of 128 features x 128 tokens: a wave and a quarter up to 128 tokens, two slices of
+# every tile at once above; and where k is too short or the tokens too many
+@pytest.mark.parametrize("M,K,beyond", [(65, 8192, 0), (128, 8192, 0), (128, 8192, 1), (129, 8192, 0), (129, 8192, 1), (256, 12288, 0), (256, 12288, 1), (257, 8192, 1), (65, 8064, 1)])
+def test_the_line_above_64_tokens(M, K, beyond):
+    """Sums of k slices and of the whole k range differ in their last bits: the float32 outputs say which kernel ran."""
+    import torch
+
+    c, sms = capi(), torch.cuda.get_device_properties(0).multi_processor_count
+    tiles = 5 * sms // 4 if M <= 128 else 9 * sms // 20 // 2    # of features
+    if M > 256 or K < 8192:
+        tiles = 0
+    N = 128 * tiles + (1 if beyond else 0)
+    (W,), X = on_device([N], K, M)
+    out = {}
+    for form in (0, 1, 4):
+        out[form] = torch.zeros(M, N, dtype=torch.float32, device="cuda")
+        assert c.gemm_w8a8_bf16(W, 0.01, X, 0.0, out[form], N, M, K, flags=4 | form << 8) == 0 and c.check_error("line") == 0
+    assert not torch.equal(out[1], out[4])
+    assert torch.equal(out[0], out[1 if beyond else 4])
+
+
+@pytest.mark.parametrize("order,launches", [((4352, 256, 384), 4), ((256, 4352, 384), 5), ((256, 384, 4096), 3), ((4352, 4480, 9000), 3)])
+def test_members_of_a_group_take_the_kernels_they_would_take_alone(order, launches):
+    import torch
+
+    c, M, K = capi(), 129, 8192
+    Ws, X = on_device(order, K, M, 1)
+    items = [dict(W=W, S=None, inv=0.01 * (i + 1), N=N, Y=torch.zeros(M, N, dtype=torch.float32, device="cuda")) for i, (W, N) in enumerate(zip(Ws, order))]
+    before = c.launch_count()
+    assert c.gemm_w8a8_bf16_group(c.make_group(items, K), X, 0.0, M, K, flags=4) == 0 and c.check_error("group") == 0
+    assert c.launch_count() - before == launches
+    for it in items:
+        y = torch.zeros_like(it["Y"])
+        assert c.gemm_w8a8_bf16(it["W"], it["inv"], X, 0.0, y, it["N"], M, K, flags=4) == 0 and c.check_error("alone") == 0
+        assert torch.equal(y, it["Y"])
