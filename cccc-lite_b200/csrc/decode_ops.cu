@@ -169,22 +169,57 @@ __global__ void __launch_bounds__(256) attn_append_kernel(const AttnDecodeParams
     }
 }
 
-// Splits of a (sequence, kv head), from a model fitted to measurements (4096 rows, 8 kv heads): the clusters run in rounds on the
-// slots of the GPU, three CTAs per SM in eight GPCs of whole clusters; a round of n CTAs takes 4 ns and the larger of 14 ns (a
-// CTA's own pace) and 0.08 n ns (HBM) per row of a split, and 5 us; a cluster takes 0.15 us per member to meet.  Hence as many
-// splits as still run in one round, and more rounds only where one would leave slots empty for long.  Measured (us, split
-// counts): 8 sequences 4: 35.5, 6: 30.4 (384 CTAs), 7: 45.7; 16 sequences 2: 59.0, 3: 50.8, 4: 71.3; 32 sequences 1: 103.9,
-// 2: 125.2, 3: 97.7, 5: 121.1; one sequence 8: 15.4, 16: 12.6.
-static unsigned int attn_splits(unsigned long long units, unsigned int T_max, int sm_count)
+struct DeviceFacts
 {
-    unsigned int best = 1;
+    std::atomic<int> ready{ 0 };
+    int sm_count = 0, max_smem = 0, sm_smem = 0, device = 0;
+};
+static DeviceFacts g_facts[64];
+static const DeviceFacts* device_facts()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { return nullptr; }
+    DeviceFacts& f = g_facts[dev];
+    if (f.ready.load(std::memory_order_acquire) == 0)
+    {
+        int a = 0, b = 0, c = 0;
+        if (cudaDeviceGetAttribute(&a, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess
+            || cudaDeviceGetAttribute(&b, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess
+            || cudaDeviceGetAttribute(&c, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
+        {
+            return nullptr;
+        }
+        f.sm_count = a;    // two threads may both write the same values: harmless
+        f.max_smem = b;
+        f.sm_smem = c;
+        f.device = dev;
+        f.ready.store(1, std::memory_order_release);
+    }
+    return &f;
+}
+
+// Splits of a (sequence, kv head), from a model fitted to measurements (4096 rows, 8 kv heads): the clusters run in rounds on the
+// slots of the GPU, up to three CTAs per SM - as many as their shared memory, which grows with the rows of a split, leaves room for -
+// in eight GPCs of whole clusters; a round of n CTAs takes 4 ns and the larger of 14 ns (a CTA's own pace) and 0.08 n ns (HBM) per row
+// of a split, and 5 us; a cluster takes 0.15 us per member to meet.  Hence as many splits as still run in one round, and more rounds
+// only where one would leave slots empty for long.  Measured (us, split counts): 8 sequences 4: 35.5, 6: 30.4 (384 CTAs), 7: 45.7; 16
+// sequences 2: 59.0, 3: 50.8, 4: 71.3; 32 sequences 1: 103.9, 2: 125.2, 3: 97.7, 5: 121.1; one sequence 8: 15.4, 16: 12.6.  Long
+// caches, 32768 rows, as three CTAs per SM would have it / as their shared memory does: 16 sequences of 4 heads per kv head 3:
+// 582 / 6: 345; of 8 heads 8 sequences 6: 281 / 8: 192, 16 sequences 3: 536 / 6: 420.
+// smem(S): bytes that a CTA of S splits asks for.
+template <class Smem>
+static unsigned int attn_splits(unsigned long long units, unsigned int T_max, const DeviceFacts& dev, Smem smem)
+{
+    unsigned int best = 8;    // (its scores always fit: see the limit in launch_attn)
     float least = INFINITY;
     for (unsigned int S = 1; S <= (unsigned int)AD_MAX_SPLITS; S = S < 8 ? S + 1 : S + 8)
     {
         if (S > 1 && T_max / S < 64u) { break; }
-        const unsigned long long slots = (3ull * ((unsigned)sm_count / 8) / S) * S * 8;
+        if (smem(S) > (size_t)dev.max_smem) { continue; }
+        const unsigned long long room = (size_t)dev.sm_smem / (smem(S) + 1024), per_sm = room < 3 ? room : 3;    // 1 KB of a CTA's is the system's
+        const unsigned long long slots = (per_sm * ((unsigned)dev.sm_count / 8) / S) * S * 8;
         const float rows = (float)((T_max + S - 1) / S);
-        if (slots == 0) { break; }
+        if (slots == 0) { continue; }
         if (S > 8 && units * S > slots) { break; }
         auto round = [&](unsigned long long n) { return n == 0 ? 0.f : rows * (4.f + fmaxf(14.f, 0.08f * (float)n)) + 5000.f; };
         const float cost = (float)(units * S / slots) * round(slots) + round(units * S % slots) + 150.f * (float)S;
@@ -198,16 +233,16 @@ static unsigned int attn_splits(unsigned long long units, unsigned int T_max, in
 }
 
 template <int G, int HD>
-static int launch_attn(const AttnDecodeParams& p, int sm_count, int max_smem, cudaStream_t stream, bool pdl)
+static int launch_attn(const AttnDecodeParams& p, const DeviceFacts& dev, cudaStream_t stream, bool pdl)
 {
+    const int max_smem = dev.max_smem;
     // Caches beyond what sixteen splits with their scores as floats in shared memory could hold were never served: callers take
     // their own path then, and still do.
     if ((attn_smem_floats<G, HD>(((p.T_max + 15u) / 16u + 31u) & ~31u) + (G < 4 ? (4 - G) * 2048 : 0)) * sizeof(float) > (size_t)max_smem) { return -1; }
     auto kernel = attn_decode_kernel<G, HD>;
-    unsigned int S = attn_splits((unsigned long long)p.B * p.Hkv, p.T_max, sm_count);
     auto row_cap = [&](unsigned int splits) { return ((p.T_max + splits * AD_TILE - 1) / (splits * AD_TILE)) * AD_TILE; };
     auto smem = [&](unsigned int splits) { return sizeof(AttnDecodeSmem<G, HD>) + (size_t)G * ad_score_row(row_cap(splits)) * 2; };
-    while (S < (unsigned int)AD_MAX_SPLITS && smem(S) > (size_t)max_smem) { S = S < 8 ? S + 1 : AD_MAX_SPLITS; }
+    unsigned int S = attn_splits((unsigned long long)p.B * p.Hkv, p.T_max, dev, smem);
     // (the same value from every thread)
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) != cudaSuccess
         || (S > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
@@ -229,53 +264,30 @@ static int launch_attn(const AttnDecodeParams& p, int sm_count, int max_smem, cu
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 2 : 1;
-    static std::atomic<int> max_cluster{ 0 };    // largest cluster this kernel can be scheduled with (0 = not probed)
-    if (S > 8 && max_cluster.load(std::memory_order_relaxed) == 0)
+    // Can a cluster of more than eight be scheduled?  That depends on the device and on what its CTAs ask for: asked for once up to the
+    // largest request that can, and down to the smallest that cannot.
+    static std::atomic<unsigned int> can[64], cannot[64];    // bytes; 0: not known
+    if (S > 8 && cfg.dynamicSmemBytes > can[dev.device].load(std::memory_order_relaxed))
     {
+        const unsigned int no = cannot[dev.device].load(std::memory_order_relaxed);
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1)
+        if ((no == 0 || cfg.dynamicSmemBytes < no) && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0)
+        {
+            can[dev.device].store((unsigned int)cfg.dynamicSmemBytes, std::memory_order_relaxed);
+        }
+        else
         {
             cudaGetLastError();
-            max_cluster.store(8, std::memory_order_relaxed);
+            if (no == 0 || cfg.dynamicSmemBytes < no) { cannot[dev.device].store((unsigned int)cfg.dynamicSmemBytes, std::memory_order_relaxed); }
+            S = 8;
+            if (smem(S) > (size_t)max_smem) { return -1; }
+            cfg.gridDim.x = attr[0].val.clusterDim.x = S;
+            cfg.dynamicSmemBytes = smem(S);
         }
-        else { max_cluster.store(16, std::memory_order_relaxed); }
-    }
-    if (S > 8 && max_cluster.load(std::memory_order_relaxed) == 8)
-    {
-        S = 8;
-        if (smem(S) > (size_t)max_smem) { return -1; }
-        cfg.gridDim.x = attr[0].val.clusterDim.x = S;
-        cfg.dynamicSmemBytes = smem(S);
     }
     count_launch();
     if (cudaLaunchKernelEx(&cfg, kernel, p, row_cap(S)) != cudaSuccess) { return report_launch("attn_decode_bf16") ? 1 : 1; }
     return 0;
-}
-
-struct DeviceFacts
-{
-    std::atomic<int> ready{ 0 };
-    int sm_count = 0, max_smem = 0;
-};
-static DeviceFacts g_facts[64];
-static const DeviceFacts* device_facts()
-{
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { return nullptr; }
-    DeviceFacts& f = g_facts[dev];
-    if (f.ready.load(std::memory_order_acquire) == 0)
-    {
-        int a = 0, b = 0;
-        if (cudaDeviceGetAttribute(&a, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess
-            || cudaDeviceGetAttribute(&b, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
-        {
-            return nullptr;
-        }
-        f.sm_count = a;    // two threads may both write the same values: harmless
-        f.max_smem = b;
-        f.ready.store(1, std::memory_order_release);
-    }
-    return &f;
 }
 
 template <class K, class... Args>
@@ -421,10 +433,10 @@ C_EXPORT int cuda_attn_decode_bf16(const cuda_attn_decode* a, void* stream, unsi
     {
         switch (G)
         {
-        case 1: return launch_attn<1, 128>(p, f->sm_count, f->max_smem, st, pdl);
-        case 2: return launch_attn<2, 128>(p, f->sm_count, f->max_smem, st, pdl);
-        case 4: return launch_attn<4, 128>(p, f->sm_count, f->max_smem, st, pdl);
-        case 8: return launch_attn<8, 128>(p, f->sm_count, f->max_smem, st, pdl);
+        case 1: return launch_attn<1, 128>(p, *f, st, pdl);
+        case 2: return launch_attn<2, 128>(p, *f, st, pdl);
+        case 4: return launch_attn<4, 128>(p, *f, st, pdl);
+        case 8: return launch_attn<8, 128>(p, *f, st, pdl);
         default: return -1;
         }
     }
@@ -432,10 +444,10 @@ C_EXPORT int cuda_attn_decode_bf16(const cuda_attn_decode* a, void* stream, unsi
     {
         switch (G)
         {
-        case 1: return launch_attn<1, 64>(p, f->sm_count, f->max_smem, st, pdl);
-        case 2: return launch_attn<2, 64>(p, f->sm_count, f->max_smem, st, pdl);
-        case 4: return launch_attn<4, 64>(p, f->sm_count, f->max_smem, st, pdl);
-        case 8: return launch_attn<8, 64>(p, f->sm_count, f->max_smem, st, pdl);
+        case 1: return launch_attn<1, 64>(p, *f, st, pdl);
+        case 2: return launch_attn<2, 64>(p, *f, st, pdl);
+        case 4: return launch_attn<4, 64>(p, *f, st, pdl);
+        case 8: return launch_attn<8, 64>(p, *f, st, pdl);
         default: return -1;
         }
     }

@@ -4,6 +4,7 @@ against the oracle's composition of the reference's ops (tests/test_gpu_decode_o
 import numpy as np
 import pytest
 
+from tests._util import assert_close_rows, capi
 from tests.test_gpu_decode_ops import attention_case
 
 pytestmark = pytest.mark.gpu
@@ -30,3 +31,39 @@ def test_a_cluster_of_sixteen(pos):
 def test_counts_of_sequences(B, Hkv, T_max):
     rng = np.random.default_rng(B)
     attention_case(B, 4 * Hkv, Hkv, 128, T_max, [int(p) for p in rng.integers(0, T_max, B)], False, B, strided=True)
+
+
+def long_case(B, Hkv, G, hd, T_max, pos, seed):
+    """Caches made on the device, queries and keys as they are (no norm, a rotation by nothing); against the reference's roundings of
+    scores and weights in float64."""
+    import torch
+
+    c, g = capi(), torch.Generator(device="cuda").manual_seed(seed)
+    bf = lambda *s: torch.randn(*s, device="cuda", generator=g, dtype=torch.bfloat16)
+    H = G * Hkv
+    q, k, v, K, V = bf(B, H, hd), bf(B, Hkv, hd), bf(B, Hkv, hd), bf(B, Hkv, T_max, hd), bf(B, Hkv, T_max, hd)
+    cos, sin = torch.ones(T_max, hd // 2, device="cuda", dtype=torch.bfloat16), torch.zeros(T_max, hd // 2, device="cuda", dtype=torch.bfloat16)
+    out, p = torch.zeros(B, H * hd, device="cuda", dtype=torch.bfloat16), torch.tensor(pos, dtype=torch.int32, device="cuda")
+    desc = c.make_attn_decode(q=q, k=k, v=v, k_cache=K, v_cache=V, pos=p, out=out, cos_tab=cos, sin_tab=sin, B=B, H=H, Hkv=Hkv, head_dim=hd, T_max=T_max)
+    rc = c.attn_decode_bf16(desc)
+    assert c.check_error("long") == 0
+    if rc != 0:
+        return rc
+    want = torch.empty(B, H, hd, dtype=torch.float64, device="cuda")
+    for b, at in enumerate(pos):
+        assert torch.equal(K[b, :, at], k[b]) and torch.equal(V[b, :, at], v[b])
+        for h in range(Hkv):
+            s = ((q[b, h * G:(h + 1) * G].double() @ K[b, h, :at + 1].double().T).float() * (1.0 / np.float32(np.sqrt(np.float32(hd))))).to(torch.bfloat16)
+            w = torch.softmax(s.double(), -1).to(torch.bfloat16)
+            want[b, h * G:(h + 1) * G] = w.double() @ V[b, h, :at + 1].double()
+    assert_close_rows(out.float().cpu().numpy().reshape(B * H, hd), want.cpu().numpy().reshape(B * H, hd), (B, Hkv, G, hd, T_max))
+    return 0
+
+
+# caches so long that the scores of a split take the shared memory of two or three CTAs
+@pytest.mark.parametrize("B,Hkv,G,hd,T_max", [(16, 8, 8, 128, 32768), (9, 8, 8, 64, 40000), (16, 4, 4, 128, 65536), (1, 1, 8, 128, 65536), (1, 2, 1, 128, 32768)])
+def test_long_caches(B, Hkv, G, hd, T_max):
+    rng = np.random.default_rng(B)
+    pos = [T_max - 1] + [int(x) for x in rng.integers(0, T_max, B - 1)]
+    assert long_case(B, Hkv, G, hd, T_max, pos, G) == 0
+    assert long_case(1, 1, G, hd, 256, [200], G) == 0    # a small cache after a large one
