@@ -210,7 +210,7 @@ static const DeviceFacts* device_facts()
 template <class Smem>
 static unsigned int attn_splits(unsigned long long units, unsigned int T_max, const DeviceFacts& dev, Smem smem)
 {
-    unsigned int best = 8;    // (its scores always fit: see the limit in launch_attn)
+    unsigned int best = 8;    // (its scores always fit: see attn_served)
     float least = INFINITY;
     for (unsigned int S = 1; S <= (unsigned int)AD_MAX_SPLITS; S = S < 8 ? S + 1 : S + 8)
     {
@@ -232,13 +232,22 @@ static unsigned int attn_splits(unsigned long long units, unsigned int T_max, co
     return best;
 }
 
+// Caches that this entry point serves: up to what sixteen splits hold whose scores are floats, in 32s of rows, beside (3 G + 5) HD + 260 G
+// + 256 + max(2048 G, 8192) floats.  This kernel holds BF16 scores and would go on for twice the rows; callers take their own path
+// from there on and rely on being told.
+template <int G, int HD>
+static bool attn_served(unsigned int T_max, int max_smem)
+{
+    constexpr size_t fixed = (3 * G + 5) * HD + 260 * G + 256 + (G < 4 ? 8192 : 2048 * G);
+    const size_t rows = ((size_t)T_max + 15) / 16;
+    return (fixed + G * ((rows + 31) / 32 * 32)) * sizeof(float) <= (size_t)max_smem;
+}
+
 template <int G, int HD>
 static int launch_attn(const AttnDecodeParams& p, const DeviceFacts& dev, cudaStream_t stream, bool pdl)
 {
     const int max_smem = dev.max_smem;
-    // Caches beyond what sixteen splits with their scores as floats in shared memory could hold were never served: callers take
-    // their own path then, and still do.
-    if ((attn_smem_floats<G, HD>(((p.T_max + 15u) / 16u + 31u) & ~31u) + (G < 4 ? (4 - G) * 2048 : 0)) * sizeof(float) > (size_t)max_smem) { return -1; }
+    if (!attn_served<G, HD>(p.T_max, max_smem)) { return -1; }
     auto kernel = attn_decode_kernel<G, HD>;
     auto row_cap = [&](unsigned int splits) { return ((p.T_max + splits * AD_TILE - 1) / (splits * AD_TILE)) * AD_TILE; };
     auto smem = [&](unsigned int splits) { return sizeof(AttnDecodeSmem<G, HD>) + (size_t)G * ad_score_row(row_cap(splits)) * 2; };

@@ -67,3 +67,15 @@ def test_long_caches(B, Hkv, G, hd, T_max):
     pos = [T_max - 1] + [int(x) for x in rng.integers(0, T_max, B - 1)]
     assert long_case(B, Hkv, G, hd, T_max, pos, G) == 0
     assert long_case(1, 1, G, hd, 256, [200], G) == 0    # a small cache after a large one
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("G", [1, 2, 4, 8])
+def test_the_longest_cache_that_is_served(G, hd):
+    import torch
+
+    floats = torch.cuda.get_device_properties(0).shared_memory_per_block_optin // 4 - ((3 * G + 5) * hd + 260 * G + 256 + max(2048 * G, 8192))
+    most = floats // G // 32 * 32 * 16
+    assert long_case(1, 1, G, hd, most, [most - 1], G) == 0
+    assert long_case(3, 2, G, hd, most, [most // 2, 0, most - 1], G) == 0
+    assert long_case(1, 1, G, hd, most + 1, [0], G) == -1
