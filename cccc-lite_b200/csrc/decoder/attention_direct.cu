@@ -409,15 +409,16 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
     for (unsigned int i = tid; i < count; i += 32 * AS_WARPS)
     {
         const unsigned int r = (first + i) / p.vdim, d = (first + i) % p.vdim;
-        const float mr = top(meet.recv_ml, S, r);
+        // (a row all of whose scores are minus infinity has weights of zero: with a sink its output is zero)
+        const float mr = top(meet.recv_ml, S, r), base = mr == -INFINITY ? 0.f : mr;
         float lr = 0.f, x = 0.f;
         for (unsigned int c = 0; c < S; c++)
         {
-            const float w = exp2f(meet.recv_ml[c][r][0] - mr);
+            const float w = exp2f(meet.recv_ml[c][r][0] - base);
             lr += w * meet.recv_ml[c][r][1];
             x += w * meet.recv[c * share + i];
         }
-        if (p.sink != nullptr) { lr += exp2f(p.sink[kvh * p.G + (r0 + r) % p.G] * 1.44269504088896341f - mr); }
+        if (p.sink != nullptr) { lr += exp2f(p.sink[kvh * p.G + (r0 + r) % p.G] * 1.44269504088896341f - base); }
         attention_store(p, qkvg, start, kvh, r0 + r, d, x / lr);
     }
 }
