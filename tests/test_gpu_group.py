@@ -137,3 +137,27 @@ def test_group_above_32_tokens_with_beta_and_float32_output(wt):
         _, y32 = O.linear_wq_bf16(wt, W, blk, inv, X, N, M, K, alpha=it["alpha"])
         got = it["Y"].cpu().numpy().reshape(M, N) - 1.0
         assert_close(got, y32, (wt, N))
+
+
+@pytest.mark.parametrize("wt", [O.FP8_E4M3, O.FP4_E2M1])
+@pytest.mark.parametrize("Ns,K,M", [((4096, 1024, 1024), 4096, 301), ((4096, 1024, 1024), 4096, 64), ((2560, 640), 1024, 129)])
+def test_a_group_whose_k_is_cut_otherwise_than_its_members(wt, Ns, K, M):
+    """A launch cuts k by all of its tiles: grouped and separate calls add the same products in FP32 in another order.  K / 16 steps on
+    either side, each rounding at 2^-24 of a partial sum of at most four times the row's rms."""
+    import torch
+
+    c, g = capi(), torch.Generator(device="cuda").manual_seed(K + M)
+    X = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    items = []
+    for N in Ns:
+        W = torch.randint(0, 256, (N, K if wt != O.FP4_E2M1 else K // 2), dtype=torch.uint8, device="cuda", generator=g)
+        if wt != O.FP4_E2M1:
+            W[(W & 0x7F) == 0x7F] = 0
+        S = torch.randint(0x28, 0x48, (N * K // 16,), dtype=torch.uint8, device="cuda", generator=g) if wt == O.FP4_E2M1 else None
+        items.append(dict(W=W, S=S, inv=1.0 if S is not None else 0.37, N=N, Y=torch.zeros(M, N, dtype=torch.float32, device="cuda")))
+    assert c.gemm_wq_bf16_group(wt, c.make_group(items, K), X, M, K, flags=c.FLAG_OUT_F32) == 0 and c.check_error("group") == 0
+    for it in items:
+        y = torch.zeros_like(it["Y"])
+        assert c.gemm_wq_bf16(wt, it["W"], it["S"], it["inv"], X, y, it["N"], M, K, flags=c.FLAG_OUT_F32) == 0 and c.check_error("alone") == 0
+        rms = y.square().mean(1, keepdim=True).sqrt()
+        assert float(((y - it["Y"]).abs() / rms).max()) <= 2 * (K / 16) * 2.0 ** -24 * 4

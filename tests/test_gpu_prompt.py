@@ -103,3 +103,27 @@ def test_prompts_match_decoding_token_by_token(folder, cap):
             assert error(np.concatenate(got[i]), want[i]) < bar, (cuts, i, error(np.concatenate(got[i]), want[i]))
             m.close_slot(slots[i])
     m.close()
+
+
+@pytest.mark.parametrize("hd,H,Hkv", [(128, 4, 2), (64, 8, 1)])
+def test_append_past_the_cache_writes_the_queries_alone(hd, H, Hkv):
+    import torch
+
+    c, T, tokens, rng = capi(), 32, 9, np.random.default_rng(hd)
+    bf = lambda *s: to_dev(O.f32_to_bf16_bits(rng.standard_normal(s).astype(np.float32)))
+    x, w, cos, sin = bf(tokens, (H + 2 * Hkv) * hd), bf(hd), bf(T, hd // 2), bf(T, hd // 2)
+    pos = torch.full((tokens,), T - 1, dtype=torch.int32, device="cuda")
+    pos[3] = T - 2    # the last row of the smaller cache
+    out = {}
+    for rows in (T, T - 1):
+        k, v, q = torch.zeros(tokens, Hkv, rows, hd, dtype=torch.int16, device="cuda"), torch.zeros(tokens, Hkv, rows, hd, dtype=torch.int16, device="cuda"), torch.zeros(
+            tokens, H * hd, dtype=torch.int16, device="cuda")
+        at = lambda n: x.data_ptr() + 2 * n * hd
+        d = c.make_attn_decode(q=at(0), k=at(H), v=at(H + Hkv), k_cache=k, v_cache=v, pos=pos, out=q, cos_tab=cos, sin_tab=sin, q_norm=w, k_norm=w, B=tokens, H=H, Hkv=Hkv,
+                               head_dim=hd, T_max=rows, ldq=x.shape[1], ldk=x.shape[1], ldv=x.shape[1])
+        assert c.attn_append_bf16(d) == 0 and c.check_error("append") == 0
+        out[rows] = (k, v, q)
+    (k, v, q), (k1, v1, q1) = out[T], out[T - 1]
+    assert bool(q.any(1).all()) and torch.equal(q, q1)
+    k[:, :, T - 1], v[:, :, T - 1] = 0, 0    # what the smaller cache has no row for
+    assert bool(k[3].any()) and torch.equal(k[:, :, :T - 1], k1) and torch.equal(v[:, :, :T - 1], v1)
