@@ -118,11 +118,13 @@ typedef struct cuda_wq_linear
 /* Several quantised linears that read the SAME activations X (and so share M_tokens, K, ldx and the
  * weight type) in one call: the q/k/v projections of a layer, or gate and up.  The reference issues
  * them as separate ops (scripts/convert_weights.py:488-524 generates one batchedMul per projection,
- * each reaching cccc/cublas_real.h:943-964); here up to 3 of them that the decode kernel takes
- * (M_tokens <= 32, TMA-eligible operands) run as ONE launch whose row blocks are dealt to the SMs
- * together, which saves the per-launch latency that dominates small linears.  Anything else (more
- * linears, more tokens, unaligned operands) is run one linear at a time, so the result is always
- * that of `count` separate cuda_gemm_wq_bf16 calls.  stream and flags as there. */
+ * each reaching cccc/cublas_real.h:943-964); here up to 3 of them with TMA-eligible operands run as ONE launch of
+ * the kernel that their token count asks for, whose tiles are dealt to the SMs together: that saves the per-launch
+ * latency that dominates small linears and fills the GPU.  Anything else (more linears, unaligned operands) is run one
+ * linear at a time.  The result is that of `count` separate cuda_gemm_wq_bf16 calls up to the order in which FP32
+ * partial sums are added: the decode and the streaming kernels cut k by the number of tiles of the launch, so that a
+ * group and its members alone may cut it differently.  (The prefill kernel never cuts k: with flags bits 8-10 = 1 .. 6
+ * the bits agree.)  stream and flags as there. */
 C_EXPORT int cuda_gemm_wq_bf16_group(int w_type, unsigned int count, const cuda_wq_linear* linears, const void* X,
     unsigned int M_tokens, unsigned int K, unsigned int ldx, void* stream, unsigned int flags);
 
