@@ -13,7 +13,9 @@
 // memory, one barrier, and the shares are summed where they lie.  (Partial results through global memory, summed by the last CTA
 // to arrive at a counter, took four more round trips to L2 of a chain that is all latency at a few hundred rows: 8 sequences
 // of 250 rows, 4 kv heads, 17 us behind the projections, now 8.4.)
+#include <atomic>
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "attention_mma.cuh"
 
@@ -423,26 +425,57 @@ __global__ void __launch_bounds__(32 * AS_WARPS, NR == 1 && DK + DV < 256 ? 3 : 
     }
 }
 
-template <int DK, int DV>
-static int run_direct(const AttnParams& p, unsigned int entries, unsigned int nr, cudaStream_t stream, bool pdl)
+// Clusters of S CTAs that the device holds at once, less what the previous kernel's CTAs, which leave one after the other, may cut up:
+// one in twenty (32 clusters of eight where 33 fit ran in two rounds behind an append), a quarter of the sizes between eight and
+// sixteen (16 clusters of thirteen where 17 fit did).  The GPCs differ in size, so this is asked for, once for each kernel and size.
+template <int DK, int DV, int NR>
+static unsigned int direct_clusters(unsigned int S, int device)
 {
-    const dim3 grid(p.splits, p.Hkv * p.row_tiles, entries);
-    return nr == 1 ? launch_cluster("attention_direct", attention_direct_kernel<DK, DV, 1>, grid, dim3(32 * AS_WARPS), 0, p.splits, stream, pdl, p)
-                   : launch_cluster("attention_direct", attention_direct_kernel<DK, DV, 2>, grid, dim3(32 * AS_WARPS), 0, p.splits, stream, pdl, p);
+    static std::atomic<int> known[64][kDirectSplits + 1];
+    int n = known[device][S].load(std::memory_order_acquire);
+    if (n == 0)
+    {
+        auto kernel = attention_direct_kernel<DK, DV, NR>;
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(S);
+        cfg.blockDim = dim3(32 * AS_WARPS);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = S;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if ((S > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess)
+        {
+            cudaGetLastError();
+            n = 0;
+        }
+        known[device][S].store(n > 0 ? n : -1, std::memory_order_release);
+    }
+    return n <= 0 ? 0u : (unsigned int)(S == 1 ? n : S > 8 && S < 16 ? n * 3 / 4 : n * 19 / 20);
 }
 
 // Splits of a unit, from a model fitted to the like kernel of the quantised models (attn_splits of decode_ops.cu, with its
 // measurements): clusters run in rounds on the slots of the GPU; a round of n CTAs takes 4 ns and the larger of 14 ns (a CTA's own
 // pace) and 0.08 n ns (HBM) per row of a split, and 5 us, and 5 more for a second one; a cluster takes 0.15 us per member to meet.
-static unsigned int direct_splits(unsigned long long units, unsigned int len, int sm_count, unsigned int ctas_per_sm)
+// Measured (16384 rows, us, split counts; with slots counted as eight GPCs of equal size and no clusters of more than eight past one
+// CTA per SM / now): 4 sequences of 4 tokens, 8 kv heads of 128, 1 query head each 8: 91.5 / 7: 59.1; 32 sequences of 4 tokens, 4 kv heads
+// of 64 2: 140 / 3: 102; 4 sequences of one token, the same heads 8: 32.0 / 16: 23.1; the other way, where nothing cuts the places up, 4
+// sequences of one token, 8 kv heads of 128, 8 query heads each 8: 52.9 / 7: 57.8.  Over 290 shapes of 256 to 16384 rows the
+// model's choice among 1 to 8 and 16 takes 1.008 times the best one's time, before 1.028.
+template <class Clusters>
+static unsigned int direct_splits(unsigned long long units, unsigned int len, Clusters clusters)
 {
     unsigned int best = 1;
     float least = INFINITY;
-    for (unsigned int S = 1; S <= kDirectSplits; S = S < 8 ? S + 1 : S + 8)
+    for (unsigned int S = 1; S <= kDirectSplits; S++)
     {
         if (S > 1 && len / S < 64u) { break; }
-        const unsigned long long slots = ((unsigned long long)ctas_per_sm * ((unsigned)sm_count / 8) / S) * S * 8;
-        if (slots == 0 || (S > 8 && units * S > (unsigned long long)sm_count)) { break; }
+        if (S > 8 && S < 16 && len / S < 256u) { continue; }    // 1024 rows, 8 units: 11 splits 7.6 us, 8 6.8
+        const unsigned long long slots = (unsigned long long)clusters(S) * S;
+        if (slots == 0 || (S > 8 && units * S > slots)) { continue; }
         const float rows = (float)((len + S - 1) / S);
         auto round = [&](unsigned long long n) { return n == 0 ? 0.f : rows * (4.f + fmaxf(14.f, 0.08f * (float)n)) + 5000.f; };
         const float cost = (float)(units * S / slots) * round(slots) + round(units * S % slots) + 150.f * (float)S + (units * S > slots ? 5000.f : 0.f);
@@ -453,6 +486,14 @@ static unsigned int direct_splits(unsigned long long units, unsigned int len, in
         }
     }
     return best;
+}
+
+template <int DK, int DV, int NR>
+static int run_direct(AttnParams p, unsigned int entries, unsigned int max_len, int device, cudaStream_t stream, bool pdl)
+{
+    p.splits = direct_splits((unsigned long long)entries * p.Hkv * p.row_tiles, max_len, [&](unsigned int S) { return direct_clusters<DK, DV, NR>(S, device); });
+    const dim3 grid(p.splits, p.Hkv * p.row_tiles, entries);
+    return launch_cluster("attention_direct", attention_direct_kernel<DK, DV, NR>, grid, dim3(32 * AS_WARPS), 0, p.splits, stream, pdl, p);
 }
 
 int launch_attention_direct(const AttnParams& p0, unsigned int entries, unsigned int max_n, unsigned int max_len, cudaStream_t stream, bool pdl)
@@ -466,9 +507,14 @@ int launch_attention_direct(const AttnParams& p0, unsigned int entries, unsigned
     const DecoderDevice* dev = decoder_device();
     if (!dev) { return 1; }
     if (p.window != 0 && max_len > p.window + max_n) { max_len = p.window + max_n; }
-    p.splits = direct_splits((unsigned long long)entries * p.Hkv * p.row_tiles, max_len, dev->sm_count, nr == 1 && (p.dim <= 64 || p.vdim <= 64) ? 3 : 2);
-    if (p.dim <= 64) { return p.vdim <= 64 ? run_direct<64, 64>(p, entries, nr, stream, pdl) : run_direct<64, 128>(p, entries, nr, stream, pdl); }
-    return p.vdim <= 64 ? run_direct<128, 64>(p, entries, nr, stream, pdl) : run_direct<128, 128>(p, entries, nr, stream, pdl);
+    auto run = [&](auto dk, auto dv) {
+        constexpr int DK = decltype(dk)::value, DV = decltype(dv)::value;
+        return nr == 1 ? run_direct<DK, DV, 1>(p, entries, max_len, dev->device, stream, pdl) : run_direct<DK, DV, 2>(p, entries, max_len, dev->device, stream, pdl);
+    };
+    using C64 = std::integral_constant<int, 64>;
+    using C128 = std::integral_constant<int, 128>;
+    if (p.dim <= 64) { return p.vdim <= 64 ? run(C64(), C64()) : run(C64(), C128()); }
+    return p.vdim <= 64 ? run(C128(), C64()) : run(C128(), C128());
 }
 
 }    // namespace b200

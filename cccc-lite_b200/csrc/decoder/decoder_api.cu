@@ -46,6 +46,7 @@ const DecoderDevice* decoder_device()
         }
         facts[dev].sm_count = sms;    // two threads may both write the same values: harmless
         facts[dev].max_smem = smem;
+        facts[dev].device = dev;
         ready[dev].store(1, std::memory_order_release);
     }
     return &facts[dev];

@@ -28,7 +28,7 @@ __device__ __forceinline__ void note_timeout(unsigned int* status, unsigned int 
 
 struct DecoderDevice
 {
-    int sm_count = 0, max_smem = 0;
+    int sm_count = 0, max_smem = 0, device = 0;
 };
 const DecoderDevice* decoder_device();
 

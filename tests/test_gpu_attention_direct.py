@@ -48,3 +48,12 @@ def test_scores_of_minus_infinity(D, pos, sink):  # noqa: F811
         w = torch.softmax(torch.cat([z, s[h:h + 1].double()]), 0)[:-1] if sink else torch.softmax(z, 0)
         want = w @ V[1, h // 2, :pos + 1].double()
         assert float((out[1].view(H, d)[h].double() - want).abs().max()) < 2.0 ** -7 * float(want.abs().max())
+
+
+# units that clusters of more than eight have room for and that they have not; a last cluster beyond one round
+@pytest.mark.parametrize("H,Hkv,d,S,n", [(16, 8, 128, 2, 1), (4, 4, 64, 5, 1), (4, 2, 128, 3, 4), (8, 8, 128, 4, 4), (16, 4, 64, 33, 4)])
+def test_long_contexts(D, H, Hkv, d, S, n):  # noqa: F811
+    T = 9000 if S < 10 else 1500
+    rng = np.random.default_rng(S)
+    a = Attn(D, BF16, H, Hkv, d, d, [(s, T - n if s == 0 else int(rng.integers(0, T - n)), n) for s in range(S)], T_max=T, slots=S, scale=0.1, seed=S)
+    close(a.run(4).reshape(S * n, -1), a.reference().reshape(S * n, -1), BF16, (H, Hkv, S, n), 1.5)
