@@ -7,8 +7,8 @@ from __future__ import annotations
 import ctypes as C
 import importlib.util
 import json
-import mmap
 import os
+import sys
 from array import array
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -62,12 +62,16 @@ def _ints(values):
     return (C.c_int * max(1, len(values)))(*values)
 
 
+_malloc, _free = C.pythonapi.PyMem_RawMalloc, C.pythonapi.PyMem_RawFree
+_malloc.restype, _malloc.argtypes, _free.restype, _free.argtypes = _vp, [C.c_size_t], None, [_vp]
+
+
 def _reserve(size):
-    """Address space for `size` bytes whose pages are not made yet."""
-    try:
-        return mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
-    except (OSError, OverflowError) as e:
-        raise MemoryError("no memory for %d bytes of logits" % size) from e
+    """Memory whose pages are not made yet, for _free()."""
+    room = _malloc(size) if size <= sys.maxsize else None
+    if not room:
+        raise MemoryError("no memory for %d bytes of logits" % size)
+    return room
 
 
 def _sampler(sampler):
@@ -112,15 +116,16 @@ class Model:
         wanted = sum(len(w) for _, _, w in entries)
         ch = (C.c_int * max(1, wanted))() if choice else None
         lg = lp = None
+        args = (len(entries), _ints(s for s, _, _ in entries), _ints(len(t) for _, t, _ in entries), _ints(x for _, t, _ in entries for x in t),
+                _ints(len(w) for _, _, w in entries), _ints(x for _, _, w in entries for x in w), bool(logits and wanted), bool(choice))
         # The pages of the logits are made while the step is under way, the room for them is taken before it begins.
         room = _reserve(4 * wanted * self.vocab) if logits and wanted else None
-        rc = self.lib.cccc_model_step_begin(self.h, len(entries), _ints(s for s, _, _ in entries), _ints(len(t) for _, t, _ in entries),
-                                            _ints(x for _, t, _ in entries for x in t), _ints(len(w) for _, _, w in entries),
-                                            _ints(x for _, _, w in entries for x in w), bool(logits and wanted), bool(choice))
+        try:
+            rc = self.lib.cccc_model_step_begin(self.h, *args)
+        finally:
+            _free(room)
         if rc == 0:
             try:
-                if room is not None:
-                    room.close()
                 lg = array("f", (0.0,)) * (wanted * self.vocab) if logits else None
                 lp = (C.c_float * len(lg)).from_buffer(lg) if logits and wanted else None
             finally:
