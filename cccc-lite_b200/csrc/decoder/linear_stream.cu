@@ -1,10 +1,14 @@
 // Linears of a few rows with BF16 weights (weight streaming, HBM-bound), and the linears of the float mode.
 //
-// The streaming kernel: eight warps, WK of which share 16 (or 2 x 16) output features and take the 64-wide k chunks in turn
-// (all eight, or two where k is short).  A lane loads 32 bytes of weight row g and of row g + 8 straight into the A fragments of mma.m16n8k16 - the k order
-// inside a chunk is permuted, identically for both operands, so that fragments are whole pieces of a row - and the rows of X
-// are the eight B columns.  The next chunks' weights are requested before the current ones are consumed, the first ones of
-// a dense member before the previous kernel of the stream has finished.  The warps' partial sums meet in shared memory.
+// The streaming kernel: eight warps, WK of which share 16 (or 2 x 16) output features and take the 64-wide k chunks in
+// turn (all of them, or two where k is short).  A lane loads 32 bytes of weight row g and of row g + 8 straight into the A fragments
+// of mma.m16n8k16 - the k order inside a chunk is permuted, identically for both operands, so that fragments are whole pieces of a
+// row - and the rows of X are the eight B columns.  What bounds it is the stream of weights, and around it, in linears of a few
+// microseconds, the chain from the previous kernel's end to the results: each chunk is requested a turn ahead into the registers of
+// the chunk just used, the first ones of a dense member before the previous kernel of the stream has finished, a task's first ones
+// while the sums of the task before it are made; what the results are added to is fetched before the products.  The warps' partial
+// sums meet in shared memory.  At 8 rows, with two turns of two chunks, one CTA per task and no such prefetch, before: 2048 x 2048
+// 4.2 us, 5120 x 2048 8.2, 6144 x 2048 8.7 (gated 12.7), 2048 x 6144 9.5, 32768 x 2048 27.4; now 3.0, 7.3, 7.3 (11.1), 6.2, 25.1.
 #include "decoder_common.cuh"
 #include "../gemv_decode.cuh"
 #include "linear.cuh"
@@ -17,7 +21,7 @@ constexpr int LS_WARPS = 8;
 struct LinearLaunch
 {
     LinearMember m[LINEAR_MAX_MEMBERS];
-    unsigned int count;
+    unsigned int count, blocks;
 };
 
 // 32 bytes of a weight row, read once
@@ -28,92 +32,152 @@ __device__ __forceinline__ void ldg_stream(const void* p, uint4& a, uint4& b)
                  : "l"(p));
 }
 
-// NT: row groups of eight; RT: 16-feature tiles per warp; U: chunks per loop turn; WK: warps that share features
-template <int NT, int RT, int U, int WK>
-__global__ void __launch_bounds__(32 * LS_WARPS, NT == 4 ? 1 : 2) linear_stream_kernel(const __grid_constant__ LinearLaunch L)
+// What one CTA does at a time: C rows (from n0) of a CTA's share of the features of one group.
+struct StreamTask
 {
-    constexpr int R = 16 * RT, C = 8 * NT;
-    __shared__ float red[LS_WARPS][C][R + 1];
-    unsigned int mi = 0;
-    if (L.count > 1 && blockIdx.x >= L.m[1].block0) { mi = 1; }
-    if (L.count > 2 && blockIdx.x >= L.m[2].block0) { mi = 2; }
-    const LinearMember& m = L.m[mi];
+    unsigned int block, member, slot, fc;    // fc: first feature of the CTA
+    unsigned int group, row0, count, n0;
+};
+
+// NT: row groups of eight; RT: 16-feature tiles per warp; U: chunks per loop turn; WK: warps that share features; OCC: CTAs per SM.
+// A warp adds up its chunks in k order and the warps' sums are added in warp order: the result depends on WK alone, and on no other
+// choice below.
+template <int NT, int RT, int U, int WK, int OCC>
+__global__ void __launch_bounds__(32 * LS_WARPS, OCC) linear_stream_kernel(const __grid_constant__ LinearLaunch L)
+{
+    constexpr int R = 16 * RT, C = 8 * NT, NW = LS_WARPS, T = 32 * NW;
+    constexpr int RED = NW * C * (R + 1);
+    constexpr bool TWO = RED * 8 <= 24 * 1024;    // two places for the partial sums: one barrier per task instead of two
+    constexpr int XD = U < 2 || (NT == 2 && U * RT > 2) ? 1 : 2;    // chunks of X in registers
+    __shared__ float red_all[(TWO ? 2 : 1) * RED];
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const unsigned int b = blockIdx.x - m.block0;
-    const bool gated = activation_gated(m.activation);
-    const unsigned int F = gated ? R / 2 : R;    // output features of a warp
     const unsigned int wk = warp % WK, wf = warp / WK;
-    const unsigned int fb = b % m.fblocks, slot = b / m.fblocks;
-    const unsigned int fc = fb * F * (LS_WARPS / WK), f0 = fc + wf * F;    // first feature of the CTA, of the warp
-    const bool grouped = m.group_offset != nullptr;
     grid_dependency_launch();
-    unsigned int group = 0, row0 = 0, count = m.rows;
-    if (grouped)
-    {
-        grid_dependency_wait();
-        if (m.active != nullptr)
+    bool waited = false;
+
+    // The next task from `block` on (rows n0 ..) that has rows; false: none.  Which rows a group holds is the previous kernel's to say.
+    auto find = [&](unsigned int block, StreamTask& k) {
+        for (; block < L.blocks; block += gridDim.x)
         {
-            const int id = m.active[slot];
-            if (id < 0) { return; }
-            group = (unsigned int)id;
+            unsigned int mi = 0;
+            if (L.count > 1 && block >= L.m[1].block0) { mi = 1; }
+            if (L.count > 2 && block >= L.m[2].block0) { mi = 2; }
+            const LinearMember& m = L.m[mi];
+            const unsigned int b = block - m.block0, fb = b % m.fblocks, slot = b / m.fblocks;
+            k.block = block;
+            k.member = mi;
+            k.slot = slot;
+            k.fc = fb * (activation_gated(m.activation) ? R / 2 : R) * (NW / WK);
+            k.group = m.blocks > 1 ? slot : 0u;
+            k.row0 = 0;
+            k.count = m.rows;
+            k.n0 = 0;
+            if (m.group_offset != nullptr)
+            {
+                if (!waited)
+                {
+                    grid_dependency_wait();
+                    waited = true;
+                }
+                const int id = m.active != nullptr ? m.active[slot] : (int)slot;
+                if (id < 0) { continue; }
+                k.group = (unsigned int)id;
+                k.row0 = (unsigned int)m.group_offset[id];
+                k.count = (unsigned int)m.group_offset[id + 1] - k.row0;
+            }
+            if (k.count != 0) { return true; }
         }
-        else { group = slot; }
-        row0 = (unsigned int)m.group_offset[group];
-        count = (unsigned int)m.group_offset[group + 1] - row0;
-        if (count == 0) { return; }
-    }
-    if (m.blocks > 1) { group = slot; }
-    const __nv_bfloat16* W = (const __nv_bfloat16*)m.W + (size_t)group * m.group_rows * m.ldw;
-    const unsigned int xcol = m.blocks > 1 ? group * m.x_step : 0u, ycol = m.blocks > 1 ? group * m.y_step : 0u;
-    const __nv_bfloat16* wr[RT][2];
+        return false;
+    };
+    const __nv_bfloat16* W = nullptr;
+    unsigned int off[RT][2], chunks = 0;    // rows of the weights in 64 elements, of the task that is being loaded
+    auto aim = [&](const StreamTask& k) {
+        const LinearMember& m = L.m[k.member];
+        const bool gated = activation_gated(m.activation);
+        const unsigned int f0 = k.fc + wf * (gated ? R / 2 : R);
+        W = (const __nv_bfloat16*)m.W + (size_t)k.group * m.group_rows * m.ldw + t * 16;
 #pragma unroll
-    for (int r = 0; r < RT; r++)
-    {
-#pragma unroll
-        for (int h = 0; h < 2; h++)
+        for (int r = 0; r < RT; r++)
         {
-            unsigned int f = f0 + (gated ? 0 : r * 16) + g + h * 8;
-            f = min(f, m.N - 1);    // rows past N: any valid row, the result is not stored
-            wr[r][h] = W + (size_t)(f + (gated && r == 1 ? m.up_row : 0u)) * m.ldw + t * 16;
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+            {
+                unsigned int f = f0 + (gated ? 0 : r * 16) + g + h * 8;
+                f = min(f, m.N - 1);    // rows past N: any valid row, the result is not stored
+                off[r][h] = (f + (gated && r == 1 ? m.up_row : 0u)) * (m.ldw / 64);
+            }
         }
-    }
-    const unsigned int chunks = (m.K + 63) / 64;
-    uint4 a[U][RT][2][2], an[U][RT][2][2];
-    auto load = [&](uint4 (&d)[U][RT][2][2], unsigned int c0) {
-#pragma unroll
-        for (int u = 0; u < U; u++)
+        chunks = (m.K + 63) / 64;
+    };
+    // A chunk's weights are requested a whole turn before their use, into the registers of the chunk just used: of the next
+    // task's where a task ends, so that the stream does not stop while sums are made.
+    uint4 a[U][RT][2][2];
+    auto load = [&](int u, unsigned int c) {
+        if (c < chunks)
         {
-            const unsigned int c = c0 + u * WK;
-            if (c < chunks)
+#pragma unroll
+            for (int r = 0; r < RT; r++)
             {
 #pragma unroll
-                for (int r = 0; r < RT; r++)
-                {
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-                    {
-                        ldg_stream(wr[r][h] + c * 64, d[u][r][h][0], d[u][r][h][1]);
-                    }
-                }
+                for (int h = 0; h < 2; h++) { ldg_stream(W + ((size_t)off[r][h] + c) * 64, a[u][r][h][0], a[u][r][h][1]); }
             }
         }
     };
-    load(a, wk);
-    if (!grouped) { grid_dependency_wait(); }
-    for (unsigned int n0 = 0; n0 < count; n0 += C)
+    StreamTask k;
+    bool more = find(blockIdx.x, k);
+    if (more)
     {
-        if (n0 != 0) { load(a, wk); }
+        aim(k);
+#pragma unroll
+        for (int u = 0; u < U; u++) { load(u, wk + u * WK); }
+    }
+    if (!waited) { grid_dependency_wait(); }
+    waited = true;
+    for (unsigned int turn_of_red = 0; more; turn_of_red ^= 1)
+    {
+        const LinearMember& m = L.m[k.member];
+        float* red = red_all + (TWO ? turn_of_red * RED : 0);
+        const bool gated = activation_gated(m.activation);
+        const unsigned int xcol = m.blocks > 1 ? k.group * m.x_step : 0u, ycol = m.blocks > 1 ? k.group * m.y_step : 0u;
         const __nv_bfloat16* xr[NT];
         bool live[NT];
 #pragma unroll
         for (int nt = 0; nt < NT; nt++)
         {
-            const unsigned int n = n0 + nt * 8 + g;
-            live[nt] = n < count;
-            unsigned int r = row0 + (live[nt] ? n : 0u);
+            const unsigned int n = k.n0 + nt * 8 + g;
+            live[nt] = n < k.count;
+            unsigned int r = k.row0 + (live[nt] ? n : 0u);
             if (m.x_row != nullptr) { r = (unsigned int)m.x_row[r]; }
             xr[nt] = (const __nv_bfloat16*)m.X + (size_t)r * m.ldx + xcol + t * 16;
         }
+        const unsigned int here = chunks;
+        uint4 x[XD][NT][2];
+        auto load_x = [&](int d, unsigned int c) {
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++)
+            {
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                {
+                    x[d][nt][q] = make_uint4(0, 0, 0, 0);
+                    if (live[nt] && c < here) { x[d][nt][q] = *reinterpret_cast<const uint4*>(xr[nt] + c * 64 + q * 8); }
+                }
+            }
+        };
+#pragma unroll
+        for (int d = 0; d < XD; d++) { load_x(d, wk + d * WK); }
+        // what the results are added to, fetched while the products are made
+        const unsigned int cols = min((unsigned int)C, k.count - k.n0);
+        const unsigned int F = gated ? R / 2 : R, all = F * (NW / WK);    // output features of a warp, of the CTA
+        float old = 0.f;
+        const bool adds = m.accumulate != 0 && threadIdx.x < cols * all && k.fc + threadIdx.x % all < m.N;
+        if (adds) { old = ((const float*)m.Y)[(size_t)(k.row0 + k.n0 + threadIdx.x / all) * m.ldy + ycol + k.fc + threadIdx.x % all]; }
+        // the task after this one
+        StreamTask nk = k;
+        bool again = true;
+        if (k.n0 + C < k.count) { nk.n0 = k.n0 + C; }
+        else { again = find(k.block + gridDim.x, nk); }
+
         float acc[RT][NT][4];
 #pragma unroll
         for (int r = 0; r < RT; r++)
@@ -125,86 +189,70 @@ __global__ void __launch_bounds__(32 * LS_WARPS, NT == 4 ? 1 : 2) linear_stream_
                 for (int j = 0; j < 4; j++) { acc[r][nt][j] = 0.f; }
             }
         }
-        for (unsigned int c0 = wk; c0 < chunks; c0 += U * WK)
+        const unsigned int turns = (here + U * WK - 1) / (U * WK);    // the same for every warp
+        for (unsigned int turn = 0; turn < turns; turn++)
         {
-            load(an, c0 + U * WK);
+            const unsigned int c0 = wk + turn * (U * WK);
+            const bool last = turn + 1 == turns;
+            if (last && again) { aim(nk); }
+            const unsigned int next = last ? wk : c0 + U * WK;
 #pragma unroll
             for (int u = 0; u < U; u++)
             {
-                const unsigned int c = c0 + u * WK;
-                if (c >= chunks) { break; }
-                uint4 x[NT][2];
-#pragma unroll
-                for (int nt = 0; nt < NT; nt++)
+                if (c0 + u * WK < here)
                 {
 #pragma unroll
-                    for (int k = 0; k < 2; k++)
-                    {
-                        x[nt][k] = make_uint4(0, 0, 0, 0);
-                        if (live[nt]) { x[nt][k] = *reinterpret_cast<const uint4*>(xr[nt] + c * 64 + k * 8); }
-                    }
-                }
-#pragma unroll
-                for (int nt = 0; nt < NT; nt++)
-                {
-#pragma unroll
-                    for (int k = 0; k < 2; k++)
+                    for (int nt = 0; nt < NT; nt++)
                     {
 #pragma unroll
-                        for (int r = 0; r < RT; r++)
+                        for (int q = 0; q < 2; q++)
                         {
-                            mma_bf16_16816(acc[r][nt], a[u][r][0][k].x, a[u][r][1][k].x, a[u][r][0][k].y, a[u][r][1][k].y, x[nt][k].x, x[nt][k].y);
-                            mma_bf16_16816(acc[r][nt], a[u][r][0][k].z, a[u][r][1][k].z, a[u][r][0][k].w, a[u][r][1][k].w, x[nt][k].z, x[nt][k].w);
+                            const uint4 b = x[u % XD][nt][q];
+#pragma unroll
+                            for (int r = 0; r < RT; r++)
+                            {
+                                mma_bf16_16816(acc[r][nt], a[u][r][0][q].x, a[u][r][1][q].x, a[u][r][0][q].y, a[u][r][1][q].y, b.x, b.y);
+                                mma_bf16_16816(acc[r][nt], a[u][r][0][q].z, a[u][r][1][q].z, a[u][r][0][q].w, a[u][r][1][q].w, b.z, b.w);
+                            }
                         }
                     }
                 }
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++)
-            {
-#pragma unroll
-                for (int r = 0; r < RT; r++)
-                {
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-                    {
-                        a[u][r][h][0] = an[u][r][h][0];
-                        a[u][r][h][1] = an[u][r][h][1];
-                    }
-                }
+                if (XD == 1) { load_x(0, c0 + (u + 1) * WK); }
+                if (!last || again) { load(u, next + u * WK); }
+                if (XD != 1) { load_x(u % XD, c0 + (u + XD) * WK); }
             }
         }
-        if (n0 != 0) { __syncthreads(); }
+        if (!TWO) { __syncthreads(); }    // the last task's sums have been read
 #pragma unroll
         for (int r = 0; r < RT; r++)
         {
 #pragma unroll
             for (int nt = 0; nt < NT; nt++)
             {
-                red[warp][nt * 8 + 2 * t][r * 16 + g] = acc[r][nt][0];
-                red[warp][nt * 8 + 2 * t + 1][r * 16 + g] = acc[r][nt][1];
-                red[warp][nt * 8 + 2 * t][r * 16 + g + 8] = acc[r][nt][2];
-                red[warp][nt * 8 + 2 * t + 1][r * 16 + g + 8] = acc[r][nt][3];
+#pragma unroll
+                for (int j = 0; j < 4; j++) { red[(warp * C + nt * 8 + 2 * t + (j & 1)) * (R + 1) + r * 16 + g + 8 * (j >> 1)] = acc[r][nt][j]; }
             }
         }
         __syncthreads();
-        const unsigned int cols = min((unsigned int)C, count - n0);
-        const unsigned int all = F * (LS_WARPS / WK);
-        for (unsigned int i = threadIdx.x; i < cols * all; i += 32 * LS_WARPS)
+        for (unsigned int i = threadIdx.x; i < cols * all; i += T)
         {
             const unsigned int f = i % all, n = i / all, w0 = f / F * WK, fl = f % F;
-            if (fc + f >= m.N) { continue; }
+            if (k.fc + f >= m.N) { continue; }
             float v = 0.f, up = 0.f;
 #pragma unroll
-            for (int w = 0; w < WK; w++) { v += red[w0 + w][n][fl]; }
+            for (int w = 0; w < WK; w++) { v += red[((w0 + w) * C + n) * (R + 1) + fl]; }
             if (gated)
             {
 #pragma unroll
-                for (int w = 0; w < WK; w++) { up += red[w0 + w][n][16 + fl]; }
+                for (int w = 0; w < WK; w++) { up += red[((w0 + w) * C + n) * (R + 1) + (RT == 2 ? 16 : 0) + fl]; }
             }
-            const float y = linear_activation<true>(m.activation, m.alpha * v, m.alpha * up, m.cap);
-            linear_store(m, row0 + n0 + n, ycol + fc + f, y * linear_row_factor<__nv_bfloat16>(m, row0 + n0 + n, group));
+            const unsigned int row = k.row0 + k.n0 + n;
+            const float y = linear_activation<true>(m.activation, m.alpha * v, m.alpha * up, m.cap) * linear_row_factor<__nv_bfloat16>(m, row, k.group);
+            if (adds && i == threadIdx.x) { ((float*)m.Y)[(size_t)row * m.ldy + ycol + k.fc + f] = old + y; }
+            else { linear_store(m, row, ycol + k.fc + f, y); }
         }
+        k = nk;
+        more = again;
     }
 }
 
@@ -287,31 +335,57 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const LinearMember m)
     }
 }
 
-template <int NT, int RT, int U, int WK>
-static int launch_stream_wk(LinearLaunch& L, cudaStream_t st, bool pdl)
+template <int NT, int RT, int U, int WK, int OCC>
+static int launch_stream_wk(LinearLaunch& L, unsigned int sm_count, unsigned int waves, cudaStream_t st, bool pdl)
 {
-    unsigned int blocks = 0;
+    L.blocks = 0;
     for (unsigned int j = 0; j < L.count; j++)
     {
         LinearMember& m = L.m[j];
         const unsigned int F = (activation_gated(m.activation) ? 8 * RT : 16 * RT) * (LS_WARPS / WK);
         m.fblocks = (m.N + F - 1) / F;
-        m.block0 = blocks;
-        blocks += m.fblocks * m.slots;
+        m.block0 = L.blocks;
+        L.blocks += m.fblocks * m.slots;
     }
+    const unsigned int places = sm_count * OCC;
     // The rows of X are read through L1, of which a kernel with much shared memory just before would otherwise leave little.
     static std::atomic<unsigned long long> done{ 0 };
-    prefer_l1(linear_stream_kernel<NT, RT, U, WK>, done);
-    return launch_kernel("linear_stream", linear_stream_kernel<NT, RT, U, WK>, dim3(blocks), dim3(32 * LS_WARPS), 0, st, pdl, L);
+    prefer_l1(linear_stream_kernel<NT, RT, U, WK, OCC>, done);
+    const unsigned int grid = L.blocks > places && L.blocks / places < waves ? places : L.blocks;
+    return launch_kernel("linear_stream", linear_stream_kernel<NT, RT, U, WK, OCC>, dim3(grid), dim3(32 * LS_WARPS), 0, st, pdl, L);
 }
 
+// Which form a launch takes (one linear in a CUDA graph of distinct weights, microseconds at 8 / 16 / 32 rows):
+//   * CTAs that take task after task, or one for each task?  Taking the next task hides its first loads behind this one's sums, a CTA
+//     of its own fits itself to what an SM gets done.  Up to 8 rows dense tasks gain nothing (5120 x 2048: 7.3 either way, at 1 row
+//     7.3 against 6.0; 32768 x 2048: 28.4 against 25.1), gated ones up to four rounds do (6144 x 2048: 11.1 against 12.0; 12288 x 4096
+//     either way 33.4); more rows do at any number (32768 x 2048: 28.7 / 45.8 against 30.1 / 51.3).
+//   * Chunks in flight: a whole k of 2048 (four per warp) up to 8 rows, two where k is longer (4096 x 12288: 20.5 with four, 18.1;
+//     151936 x 4096: 218 with four, 202.5) and up to 16 rows, where registers are short (4096 x 4096: 9.7, 8.0).
+//   * One CTA per SM with twice the chunks in flight where the tasks are fewer than the SMs and k is long: 2048 x 6144 9.5, 6.2.
 template <int NT, int RT, int U>
 static int launch_stream(LinearLaunch& L, cudaStream_t st, bool pdl)
 {
+    const DecoderDevice* dev = decoder_device();
+    if (!dev) { return 1; }
+    const unsigned int sms = (unsigned int)dev->sm_count, waves = NT > 1 ? 0xFFFFFFFFu : RT == 2 ? 4u : 1u;
+    unsigned int longest = 0, blocks = 0;
+    for (unsigned int j = 0; j < L.count; j++)
+    {
+        const LinearMember& m = L.m[j];
+        longest = m.K > longest ? m.K : longest;
+        const unsigned int F = activation_gated(m.activation) ? 8 * RT : 16 * RT;
+        blocks += (m.N + F - 1) / F * m.slots;
+    }
     // eight warps over few chunks would leave some without any; the members of a launch take one form
-    unsigned int longest = 0;
-    for (unsigned int j = 0; j < L.count; j++) { longest = L.m[j].K > longest ? L.m[j].K : longest; }
-    return longest <= 1024 ? launch_stream_wk<NT, RT, U, 2>(L, st, pdl) : launch_stream_wk<NT, RT, U, 8>(L, st, pdl);
+    constexpr int OCC = NT == 4 ? 1 : 2;
+    if (longest <= 1024) { return launch_stream_wk<NT, RT, U, 2, OCC>(L, sms, waves, st, pdl); }
+    if constexpr (NT == 1)
+    {
+        if (blocks <= sms && longest >= 4096) { return launch_stream_wk<NT, RT, 2 * U, 8, 1>(L, sms, waves, st, pdl); }
+        if (RT == 1 && longest > 2048) { return launch_stream_wk<NT, RT, 2, 8, OCC>(L, sms, waves, st, pdl); }
+    }
+    return launch_stream_wk<NT, RT, U, 8, OCC>(L, sms, waves, st, pdl);
 }
 
 }    // namespace b200
@@ -424,9 +498,9 @@ C_EXPORT int cuda_b200_linear_rows(int dtype, unsigned int count, const cuda_b20
             }
             if (part.count == 0) { continue; }
             int rc;
-            if (width == 8) { rc = gated ? launch_stream<1, 2, 1>(part, st, pdl) : launch_stream<1, 1, 2>(part, st, pdl); }
-            else if (width == 16) { rc = gated ? launch_stream<2, 2, 1>(part, st, pdl) : launch_stream<2, 1, 2>(part, st, pdl); }
-            else { rc = launch_stream<4, 2, 1>(part, st, pdl); }
+            if (width == 8) { rc = gated ? launch_stream<1, 2, 2>(part, st, pdl) : launch_stream<1, 1, 4>(part, st, pdl); }
+            else if (width == 16) { rc = gated ? launch_stream<2, 2, 2>(part, st, pdl) : launch_stream<2, 1, 2>(part, st, pdl); }
+            else { rc = launch_stream<4, 2, 2>(part, st, pdl); }
             if (rc) { return rc; }
         }
         return 0;

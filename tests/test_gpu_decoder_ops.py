@@ -237,6 +237,34 @@ def test_a_group_of_members_is_the_separate_launches(D):
         close(host(Y)[:, :N], want, FLOAT, N, 10)
 
 
+@pytest.mark.parametrize("rows,members", [
+    (3, [(4997, 200, 0)]),                                # more tasks than places, a CTA for each
+    (7, [(2500, 1088, 2)]),                               # gated: CTAs that take a second task, its k no multiple of a turn
+    (8, [(100, 4160, 0), (60, 64, 1)]),                   # one CTA per SM, a member with a single chunk of k
+    (5, [(130, 4096, 2)]),
+    (8, [(70, 6144, 0)]),
+    (12, [(5000, 1100, 0), (2500, 128, 2), (300, 2112, 1)]),    # 9 to 16 rows, members of unlike k one behind the other
+    (16, [(2600, 1344, 2)]),
+    (27, [(9700, 256, 0), (70, 1032, 2)]),                # 17 to 32 rows
+])
+def test_streaming_tasks_one_behind_the_other(D, rows, members):
+    """Sizes at which a CTA of the streaming kernel goes from task to task, or takes another form."""
+    rng = np.random.default_rng(rows + len(members))
+    descs, checks = [], []
+    for N, K, act in members:
+        w, x = rand(rng, 2 * N if act == 2 else N, K, scale=K ** -0.5), rand(rng, rows, K)
+        start = rng.standard_normal((rows, N)).astype(np.float32)
+        W, X, Y = padded(w, BF16), padded(x, BF16, junk=3.0), padded(start, FLOAT, N + 3, junk=-3.0)
+        full = x.astype(np.float64) @ w.T.astype(np.float64)
+        descs.append(D.fill(D.Linear, W=W, X=X, Y=Y, rows=rows, N=N, K=K, ldw=pad64(K), ldx=pad64(K), ldy=N + 3, up_row=N, activation=act, accumulate=1, alpha=1.0))
+        checks.append((W, X, Y, N, K, start + act_ref(act, full[:, :N], full[:, N:])))
+    assert D.linear(BF16, descs, flags=1, kernel=1) == 0 and D.check() == 0
+    for W, X, Y, N, K, want in checks:
+        # a warp's products of 16 k add up one behind the other: K / 16 roundings of 2^-23 (the tensor cores truncate) at most, spread over eight warps
+        close(host(Y)[:, :N], want, FLOAT, (N, K), max(10, K / 16 / 8 * 2 ** -23 / TOL[FLOAT]) + 10)
+        assert np.all(host(Y)[:, N:] == -3.0)
+
+
 def test_descriptors_that_are_not_taken(D):
     X = padded(np.ones((2, 64)), BF16)
     base = dict(W=X, X=X, Y=X, rows=2, N=2, K=64, ldw=64, ldx=64, ldy=64, alpha=1.0)
