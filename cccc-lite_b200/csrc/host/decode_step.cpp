@@ -382,7 +382,7 @@ bool DecodeStep::load(GpuControl* gpu, const BinFile& file, const ModelConfig& c
     // (the step's stream does not wait for the default stream: its zeros are written on it)
     const bool cleared = cudaMemsetAsync(d_ids_, 0, (size_t)max_batch * 16, gpu_->stream()) == cudaSuccess;
     if (tp_) { tp_->barrier(); }
-    const int rc = cleared ? issue(1, gpu_->stream()) : -1;
+    const int rc = cleared ? issue(1, gpu_->stream(), false) : -1;
     gpu_->synchronize();
     const bool stepped = rc >= 0 && cuda_check_error("decode step warm-up") == 0;
     launches_per_step_ = rc;
@@ -480,7 +480,7 @@ bool DecodeStep::loadTensors(const BinFile& file, std::string* err)
         cudaMemset(seq_counters_, 0, cb);
         if (tp_->nMax() < (unsigned int)(B * cfg.hidden)) { return fail(err, "the exchange areas are smaller than max_batch * hidden"); }
     }
-    graphs_.assign(max_batch + 1, nullptr);
+    graphs_.assign(2 * (max_batch + 1), nullptr);
     // The default stream's copies and the zeros above end before anything runs on the step's own stream, which is not ordered behind it.
     if (cudaDeviceSynchronize() != cudaSuccess) { return fail(err, "a CUDA error while loading"); }
     return true;
@@ -516,7 +516,7 @@ void DecodeStep::groupGateUp(const Layer& L, uint16_t* out, cuda_wq_linear* g) c
     g[1] = member(L.up.w, L.up.s, L.up.inv, ffn_loc_, out + ffn_loc_, cfg_.hidden, 2 * ffn_loc_);
 }
 
-int DecodeStep::issue(int M, cudaStream_t st)
+int DecodeStep::issue(int M, cudaStream_t st, bool direct)
 {
     const unsigned int PDL = 1u, RES = 8u;
     const int wt = (int)wt_;
@@ -559,8 +559,8 @@ int DecodeStep::issue(int M, cudaStream_t st)
         pending = tp;
     }
     norm(final_norm_, pending);
-    ok(cuda_gemm_wq_bf16(wt, lm_head_.w, lm_head_.s, lm_head_.inv, xn_, logits_, vocab_loc_, M, hid, hid, hid, vocab_loc_, 1, 1.0f, 0.0f, st, PDL));
-    ok(cuda_argmax_bf16(logits_, M, vocab_loc_, vocab_loc_, d_ids_, d_best_, st));
+    ok(cuda_gemm_wq_bf16(wt, lm_head_.w, lm_head_.s, lm_head_.inv, xn_, direct ? h_logits_ : logits_, vocab_loc_, M, hid, hid, hid, vocab_loc_, 1, 1.0f, 0.0f, st, PDL));
+    if (!direct) { ok(cuda_argmax_bf16(logits_, M, vocab_loc_, vocab_loc_, d_ids_, d_best_, st)); }
     return bad ? -1 : n;
 }
 
@@ -826,13 +826,13 @@ bool DecodeStep::useProgram(bool on)
 
 int DecodeStep::step(const int* token_ids, const int* positions, int M, int* next_ids, float* best_logits, uint16_t* logits_host, const int* slots)
 {
-    int rc = launch(token_ids, positions, M, logits_host != nullptr, slots);
+    int rc = launch(token_ids, positions, M, logits_host != nullptr, true, slots);
     if (rc == 0) { rc = finish(next_ids, best_logits); }
     if (rc == 0 && logits_host) { std::memcpy(logits_host, h_logits_, (size_t)M * vocab_loc_ * 2); }
     return rc;
 }
 
-int DecodeStep::launch(const int* token_ids, const int* positions, int M, bool logits, const int* slots)
+int DecodeStep::launch(const int* token_ids, const int* positions, int M, bool logits, bool choice, const int* slots)
 {
     if (M < 1 || M > max_batch_) { return -1; }
     gpu_->setAsCurrent();
@@ -844,25 +844,39 @@ int DecodeStep::launch(const int* token_ids, const int* positions, int M, bool l
         h_slot_[i] = slots ? slots[i] : i;
     }
     // ids, positions and slots lie one behind the other, here and on the device
-    cudaMemcpyAsync(d_ids_, h_ids_, (size_t)max_batch_ * 12, cudaMemcpyHostToDevice, st);
+    auto upload = [&] { return cudaMemcpyAsync(d_ids_, h_ids_, (size_t)max_batch_ * 12, cudaMemcpyHostToDevice, st) == cudaSuccess; };
+    // the chosen ids and, behind two other arrays, their logits; the status word
+    auto download = [&](bool chosen) {
+        if (chosen) { cudaMemcpyAsync(h_out_, d_ids_, (size_t)max_batch_ * 16, cudaMemcpyDeviceToHost, st); }
+        return cuda_b200_status(h_status_, st);
+    };
     int rc = 0;
+    // Logits that the host wants without the greedy choice, which reads them again, are written into its memory by the head's linear:
+    // they cross the bus while the weights are read.
+    bool direct = false;
     if (use_program_ && M == 1 && program_)
     {
-        rc = cuda_embed_bf16(d_ids_, emb_, x_, cfg_.hidden, 1, cfg_.vocab, st, 0);
+        rc = upload() ? 0 : 1;
+        rc |= cuda_embed_bf16(d_ids_, emb_, x_, cfg_.hidden, 1, cfg_.vocab, st, 0);
         rc |= cuda_decode_program_launch(program_, st);
         rc |= cuda_argmax_bf16(logits_, 1, vocab_loc_, vocab_loc_, d_ids_, d_best_, st);
+        rc |= download(true);
         last_launches_ = 3;
     }
     else
     {
-        if (!graphs_[M])
+        direct = logits && !choice && world_ == 1 && M <= kDirectRows;
+        cudaGraphExec_t& step = graphs_[M + (direct ? max_batch_ + 1 : 0)];
+        if (!step)
         {
-            // the first step for this M records the launches; later ones replay the graph
+            // the first step for this M records the launches, and the copies around them; later ones replay the graph
             cudaGraph_t graph = nullptr;
             if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { return 1; }
-            const int n = issue(M, st);
+            const bool sent = upload();
+            const int n = issue(M, st, direct);
+            const bool good = download(!direct) == 0 && sent;
             const cudaError_t e = cudaStreamEndCapture(st, &graph);
-            if (n < 0 || e != cudaSuccess || !graph)
+            if (n < 0 || !good || e != cudaSuccess || !graph)
             {
                 if (graph) { cudaGraphDestroy(graph); }
                 cudaGetLastError();
@@ -872,17 +886,14 @@ int DecodeStep::launch(const int* token_ids, const int* positions, int M, bool l
             const cudaError_t ei = cudaGraphInstantiate(&exec, graph, 0);
             cudaGraphDestroy(graph);
             if (ei != cudaSuccess) { return 1; }
-            graphs_[M] = exec;
+            step = exec;
         }
         // every rank is about to launch: the exchange inside the row-parallel linears waits for the peers
         if (tp_ && world_ > 1) { tp_->barrier(); }
-        rc = cudaGraphLaunch(graphs_[M], st) == cudaSuccess ? 0 : 1;
-        last_launches_ = launches_per_step_;
+        rc = cudaGraphLaunch(step, st) == cudaSuccess ? 0 : 1;
+        last_launches_ = launches_per_step_ - (direct ? 1 : 0);
     }
-    // the chosen ids and, behind two other arrays, their logits
-    cudaMemcpyAsync(h_out_, d_ids_, (size_t)max_batch_ * 16, cudaMemcpyDeviceToHost, st);
-    rc |= cuda_b200_status(h_status_, st);
-    if (logits) { cudaMemcpyAsync(h_logits_, logits_, (size_t)M * vocab_loc_ * 2, cudaMemcpyDeviceToHost, st); }
+    if (logits && !direct) { cudaMemcpyAsync(h_logits_, logits_, (size_t)M * vocab_loc_ * 2, cudaMemcpyDeviceToHost, st); }
     running_ = M;
     if (rc != 0) { finish(h_out_, nullptr); }    // nothing stays under way
     return rc;

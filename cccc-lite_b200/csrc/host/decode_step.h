@@ -93,8 +93,9 @@ public:
     // slots (nullable): the cache slot of each sequence; without it sequence i has slot i.
     int step(const int* token_ids, const int* positions, int M, int* next_ids, float* best_logits, uint16_t* logits_host, const int* slots = nullptr);
     // The same in two halves: launch() starts the step (and the way of the logits to the host); where it returns 0, finish() waits
-    // for it, after which hostLogits() holds the [M][vocab / world] logits until the next launch.
-    int launch(const int* token_ids, const int* positions, int M, bool logits, const int* slots);
+    // for it, after which hostLogits() holds the [M][vocab / world] logits until the next launch.  choice false: the ids and logits
+    // that finish() gives stand for nothing.
+    int launch(const int* token_ids, const int* positions, int M, bool logits, bool choice, const int* slots);
     int finish(int* next_ids, float* best_logits);
     const uint16_t* hostLogits() const { return h_logits_; }
     // New tokens of one sequence, which continue row `pos` of cache slot `slot`.
@@ -151,7 +152,7 @@ private:
     bool loadTensors(const BinFile& file, std::string* err);
     bool loadLinear(const BinFile& f, const std::string& name, int N, int K, char kind, Linear* out, std::string* err);
     bool loadBf16(const BinFile& f, const std::string& name, size_t n, uint16_t** out, bool required, std::string* err);
-    int issue(int M, cudaStream_t st);
+    int issue(int M, cudaStream_t st, bool direct);    // direct: the logits go to the host's memory, nothing is chosen
     void groupQkv(const Layer& L, uint16_t* out, cuda_wq_linear* g) const;
     void groupGateUp(const Layer& L, uint16_t* out, cuda_wq_linear* g) const;
     cuda_attn_decode attnArgs(size_t layer, int M) const;
@@ -180,7 +181,8 @@ private:
     std::vector<Stored> stored_;
     std::vector<std::pair<std::string, std::vector<uint16_t>>> plain_;    // norm weights and the embedding, as BF16
     bool keep_host_ = false;
-    std::vector<cudaGraphExec_t> graphs_;    // index M
+    static constexpr int kDirectRows = 16;
+    std::vector<cudaGraphExec_t> graphs_;    // index M, then those that write the logits directly
     ::cuda_decode_program* program_ = nullptr;
     bool use_program_ = false;
     size_t weight_bytes_ = 0;

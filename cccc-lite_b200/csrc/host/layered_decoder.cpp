@@ -384,7 +384,7 @@ void LayeredDecoder::makePass(const std::vector<StepEntry>& entries, const std::
     }
 }
 
-int LayeredDecoder::issueHead(const Pass& p, int row0, int rows, cudaStream_t st)
+int LayeredDecoder::issueHead(const Pass& p, int row0, int rows, cudaStream_t st, bool direct)
 {
     const unsigned int PDL = 1u;
     int bad = 0, n = 0;
@@ -407,18 +407,18 @@ int LayeredDecoder::issueHead(const Pass& p, int row0, int rows, cudaStream_t st
     cuda_b200_linear h = {};
     h.W = head_.w;
     h.X = head_x_;
-    h.Y = logits_;
+    h.Y = direct ? h_logits_ : logits_;
     h.rows = (unsigned int)rows;
     h.N = (unsigned int)spec_.vocab;
     h.K = (unsigned int)spec_.width;
     h.ldw = (unsigned int)head_.ld;
     h.ldx = (unsigned int)ldw_;
-    h.ldy = (unsigned int)ld_logits_;
+    h.ldy = (unsigned int)(direct ? spec_.vocab : ld_logits_);
     h.alpha = spec_.logit_scale;
     h.cap = spec_.logit_softcap;
     if (h.cap > 0.f) { h.activation = B200_ACT_SOFTCAP; }
     ok(cuda_b200_linear_rows(act(), 1, &h, st, PDL, 0));
-    ok(cuda_b200_argmax_f32(logits_, (unsigned int)rows, (unsigned int)spec_.vocab, (unsigned int)ld_logits_, d_choice_, d_best_, st, PDL));
+    if (!direct) { ok(cuda_b200_argmax_f32(logits_, (unsigned int)rows, (unsigned int)spec_.vocab, (unsigned int)ld_logits_, d_choice_, d_best_, st, PDL)); }
     return bad ? -1 : n;
 }
 
@@ -573,17 +573,20 @@ void LayeredDecoder::sendResults(int rows, bool logits, bool choice)
     }
 }
 
-// Row i goes to row place[i] of `logits`: a piece is copied on while the next one arrives.
-int LayeredDecoder::takeResults(int rows, const int* place, float* logits, int* choice)
+// Row i goes to row place[i] of `logits`: a piece is copied on while the next one arrives (the device has written all of them where
+// the head wrote them itself).
+int LayeredDecoder::takeResults(int rows, const int* place, float* logits, int* choice, bool direct)
 {
     const size_t V = (size_t)spec_.vocab;
+    if (direct && cudaStreamSynchronize(gpu_.stream()) != cudaSuccess) { return 1; }
     for (int i = 0; i < kPieces && logits; i++)
     {
         const size_t r0 = (size_t)rows * i / kPieces, r1 = (size_t)rows * (i + 1) / kPieces;
         if (r0 == r1) { continue; }
-        if (cudaEventSynchronize(piece_[i]) != cudaSuccess) { return 1; }
+        if (!direct && cudaEventSynchronize(piece_[i]) != cudaSuccess) { return 1; }
         for (size_t r = r0; r < r1; r++) { std::memcpy(logits + (size_t)place[r] * V, h_logits_ + r * V, V * 4); }
     }
+    if (direct) { return 0; }
     if (cudaStreamSynchronize(gpu_.stream()) != cudaSuccess) { return 1; }
     for (int r = 0; r < rows && choice; r++) { choice[place[r]] = h_choice_[r]; }
     return 0;
@@ -597,18 +600,34 @@ int LayeredDecoder::decodeBucket(const Pass& p, int rows)
     return std::min(len, rows);
 }
 
+// The head's linear writes the logits of a decode step's rows into the host's memory itself where they are wanted there and the greedy
+// choice, which reads them again, is not: they cross the bus while the weights are read, and nothing has to be copied behind it.
+bool LayeredDecoder::writesDirectly(const Pass& p, bool logits, bool choice) const
+{
+    return p.decode && logits && !choice && dtype_ == BFLOAT16 && p.wants <= kDirectRows;
+}
+
+// A decode step behind its arrays' copy: the pass, the head; where that writes directly, the status word follows.
+int LayeredDecoder::issueDecode(const Pass& p, bool direct, cudaStream_t st)
+{
+    const int body = issue(p, st), head = body < 0 ? -1 : issueHead(p, 0, p.wants, st, direct);
+    if (head >= 0 && direct && cuda_b200_decoder_status(h_status_, st) != 0) { return -1; }
+    return head < 0 ? -1 : body + head;
+}
+
 // Starts a decode step whose graph there is; its results (as asked for) follow it to the host.
 int LayeredDecoder::startDecode(const Pass& p, bool logits, bool choice, bool* started)
 {
     cudaStream_t st = gpu_.stream();
     *started = false;
     if (!p.decode || p.wants > want_cap_) { return 0; }
-    auto it = graphs_.find({ p.entries, decodeBucket(p, cache_.rows()) });
+    const bool direct = writesDirectly(p, logits, choice);
+    auto it = graphs_.find({ p.entries, decodeBucket(p, cache_.rows()), direct });
     if (it == graphs_.end()) { return 0; }
     std::memcpy(h_meta_, p.host.data(), p.host.size() * 4);
-    if (cudaMemcpyAsync(d_meta_, h_meta_, p.host.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess || cudaGraphLaunch(it->second.first, st) != cudaSuccess) { return 1; }
+    if (cudaGraphLaunch(it->second.first, st) != cudaSuccess) { return 1; }
     last_launches_ += it->second.second;
-    sendResults(p.wants, logits, choice);
+    if (!direct) { sendResults(p.wants, logits, choice); }
     *started = true;
     return 0;
 }
@@ -619,27 +638,29 @@ int LayeredDecoder::run(const Pass& p, const std::vector<int>& place, float* log
     cudaStream_t st = gpu_.stream();
     bool started = false;
     if (startDecode(p, logits != nullptr, choice != nullptr, &started)) { return 1; }
-    if (started) { return takeResults(p.wants, place.data(), logits, choice); }
+    const bool direct = writesDirectly(p, logits != nullptr, choice != nullptr);
+    if (started) { return takeResults(p.wants, place.data(), logits, choice, direct); }
     std::memcpy(h_meta_, p.host.data(), p.host.size() * 4);
-    if (cudaMemcpyAsync(d_meta_, h_meta_, p.host.size() * 4, cudaMemcpyHostToDevice, st) != cudaSuccess) { return 1; }
+    auto upload = [&] { return cudaMemcpyAsync(d_meta_, h_meta_, p.host.size() * 4, cudaMemcpyHostToDevice, st) == cudaSuccess; };
+    if (!upload()) { return 1; }
     const unsigned long long before = cuda_b200_decoder_launches();
     auto fetch = [&](int row0, int rows) {
-        sendResults(rows, logits != nullptr, choice != nullptr);
-        return takeResults(rows, place.data() + row0, logits, choice) == 0;
+        if (!direct) { sendResults(rows, logits != nullptr, choice != nullptr); }
+        return takeResults(rows, place.data() + row0, logits, choice, direct) == 0;
     };
     if (p.decode && p.wants <= want_cap_)
     {
         Pass q = p;
         const int len = q.parts[0].max_len = decodeBucket(p, cache_.rows());
         // the first step of this shape runs launch by launch (which also loads the kernels), then the launches are recorded
-        if (issue(q, st) < 0 || issueHead(q, 0, q.wants, st) < 0) { return -1; }
+        if (issueDecode(q, direct, st) < 0) { return -1; }
         const int launches = (int)(cuda_b200_decoder_launches() - before);
         last_launches_ += launches;
         if (!fetch(0, p.wants)) { return 1; }
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { return 1; }
-        const bool recorded = issue(q, st) >= 0 && issueHead(q, 0, q.wants, st) >= 0;
+        const bool recorded = upload() && issueDecode(q, direct, st) >= 0;    // the arrays' copy belongs to the graph
         const cudaError_t e = cudaStreamEndCapture(st, &graph);
         const bool good = recorded && e == cudaSuccess && graph && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
         if (graph) { cudaGraphDestroy(graph); }
@@ -648,7 +669,7 @@ int LayeredDecoder::run(const Pass& p, const std::vector<int>& place, float* log
             cudaGetLastError();
             return 1;
         }
-        graphs_[{ p.entries, len }] = { exec, launches };
+        graphs_[{ p.entries, len, direct }] = { exec, launches };
         return 0;
     }
     *h_status_ = 1;    // a pass without results: step() looks at the device's word
@@ -656,7 +677,7 @@ int LayeredDecoder::run(const Pass& p, const std::vector<int>& place, float* log
     for (int r0 = 0; r0 < p.wants; r0 += want_cap_)
     {
         const int rows = std::min(want_cap_, p.wants - r0);
-        if (issueHead(p, r0, rows, st) < 0) { return -1; }
+        if (issueHead(p, r0, rows, st, false) < 0) { return -1; }
         if ((logits || choice) && !fetch(r0, rows)) { return 1; }
     }
     last_launches_ += (int)(cuda_b200_decoder_launches() - before);
@@ -704,7 +725,8 @@ int LayeredDecoder::end(float* logits, int* choice)
     if (!started_) { return LanguageModel::end(logits, choice); }
     started_ = false;
     gpu_.setAsCurrent();
-    if (takeResults(held_pass_.wants, places(held_pass_, held_).data(), held_logits_ ? logits : nullptr, held_choice_ ? choice : nullptr) != 0) { return 1; }
+    const bool direct = writesDirectly(held_pass_, held_logits_, held_choice_);
+    if (takeResults(held_pass_.wants, places(held_pass_, held_).data(), held_logits_ ? logits : nullptr, held_choice_ ? choice : nullptr, direct) != 0) { return 1; }
     advance(held_, std::vector<int>(held_.size(), 1));
     return *h_status_ == 0 && cudaPeekAtLastError() == cudaSuccess ? 0 : cuda_b200_decoder_check("decoder step");
 }
@@ -766,7 +788,8 @@ float LayeredDecoder::timeStep(int entries, int tokens, int context, int inner, 
     {
         for (auto it = graphs_.begin(); it != graphs_.end(); ++it)
         {
-            if (it->first.first == entries && it->first.second >= std::min(p.parts[0].max_len, cache_.rows()) && (g == graphs_.end() || it->first.second < g->first.second)) { g = it; }
+            const auto [n, len, direct] = it->first;
+            if (n == entries && !direct && len >= std::min(p.parts[0].max_len, cache_.rows()) && (g == graphs_.end() || len < std::get<1>(g->first))) { g = it; }
         }
         ok = g != graphs_.end();
     }
@@ -775,7 +798,7 @@ float LayeredDecoder::timeStep(int entries, int tokens, int context, int inner, 
         cudaEventRecord(a, st);
         for (int i = 0; i < inner && ok; i++)
         {
-            ok = p.decode ? cudaGraphLaunch(g->second.first, st) == cudaSuccess : issue(p, st) >= 0 && issueHead(p, 0, p.wants, st) >= 0;
+            ok = p.decode ? cudaGraphLaunch(g->second.first, st) == cudaSuccess : issue(p, st) >= 0 && issueHead(p, 0, p.wants, st, false) >= 0;
         }
         cudaEventRecord(z, st);
         ok = ok && cudaEventSynchronize(z) == cudaSuccess;

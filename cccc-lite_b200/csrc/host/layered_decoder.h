@@ -17,6 +17,7 @@
 #include "../../../include/cccc_b200_decoder.h"
 
 #include <map>
+#include <tuple>
 
 namespace cccc
 {
@@ -210,7 +211,9 @@ private:
     void* dmalloc(size_t bytes, bool zero);
     void makePass(const std::vector<StepEntry>& entries, const std::vector<int>& from, const std::vector<int>& count, Pass* p) const;
     int issue(const Pass& p, cudaStream_t st);          // the whole pass; launches, or -1
-    int issueHead(const Pass& p, int row0, int rows, cudaStream_t st);
+    int issueHead(const Pass& p, int row0, int rows, cudaStream_t st, bool direct);
+    bool writesDirectly(const Pass& p, bool logits, bool choice) const;
+    int issueDecode(const Pass& p, bool direct, cudaStream_t st);
     // layered_mixers.cpp: xn_ -> att_, all but the output projection
     void issueAttention(Issue& r, int layer);
     void issueLatent(Issue& r, int layer);
@@ -223,7 +226,7 @@ private:
     int run(const Pass& p, const std::vector<int>& place, float* logits, int* choice);
     int startDecode(const Pass& p, bool logits, bool choice, bool* started);
     void sendResults(int rows, bool logits, bool choice);
-    int takeResults(int rows, const int* place, float* logits, int* choice);
+    int takeResults(int rows, const int* place, float* logits, int* choice, bool direct);
     static int decodeBucket(const Pass& p, int rows);
     std::vector<int> places(const Pass& p, const std::vector<StepEntry>& entries) const;
     void advance(const std::vector<StepEntry>& entries, const std::vector<int>& count);
@@ -267,7 +270,8 @@ private:
     int* h_meta_ = nullptr;
     int* h_choice_ = nullptr;
     float* h_logits_ = nullptr;
-    std::map<std::pair<int, int>, std::pair<cudaGraphExec_t, int>> graphs_;    // (entries, length bucket) -> graph, launches
+    static constexpr int kDirectRows = 16;
+    std::map<std::tuple<int, int, bool>, std::pair<cudaGraphExec_t, int>> graphs_;    // (entries, length bucket, writes directly) -> graph, launches
     int last_launches_ = 0;
     // results on their way to the host: the rows' logits in pieces, each with an event behind it, and the status word
     static constexpr int kPieces = 4;

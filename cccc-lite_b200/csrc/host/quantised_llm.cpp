@@ -76,7 +76,7 @@ public:
         // one token of all entries that have one after the other; the graph of a step takes them all
         for (size_t i = 0; i < longest; i++)
         {
-            int rc = launch(entries, i, logits != nullptr);
+            int rc = launch(entries, i, logits != nullptr, choice != nullptr);
             if (rc == 0) { rc = finish(entries, i, first, logits, choice); }
             if (rc != 0) { return 1; }
         }
@@ -90,7 +90,7 @@ public:
         for (const auto& e : held_) { started_ = started_ && e.tokens.size() == 1; }
         if (!started_) { return rc; }
         launches_ = 0;
-        started_rc_ = launch(held_, 0, logits);
+        started_rc_ = launch(held_, 0, logits, choice);
         return 0;
     }
     int end(float* logits, int* choice) override
@@ -152,7 +152,7 @@ private:
     }
 
     // The i-th tokens of the entries that have one, as one step.
-    int launch(const std::vector<StepEntry>& entries, size_t i, bool logits)
+    int launch(const std::vector<StepEntry>& entries, size_t i, bool logits, bool choice)
     {
         std::vector<int> ids, pos, slot;
         bool any = false;
@@ -164,7 +164,7 @@ private:
             pos.push_back(cache().length(e.slot));
             any = any || std::count(e.want.begin(), e.want.end(), (int)i);
         }
-        return step_.launch(ids.data(), pos.data(), (int)ids.size(), logits && any, slot.data());
+        return step_.launch(ids.data(), pos.data(), (int)ids.size(), logits && any, choice, slot.data());
     }
     int finish(const std::vector<StepEntry>& entries, size_t i, const std::vector<size_t>& first, float* logits, int* choice)
     {

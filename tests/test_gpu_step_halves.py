@@ -75,3 +75,34 @@ def test_the_halves_of_the_quantised_model(folder):  # noqa: F811
         assert list(ids[1]) == (list(ids[0]) if i != 3 else [-1] * wanted)
         assert [b.slot_length(s) for s in slots] == [a.slot_length(s) for s in slots]
     a.close(), b.close()
+
+
+@pytest.mark.parametrize("n", [1, 8, 16, 17])
+def test_logits_alone_are_those_beside_the_choice(tmp_path, n):
+    """Up to sixteen rows the head writes logits that nothing chooses from into the host's memory; steps of both kinds by turns."""
+    c = CONFIGS["odd"]
+    (tmp_path / "config.json").write_text(json.dumps(c))
+    F.write_safetensors(str(tmp_path / "model.safetensors"), F.random_weights(c, seed=6))
+    serve = load_package().serve
+    a, b = (serve.Model(str(tmp_path), max_context=64, max_sequences=n) for _ in range(2))
+    slots = [(a.open_slot(), b.open_slot())[0] for _ in range(n)]
+    for i in range(8):
+        e = [(s, tokens_for(c, 1, 7 * i + s), [0]) for s in slots]
+        want, chosen = a.step(e, choice=True)
+        got, none = b.step(e, choice=i in (3, 6))
+        assert got == want and (none is None or none == chosen)
+    a.close(), b.close()
+
+
+@pytest.mark.parametrize("n", [1, 16, 17])
+def test_logits_alone_of_the_quantised_model(folder, n):  # noqa: F811
+    serve = load_package().serve
+    d, cfg = folder
+    a, b = (serve.Model(d, max_context=64, max_sequences=n) for _ in range(2))
+    slots = [(a.open_slot(), b.open_slot())[0] for _ in range(n)]
+    for i in range(6):
+        e = [(s, [(31 * i + 7 * s) % cfg.vocab], [0]) for s in slots]
+        want, chosen = a.step(e, choice=True)
+        got, none = b.step(e, choice=i == 3)
+        assert got == want and (none is None or none == chosen)
+    a.close(), b.close()
