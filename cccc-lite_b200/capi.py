@@ -163,10 +163,7 @@ def gemm_wq_bf16(w_type: int, W, blk, inv_scale: float, X, Y, N: int, M: int, K:
                  ldx: int | None = None, ldy_m: int | None = None, ldy_n: int = 1, alpha: float = 1.0,
                  beta: float = 0.0, stream: int | None = None, flags: int = 0) -> int:
     """Asynchronous fused linear on `stream` (a raw cudaStream_t value; None = torch's current stream)."""
-    if stream is None:
-        import torch
-
-        stream = torch.cuda.current_stream().cuda_stream
+    stream = _stream(stream)
     return lib().cuda_gemm_wq_bf16(w_type, _ptr(W), _ptr(blk), inv_scale, _ptr(X), _ptr(Y), N, M, K,
                                    K if ldw is None else ldw, K if ldx is None else ldx,
                                    N if ldy_m is None else ldy_m, ldy_n, alpha, beta, stream, flags)
@@ -176,10 +173,7 @@ def gemm_w8a8_bf16(W, w_inv_scale: float, X, act_scale: float, Y, N: int, M: int
                    ldx: int | None = None, ldy_m: int | None = None, ldy_n: int = 1, alpha: float = 1.0, beta: float = 0.0,
                    stream: int | None = None, flags: int = 0) -> int:
     """W8A8 linear: E4M3 weights, BF16 activations quantised to E4M3 inside the call (act_scale > 0 static, 0 dynamic)."""
-    if stream is None:
-        import torch
-
-        stream = torch.cuda.current_stream().cuda_stream
+    stream = _stream(stream)
     return lib().cuda_gemm_w8a8_bf16(_ptr(W), w_inv_scale, _ptr(X), act_scale, _ptr(Y), N, M, K, K if ldw is None else ldw,
                                      K if ldx is None else ldx, N if ldy_m is None else ldy_m, ldy_n, alpha, beta, stream, flags)
 
@@ -187,10 +181,7 @@ def gemm_w8a8_bf16(W, w_inv_scale: float, X, act_scale: float, Y, N: int, M: int
 def gemm_w8a8_bf16_group(group, X, act_scale: float, M: int, K: int, *, ldx: int | None = None, stream: int | None = None,
                          flags: int = 0) -> int:
     """Up to three W8A8 linears sharing X (`group` from make_group) in one call: one quantisation, one launch."""
-    if stream is None:
-        import torch
-
-        stream = torch.cuda.current_stream().cuda_stream
+    stream = _stream(stream)
     return lib().cuda_gemm_w8a8_bf16_group(len(group), group, _ptr(X), act_scale, M, K, K if ldx is None else ldx, stream, flags)
 
 
@@ -202,10 +193,7 @@ def gemm_wq_bf16_static(w_type: int, W, blk, inv_scale: float, X, Y, N: int, M: 
                         ldx: int | None = None, ldy_m: int | None = None, ldy_n: int = 1, alpha: float = 1.0,
                         beta: float = 0.0, stream: int | None = None, flags: int = 0) -> int:
     """The allocation-free variant (fixed scratch inside the library, M <= 8); same arguments."""
-    if stream is None:
-        import torch
-
-        stream = torch.cuda.current_stream().cuda_stream
+    stream = _stream(stream)
     return lib().cuda_gemm_wq_bf16_static(w_type, _ptr(W), _ptr(blk), inv_scale, _ptr(X), _ptr(Y), N, M, K,
                                           K if ldw is None else ldw, K if ldx is None else ldx,
                                           N if ldy_m is None else ldy_m, ldy_n, alpha, beta, stream, flags)
@@ -232,10 +220,7 @@ def make_group(linears, K: int):
 def gemm_wq_bf16_group(w_type: int, group, X, M: int, K: int, *, ldx: int | None = None, stream: int | None = None,
                        flags: int = 0) -> int:
     """Several linears sharing the activations X in one call (`group` from make_group)."""
-    if stream is None:
-        import torch
-
-        stream = torch.cuda.current_stream().cuda_stream
+    stream = _stream(stream)
     return lib().cuda_gemm_wq_bf16_group(w_type, len(group), group, _ptr(X), M, K, K if ldx is None else ldx, stream, flags)
 
 
@@ -271,10 +256,7 @@ class PushAllReduce:
         dist.barrier(group)
 
     def __call__(self, partial, out, n: int, stream: int | None = None, flags: int = 0) -> int:
-        if stream is None:
-            import torch
-
-            stream = torch.cuda.current_stream().cuda_stream
+        stream = _stream(stream)
         return lib().cuda_b200_allreduce_f32_to_bf16(self.recv_ptrs, self.flag_ptrs, _ptr(self.counters), _ptr(partial), _ptr(out),
                                                      n, self.n_max, self.rank, self.world, stream, flags)
 
@@ -320,10 +302,7 @@ class FusedRowLinear:
     def __call__(self, w_type: int, W, blk, inv_scale: float, X, Y, N: int, M: int, K: int, *, ldw: int | None = None,
                  ldx: int | None = None, ldy_m: int | None = None, ldy_n: int = 1, alpha: float = 1.0,
                  stream: int | None = None, flags: int = 0) -> int:
-        if stream is None:
-            import torch
-
-            stream = torch.cuda.current_stream().cuda_stream
+        stream = _stream(stream)
         return lib().cuda_gemm_wq_bf16_allreduce(w_type, _ptr(W), _ptr(blk), inv_scale, _ptr(X), _ptr(Y), N, M, K,
                                                  K if ldw is None else ldw, K if ldx is None else ldx,
                                                  N if ldy_m is None else ldy_m, ldy_n, alpha, self.recv_ptrs, self.flag_ptrs,
@@ -331,10 +310,14 @@ class FusedRowLinear:
 
 
 def _stream(stream):
+    """The raw stream: torch's current one for None.  Asked for directly where torch has been initialised: the object that
+    torch.cuda.current_stream() makes takes 3.2 us, a third of a call."""
     if stream is None:
         import torch
 
-        return torch.cuda.current_stream().cuda_stream
+        if not torch.cuda.is_initialized():
+            return torch.cuda.current_stream().cuda_stream
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     return stream
 
 
@@ -422,10 +405,7 @@ class DecodeProgram:
 
 
 def argmax_bf16(logits, rows: int, cols: int, idx_out, val_out=None, ld: int | None = None, stream: int | None = None) -> int:
-    if stream is None:
-        import torch
-
-        stream = torch.cuda.current_stream().cuda_stream
+    stream = _stream(stream)
     return lib().cuda_argmax_bf16(_ptr(logits), rows, cols, cols if ld is None else ld, _ptr(idx_out), _ptr(val_out), stream)
 
 

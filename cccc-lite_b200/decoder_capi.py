@@ -84,7 +84,9 @@ def _ptr(t):
 def _stream():
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def fill(cls, **kw):
