@@ -32,11 +32,17 @@ static inline bool w8a8_split_early(unsigned int M, unsigned int K) { return M >
 // Hence above 128 tokens as long as every tile gets two slices, which then run at once.  Up to 128 tokens the line lies behind what
 // would be the best one, at five quarters of a wave instead of one: the outputs of a feature keep their bits whatever matrix they are
 // part of at up to 20480 features, which the tests hold.
+// Shorter k: up to 128 tokens, where the tiles leave more than half of the SMs idle (dynamic scale, K = 4096, pairs / slices at 65 / 100 / 128
+// tokens: 1024 features 15.9 / 11.1, 15.3 / 12.6, 15.7 / 13.5; 4096 15.0 / 13.6, 15.8 / 13.4, 16.9 / 14.1; 6144 15.4 / 15.7, 16.1 / 17.2, 17.4 / 18.0;
+// 8192 16.2 / 16.7, 17.6 / 16.8, 18.5 / 17.7; 12288 18.9 / 19.6, 19.7 / 21.6, 20.2 / 22.5).  The line is one for all of a layer's q, k and v, which then
+// stay one launch.  Above 128 tokens 4096 features gain (20.8 / 17.8 at 256) less than q, k and v together lose (19.3 / 21.6 at 200), and at K = 2048
+// the pairs are ahead (4096 features at 128 11.8 / 13.5).  Fewer than eight tiles, a thousand features, keep the pairs.
 static inline bool w8a8_split_preferred(unsigned int M, unsigned int K, unsigned int N, int sm_count)
 {
     if (M <= 64) { return true; }
-    if (M > 256 || K < 8192) { return false; }
     const unsigned long long tiles = (unsigned long long)((N + 127) / 128) * ((M + 127) / 128), sms = (unsigned)sm_count;
+    if (K < 8192) { return K >= 4096 && M <= 128 && tiles >= 8 && 20 * tiles <= 9 * sms; }
+    if (M > 256) { return false; }
     return M <= 128 ? 4 * tiles <= 5 * sms : 20 * tiles <= 9 * sms;
 }
 
@@ -310,7 +316,7 @@ static int launch_w8a8(const GemvScratch* ws, const W8A8Member* mem, unsigned in
                 n.tiles += (mem[i].N_out + NK_BM - 1) / NK_BM;
             }
             int r = slices(j) ? launch_w8a8_split(n, mem + j, q, ldq, ws->device, ws->sm_count, stream, after || pdl) : -2;
-            if (r == -2) { r = launch_w8a8_pair(n, mem + j, q, ldq, ws->device, ws->sm_count, pair_fh, stream); }
+            if (r == -2) { r = launch_w8a8_pair(n, mem + j, q, ldq, ws->device, ws->sm_count, pair_fh, stream, after || pdl); }
             if (r != 0) { return r; }
         }
         return 0;

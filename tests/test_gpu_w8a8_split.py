@@ -142,6 +142,22 @@ def test_the_line_above_64_tokens(M, K, beyond):
     assert torch.equal(out[0], out[1 if beyond else 4])
 
 
+@pytest.mark.parametrize("M,K,tiles,slices", [(65, 4096, 8, True), (65, 4096, 7, False), (128, 8064, 66, True), (128, 4096, 67, False), (129, 4096, 32, False), (100, 3968, 32, False)])
+def test_the_line_of_shorter_k(M, K, tiles, slices):
+    """As above, for k below 8192: 8 tiles of features to nine twentieths of the SMs (66 of 148), up to 128 tokens."""
+    import torch
+
+    c, sms = capi(), torch.cuda.get_device_properties(0).multi_processor_count
+    N = 128 * (tiles if tiles < 60 else 9 * sms // 20 + tiles - 66) - (5 if slices else 0)
+    (W,), X = on_device([N], K, M, 2)
+    out = {}
+    for form in (0, 1, 4):
+        out[form] = torch.zeros(M, N, dtype=torch.float32, device="cuda")
+        assert c.gemm_w8a8_bf16(W, 0.01, X, 0.0, out[form], N, M, K, flags=5 | form << 8) == 0 and c.check_error("line") == 0
+    assert not torch.equal(out[1], out[4])
+    assert torch.equal(out[0], out[4 if slices else 1])
+
+
 @pytest.mark.parametrize("order,launches", [((4352, 256, 384), 4), ((256, 4352, 384), 5), ((256, 384, 4096), 3), ((4352, 4480, 9000), 3)])
 def test_members_of_a_group_take_the_kernels_they_would_take_alone(order, launches):
     import torch
