@@ -56,6 +56,30 @@ def test_ragged_and_config_shapes(wt, N, K, M):
     assert_close(O.bf16_bits_to_f32(Y).reshape(M, N), y32, (wt, N, K, M))
 
 
+@pytest.mark.parametrize("wt", WTS)
+@pytest.mark.parametrize("M,K", [(1, 1280), (2, 4096), (3, 2048), (8, 4096), (8, 2304), (5, 256)])
+def test_a_features_bits_do_not_depend_on_the_matrix(wt, M, K):
+    """The shape of the row blocks follows the number of features (one block of 64 rows per SM and fewer, several per SM, one too many); a feature's bits do not."""
+    import torch
+
+    c = capi()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    most = 64 * 2 * sms + 64
+    W, blk, inv, X = O.make_inputs(wt, most, K, M, seed=K + M, scaled=True)
+    row, row_s = (K // 2, K // 16) if wt == O.FP4_E2M1 else (K, 0)
+    dW, dX = to_dev(W).reshape(-1), to_dev(X)
+    dB = to_dev(blk).reshape(-1) if blk is not None else None
+    first = 40
+    _, y32 = O.linear_wq_bf16(wt, W.reshape(most, -1)[:first].copy(), blk.reshape(-1)[:first * row_s].copy() if blk is not None else None, inv, X, first, M, K)
+    alone = None
+    for N in (first, 64 * (sms // 2), 64 * sms - 24, 64 * sms, 64 * sms + 1, most - 64, most):
+        Y = torch.zeros(M, N, dtype=torch.int16, device="cuda")
+        assert c.gemm_wq_bf16(wt, dW[:N * row], dB[:N * row_s] if dB is not None else None, inv, dX, Y, N, M, K, flags=0x2801) == 0 and c.check_error("rows") == 0
+        alone = Y[:, :first].clone() if alone is None else alone
+        assert torch.equal(Y[:, :first], alone), N
+    assert_close(O.bf16_bits_to_f32(from_dev_u16(alone.contiguous())).reshape(M, first), y32, (wt, M, K))
+
+
 def test_config1_unit_scale_w8a16():
     """Benchmark configuration 1: x[1,4096] ~ N(0,1) BF16, W[4096,4096] ~ N(0,0.02) E5M2, scale 1.0, seed 0."""
     N = K = 4096
