@@ -104,6 +104,30 @@ __global__ void __launch_bounds__(256) swiglu_bf16_kernel(const uint16_t* __rest
     }
 }
 
+// Eight elements a thread, from rows that start on 16 bytes: a prompt's.  Bound by the sigmoids' instructions and by HBM (38 MB in
+// 6 us at 6144 columns x 1024 rows); the one-element form above is bound by its two-byte accesses and its blocks' starts.  6144
+// columns x 256 / 1024 rows 6.8 / 25.8 -> 4.6 / 10.1 us.
+__global__ void __launch_bounds__(256) swiglu_bf16_wide_kernel(const uint16_t* __restrict__ G, const uint16_t* __restrict__ U,
+    uint16_t* __restrict__ O, unsigned int cols, unsigned int ldg, unsigned int ldu, unsigned int ldo)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t row = blockIdx.y;
+    const unsigned int i = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (i >= cols) { return; }
+    const uint4 g = *reinterpret_cast<const uint4*>(G + row * ldg + i), u = *reinterpret_cast<const uint4*>(U + row * ldu + i);
+    const uint32_t gw[4] = { g.x, g.y, g.z, g.w }, uw[4] = { u.x, u.y, u.z, u.w };
+    uint32_t ow[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+    {
+        const uint32_t lo = bf16_bits(swiglu_one(__uint_as_float(gw[j] << 16), __uint_as_float(uw[j] << 16)));
+        const uint32_t hi = bf16_bits(swiglu_one(__uint_as_float(gw[j] & 0xFFFF0000u), __uint_as_float(uw[j] & 0xFFFF0000u)));
+        ow[j] = lo | (hi << 16);
+    }
+    *reinterpret_cast<uint4*>(O + row * ldo + i) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+}
+
 // ---- q/k norm, RoPE and cache append of many tokens ----------------------------------------------------
 // One warp per (token, head); heads 0 .. H-1 are queries, then Hkv keys, then Hkv values.  Lane l holds the elements l, l + 32,
 // ..: a rotation's two elements meet in one lane, and the squares are added in the order of team_sum_squares, so that a row
@@ -369,6 +393,14 @@ C_EXPORT int cuda_swiglu_bf16(const void* gate, const void* up, void* out, unsig
     if (rows == 0 || cols == 0) { return 0; }
     if (!gate || !up || !out || rows > 65535u) { return -1; }
     const unsigned int gx = (cols + 255) / 256 < 64 ? (cols + 255) / 256 : 64;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out);
+    // Under three quarters of a million elements the one-element form's many short threads are done first (6144 columns of 64 rows
+    // 1.9 against 3.2 us, of 1 row 1.1 against 1.6); from there on eight a thread are (128 rows 3.6 against 2.9).
+    if ((unsigned long long)rows * cols >= 786432ull && ((cols | ld_gate | ld_up | ld_out) & 7u) == 0 && (at & 15u) == 0)
+    {
+        return launch_simple("swiglu_bf16", swiglu_bf16_wide_kernel, dim3((cols + 2047) / 2048, rows), dim3(256), 0, (cudaStream_t)stream,
+            (flags & 1u) != 0, (const uint16_t*)gate, (const uint16_t*)up, (uint16_t*)out, cols, ld_gate, ld_up, ld_out);
+    }
     return launch_simple("swiglu_bf16", swiglu_bf16_kernel, dim3(gx, rows), dim3(256), 0, (cudaStream_t)stream, (flags & 1u) != 0,
         (const uint16_t*)gate, (const uint16_t*)up, (uint16_t*)out, cols, ld_gate, ld_up, ld_out);
 }

@@ -139,6 +139,31 @@ def test_swiglu(rows, cols):
     assert_nearly_bit_equal(from_dev_u16(dO).reshape(rows, cols), want, "swiglu")
 
 
+@pytest.mark.parametrize("rows,cols,pad,shift", [(96, 8192, 0, 0), (97, 8200, 0, 0), (788, 1000, 8, 0), (97, 8201, 0, 0), (96, 8200, 4, 0),
+                                                 (97, 8200, 0, 1)])
+def test_swiglu_of_a_prompt(rows, cols, pad, shift):
+    """Large calls take eight elements a thread where rows lie on 16 bytes (the first three), else one: every element has the bits that a
+    call of its row alone gives it, infinities and NaN among them, and nothing beside the rows is written."""
+    import torch
+
+    c = capi()
+    rng = np.random.default_rng(rows + cols)
+    ld = cols + pad
+    G, U = bf16_rand(rng, (rows, ld), 3.0), bf16_rand(rng, (rows, ld))
+    G[0, :6], U[0, :6] = [0x7F80, 0xFF80, 0x7FC0, 0x0000, 0x42F0, 0xC2F0], [0x3F80, 0x3F80, 0x3F80, 0x7F80, 0x7F00, 0x7F00]
+    room = [torch.zeros(rows * ld + shift, dtype=torch.int16, device="cuda") for _ in range(2)]
+    for r, a in zip(room, (G, U)):
+        r[shift:] = to_dev(a).flatten()
+    dG, dU = (r[shift:] for r in room)
+    dO = torch.full((rows * ld + shift,), 0x1234, dtype=torch.int16, device="cuda")
+    dR = dO.clone()
+    assert c.swiglu_bf16(dG, dU, dO[shift:], rows, cols, ld, ld, ld) == 0
+    for r in range(rows):
+        assert c.swiglu_bf16(dG[r * ld:], dU[r * ld:], dR[shift + r * ld:], 1, cols, ld, ld, ld) == 0
+    assert c.check_error("swiglu") == 0
+    assert torch.equal(dO, dR)
+
+
 def attention_case(B, H, Hkv, hd, T_max, pos, qk_norm, seed, strided=False):
     """Runs cuda_attn_decode_bf16 and the oracle's composition of the reference's ops on the same inputs."""
     import torch
