@@ -60,6 +60,22 @@ def test_alpha_beta_strides_and_output_modes(wt):
 
 
 @pytest.mark.parametrize("wt", WTS)
+@pytest.mark.parametrize("N,K,M", [(203, 512, 150), (4, 256, 129), (260, 4096, 385)])
+@pytest.mark.parametrize("mode", [0, 8])
+def test_rows_that_lie_on_8_bytes_have_the_same_bits(wt, N, K, M, mode):
+    """Four elements of Y at once where its rows allow it, the added Y among them, else one by one: the same bits, and nothing beside the rows."""
+    W, blk, inv, X = O.make_inputs(wt, N, K, M, seed=N, scaled=True)
+    Y0 = O.f32_to_bf16_bits(np.random.default_rng(M).standard_normal((M, N)).astype(np.float32))
+    got = []
+    for ld in ((N + 3) // 4 * 4 + 4, (N + 3) // 4 * 4 + 5):
+        Y = np.full((M, ld), 0x1234, np.uint16)
+        Y[:, :N] = Y0
+        got.append(run(wt, W, blk, inv, X, N, M, K, Y0=Y, flags=WIDE | mode, ldy_m=ld, alpha=0.75, beta=1.5).reshape(M, ld))
+        assert (got[-1][:, N:] == 0x1234).all()
+    assert np.array_equal(got[0][:, :N], got[1][:, :N]) and not np.array_equal(got[0][:, :N], Y0)
+
+
+@pytest.mark.parametrize("wt", WTS)
 @pytest.mark.parametrize("M", [130, 512])
 def test_weights_are_dequantised_bit_exactly(wt, M):
     N, K = 508, 512
