@@ -44,6 +44,102 @@ __global__ void __launch_bounds__(kTeam) rms_norm_bf16_kernel(const uint16_t* __
     }
 }
 
+// The same with a row's elements in eights, for rows that start on 16 bytes.  Bound by its latencies: in a decode step it stands
+// between two linears with a block to a token.  The row and its scale are under way together, before anything is summed, and stay in
+// registers; the sums of squares keep the order of team_sum_squares (thread t the elements t, t + 256, ..: through shared memory), and
+// every warp adds the 256 sums by itself, in the halving tree's order, so that two barriers are left of six.  4 rows of 4096 columns
+// 2.7 -> 1.9 us, with a residual 3.7 -> 2.3; 1024 rows 7.1 -> 5.2 and 9.1 -> 7.0 (17 MB to move, 2.6 us).
+template <int C>    // eights per thread
+__global__ void __launch_bounds__(kTeam) rms_norm_bf16_wide_kernel(const uint16_t* __restrict__ X, const uint16_t* __restrict__ R,
+    uint16_t* __restrict__ S, uint16_t* __restrict__ Y, const uint16_t* __restrict__ scale, unsigned int inner, float eps)
+{
+    __shared__ __align__(16) float xs[C * kTeam * 8];
+    __shared__ float part[kTeam];
+    const unsigned int tid = threadIdx.x, lane = tid & 31u;
+    const size_t row = (size_t)blockIdx.x * inner;
+    pdl_launch_dependents();
+    pdl_wait();
+    uint4 xv[C], rv[C], wv[C];
+#pragma unroll
+    for (int c = 0; c < C; c++)
+    {
+        const unsigned int i = (c * kTeam + tid) * 8;
+        xv[c] = rv[c] = make_uint4(0u, 0u, 0u, 0u);
+        wv[c] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+        if (i < inner)
+        {
+            xv[c] = *reinterpret_cast<const uint4*>(X + row + i);
+            if (R != nullptr) { rv[c] = *reinterpret_cast<const uint4*>(R + row + i); }
+            if (scale != nullptr) { wv[c] = *reinterpret_cast<const uint4*>(scale + i); }
+        }
+    }
+    float v[C][8];
+#pragma unroll
+    for (int c = 0; c < C; c++)
+    {
+        const unsigned int i = (c * kTeam + tid) * 8;
+        const uint32_t x[4] = { xv[c].x, xv[c].y, xv[c].z, xv[c].w }, r[4] = { rv[c].x, rv[c].y, rv[c].z, rv[c].w };
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            v[c][2 * j] = __uint_as_float(x[j] << 16);
+            v[c][2 * j + 1] = __uint_as_float(x[j] & 0xFFFF0000u);
+            if (R != nullptr)
+            {
+                v[c][2 * j] = bf16_round(__fadd_rn(v[c][2 * j], __uint_as_float(r[j] << 16)));
+                v[c][2 * j + 1] = bf16_round(__fadd_rn(v[c][2 * j + 1], __uint_as_float(r[j] & 0xFFFF0000u)));
+            }
+        }
+        if (i < inner)
+        {
+            if (R != nullptr && S != nullptr)
+            {
+                uint32_t s[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) { s[j] = bf16_bits(v[c][2 * j]) | ((uint32_t)bf16_bits(v[c][2 * j + 1]) << 16); }
+                *reinterpret_cast<uint4*>(S + row + i) = make_uint4(s[0], s[1], s[2], s[3]);
+            }
+            *reinterpret_cast<float4*>(xs + i) = make_float4(v[c][0], v[c][1], v[c][2], v[c][3]);
+            *reinterpret_cast<float4*>(xs + i + 4) = make_float4(v[c][4], v[c][5], v[c][6], v[c][7]);
+        }
+    }
+    __syncthreads();
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8 * C; j++)
+    {
+        const unsigned int i = tid + j * kTeam;
+        if (i < inner) { s = __fmaf_rn(xs[i], xs[i], s); }
+    }
+    part[tid] = s;
+    __syncthreads();
+    float q[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) { q[j] = part[lane + 32 * j]; }
+#pragma unroll
+    for (int j = 0; j < 4; j++) { q[j] += q[j + 4]; }
+    q[0] += q[2];
+    q[1] += q[3];
+    s = q[0] + q[1];
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) { s += __shfl_down_sync(0xFFFFFFFFu, s, k); }
+    const float invstd = rms_invstd(__shfl_sync(0xFFFFFFFFu, s, 0), inner, eps);
+#pragma unroll
+    for (int c = 0; c < C; c++)
+    {
+        const unsigned int i = (c * kTeam + tid) * 8;
+        const uint32_t w[4] = { wv[c].x, wv[c].y, wv[c].z, wv[c].w };
+        uint32_t y[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+        {
+            y[j] = bf16_bits(rms_apply(v[c][2 * j], invstd, __uint_as_float(w[j] << 16)))
+                | ((uint32_t)bf16_bits(rms_apply(v[c][2 * j + 1], invstd, __uint_as_float(w[j] & 0xFFFF0000u))) << 16);
+        }
+        if (i < inner) { *reinterpret_cast<uint4*>(Y + row + i) = make_uint4(y[0], y[1], y[2], y[3]); }
+    }
+}
+
 // ---- RoPE (standalone) ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) rope_bf16_kernel(const uint16_t* __restrict__ X, uint16_t* __restrict__ Y,
     const uint16_t* __restrict__ cos_tab, const uint16_t* __restrict__ sin_tab, unsigned int D, unsigned int T, unsigned long long total,
@@ -359,6 +455,21 @@ C_EXPORT int cuda_rms_norm_bf16(const void* X, const void* residual, void* sum_o
     const DeviceFacts* f = device_facts();
     if (!f) { return 1; }
     if (smem > (size_t)f->max_smem) { return -1; }
+    const uintptr_t at = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(sum_out)
+        | reinterpret_cast<uintptr_t>(Y) | reinterpret_cast<uintptr_t>(scale);
+    // Rows of a few hundred columns, as a head's norms have, leave most of a team of eights without one: with more rows than SMs
+    // the form of one element a thread is done first (128 columns, 300 rows: 2.0 against 2.2 us; 100 rows 1.7 against 1.5; of 512
+    // columns, 300 rows 2.8 against 2.4).  Above 8192 columns a thread would hold too many eights.
+    if ((at & 15u) == 0 && (inner & 7u) == 0 && inner <= 4 * 8 * kTeam && (inner >= 512 || rows <= 128))
+    {
+        auto run = [&](auto kernel) {
+            return launch_simple("rms_norm_bf16", kernel, dim3(rows), dim3(kTeam), 0, (cudaStream_t)stream, (flags & 1u) != 0, (const uint16_t*)X,
+                (const uint16_t*)residual, (uint16_t*)sum_out, (uint16_t*)Y, (const uint16_t*)scale, inner, epsilon);
+        };
+        if (inner <= 8 * kTeam) { return run(rms_norm_bf16_wide_kernel<1>); }
+        if (inner <= 2 * 8 * kTeam) { return run(rms_norm_bf16_wide_kernel<2>); }
+        return inner <= 3 * 8 * kTeam ? run(rms_norm_bf16_wide_kernel<3>) : run(rms_norm_bf16_wide_kernel<4>);
+    }
     if (smem > 48 * 1024 && cudaFuncSetAttribute(rms_norm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     {
         return report_launch("rms_norm_bf16") ? 1 : 1;

@@ -73,6 +73,35 @@ def test_rms_norm(rows, inner, with_residual):
         assert torch.equal(ref, dY), ("reference kernel", rows, inner)
 
 
+@pytest.mark.parametrize("rows,inner", [(3, 8), (1, 128), (129, 128), (300, 2040), (2, 2048), (5, 2056), (33, 4096), (2, 5120), (3, 6152), (2, 8192), (2, 8200), (3, 1001)])
+@pytest.mark.parametrize("mode", ["plain", "residual", "in place", "no scale"])
+def test_rms_norm_bits_do_not_depend_on_the_address(rows, inner, mode):
+    """Rows on 16 bytes are read in eights, others (the second call) element by element: the same bits, and nothing behind the rows is written."""
+    import torch
+
+    c = capi()
+    rng = np.random.default_rng(rows * inner)
+    X, R = bf16_rand(rng, rows * inner, 2.0), bf16_rand(rng, rows * inner)
+    X[:2] = [0x7F80, 0x7FC0]    # one row of infinities and NaN
+    w = bf16_rand(rng, inner)
+    got = []
+    for shift in (0, 1):
+        def room(a):
+            t = torch.full((rows * inner + 16,), 0x1234, dtype=torch.int16, device="cuda")
+            if a is not None:
+                t[shift:shift + a.size] = to_dev(a)
+            return t
+        dX, dR, dW, dS, dY = room(X), room(R), room(w), room(None), room(None)
+        x, r, s, y = (t[shift:] for t in (dX, dR, dS, dY))
+        if mode == "in place":
+            s, y = r, x
+        assert c.rms_norm_bf16(x, y, None if mode == "no scale" else dW[shift:], rows, inner, 1e-6, residual=None if mode == "plain" else r,
+                               sum_out=None if mode == "plain" else s) == 0
+        assert c.check_error("rms") == 0
+        got.append([torch.cat((t[shift:shift + rows * inner], t[shift + rows * inner:][:15])) for t in (dX, dR, dS, dY)])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("D,T,B,off", [(128, 1, 40, 4095), (128, 7, 3, 11), (64, 5, 2, 0), (128, 64, 8, 100)])
 def test_rope(D, T, B, off):
     import torch
