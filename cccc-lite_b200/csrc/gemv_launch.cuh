@@ -5,6 +5,7 @@
 
 #include "common.cuh"
 #include "gemv_decode.cuh"
+#include "gemv_form.cuh"
 #include "tensor_map.cuh"
 #include "prefill_launch.cuh"
 #include "gemm_stream.cuh"
@@ -86,19 +87,8 @@ static int launch_gemv_cfg(GemvParams p, const GemvScratch* ws, cudaStream_t str
     if (total == 0 || total > 0x7FFFFFFFull) { return -2; }
     p.total_items = (unsigned int)total;
     p.n_stages = (unsigned int)ns;
-    // With at least one row block per SM, whole row blocks are dealt out: no CTA shares a row block,
-    // so nothing is exchanged between CTAs.  With fewer, the k range is split as well (stream-K).
-    // Measured on B200: the exchange costs about 5 us of serial latency, one SM alone streams about
-    // 45 GB/s; so the k range is only split when whole row blocks would leave most SMs idle for long.
-    bool whole_blocks = true;
-    {
-        const double block_bytes = (double)Cfg::R * (double)((WT == DT_FP4) ? p.K / 2 + p.K / 16 : p.K);
-        const double sms = (double)ws->sm_count;
-        const double rounds = (double)((p.n_row_blocks + ws->sm_count - 1) / ws->sm_count);
-        const double t_whole = rounds * block_bytes / 45e9;
-        const double t_split = 5e-6 + (double)p.n_row_blocks * block_bytes / (sms * 40e9);
-        whole_blocks = t_whole <= t_split || Cfg::MT > 1;    // large partial tiles make the exchange far dearer
-    }
+    // (large partial tiles make the exchange between CTAs far dearer)
+    const bool whole_blocks = Cfg::MT > 1 || gemv_whole_blocks(Cfg::R, WT == DT_FP4, p.n_row_blocks, p.K, ws->sm_count);
     p.gran = whole_blocks ? p.n_kstages : 1u;
     const unsigned long long groups = total / p.gran;
     const unsigned int grid = (unsigned int)(groups < (unsigned long long)ws->sm_count ? groups : ws->sm_count);
@@ -169,53 +159,31 @@ static int launch_gemv_cfg(GemvParams p, const GemvScratch* ws, cudaStream_t str
     return 0;
 }
 
-// Row blocks of 64 rows and sixteen warps, or of 32 and eight?  Twice the warps keep a stage's conversions going better (at 1 token, 32 / 64 rows, us:
-// E4M3 6144 x 4096 10.1 / 8.9, 24576 x 4096 26.2 / 24.5, 151936 x 4096 120.1 / 113.8; E5M2 9.0 / 7.8, 22.5 / 21.3, 101.3 / 95.4), but whole
-// blocks are dealt out: it is for launches whose busiest SM then has no more rows, or hardly more (28672 x 4096, 256 rows against 224, 29.0 / 30.9; 4096 x
-// 4096 6.0 / 7.6).  FP8 at 3 to 8 tokens, in stages of 96 KB, gains where every block has an SM of its own (6144 x 4096 9.7 / 8.8) and not beyond
-// (151936 x 4096 118.0 / 118.9).  FP4 gains alone (6144 x 4096 at 1 token 9.7 / 8.5) and loses in a layer (8 tokens, four calls, 49.3 / 50.9: fewer, longer
-// CTAs keep the next kernel's out).  A warp's k steps and the order of the sums are the same either way: so are the bits.
-static bool gemv_tall(int w_type, const GemvParams& p, const GemvScratch* ws)
-{
-    if (w_type == DT_FP4 || p.M > 8 || p.ar.world > 1 || (size_t)ws->sm_count * 2 * 64 * 8 * sizeof(float) > ws->partial_bytes) { return false; }
-    unsigned long long tall = 0, low = 0;
-    for (unsigned int j = 0; j < (p.n_seg != 0 ? p.n_seg : 1u); j++)
-    {
-        const unsigned int N = p.n_seg != 0 ? p.seg[j].N : p.N;
-        tall += (N + 63) / 64;
-        low += (N + 31) / 32;
-    }
-    const unsigned long long sms = (unsigned long long)ws->sm_count;
-    const unsigned long long rows_tall = (tall + sms - 1) / sms * 64, rows_low = (low + sms - 1) / sms * 32;
-    if (p.M > 2) { return rows_tall <= rows_low && tall <= sms; }
-    return rows_tall * 93 <= rows_low * 100;
-}
-
 template <int WT, bool SCALED>
 static int launch_gemv(const GemvParams& p, const GemvScratch* ws, cudaStream_t stream, bool pdl)
 {
     // More tokens: more rows per CTA, so that the activation slice (re-read from L2 by every CTA) stays
     // at or below the weight bytes it is multiplied with.
     //                                              WT MT RT WR WK SKS XB OCC
+    unsigned long long low = 0, tall = 0;
+    for (unsigned int j = 0; j < (p.n_seg != 0 ? p.n_seg : 1u); j++)
+    {
+        const unsigned int N = p.n_seg != 0 ? p.seg[j].N : p.N;
+        low += (N + 31) / 32;
+        tall += (N + 63) / 64;
+    }
+    const GemvForm form = gemv_form(WT == DT_FP4, p.M, p.K, low, tall, ws->sm_count, p.ar.world, ws->partial_bytes);
     if constexpr (WT != DT_FP4)
     {
-        if (gemv_tall(WT, p, ws))
+        if (form == GemvForm::Tall)
         {
             return p.M <= 2 ? launch_gemv_cfg<GemvCfg<WT, 1, 2, 2, 8, 16, 2, 1>, SCALED>(p, ws, stream, pdl)
                             : launch_gemv_cfg<GemvCfg<WT, 1, 2, 2, 8, 16, 8, 1>, SCALED>(p, ws, stream, pdl);
         }
+        if (form == GemvForm::Long) { return launch_gemv_cfg<GemvCfg<WT, 1, 2, 1, 8, 32, 8, 1>, SCALED>(p, ws, stream, pdl); }
     }
     if (p.M <= 2) { return launch_gemv_cfg<GemvCfg<WT, 1, 2, 1, 8, 32, 2, 1>, SCALED>(p, ws, stream, pdl); }
-    if (p.M <= 8)
-    {
-        // FP8, whole stages of 2048 k: two of 96 KB instead of four of 48 (E4M3 at 3 tokens: 4096 x 4096 6.8 -> 6.3, 4096 x 12288 14.8 -> 13.2, 24576 x 4096
-        // 28.4 -> 25.3, 151936 x 4096 138.6 -> 118.0); FP4, twice the elements per byte, has no room for two such
-        if constexpr (WT != DT_FP4)
-        {
-            if (p.K % 2048 == 0) { return launch_gemv_cfg<GemvCfg<WT, 1, 2, 1, 8, 32, 8, 1>, SCALED>(p, ws, stream, pdl); }
-        }
-        return launch_gemv_cfg<GemvCfg<WT, 1, 2, 1, 8, 16, 8, 1>, SCALED>(p, ws, stream, pdl);
-    }
+    if (p.M <= 8) { return launch_gemv_cfg<GemvCfg<WT, 1, 2, 1, 8, 16, 8, 1>, SCALED>(p, ws, stream, pdl); }
     // (FP4 stages hold twice the elements per weight byte, so twice the activations: half the k steps)
     constexpr int S16 = (WT == DT_FP4) ? 8 : 16, S32 = (WT == DT_FP4) ? 4 : 8;
     if (p.M <= 16) { return launch_gemv_cfg<GemvCfg<WT, 2, 4, 1, 8, S16, 16, 1>, SCALED>(p, ws, stream, pdl); }

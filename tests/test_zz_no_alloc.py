@@ -44,6 +44,24 @@ def test_static_scratch_entry_matches_regular_entry(wt, N, K, M):
     assert_close(out.reshape(M, N), y32, "oracle")
 
 
+@pytest.mark.parametrize("wt", [O.FP8_E5M2, O.FP8_E4M3])
+@pytest.mark.parametrize("N,K,M", [(5120, 13824, 1), (5120, 13824, 4), (5120, 12288, 3), (6144, 16384, 2)])
+def test_split_schedules_are_cut_alike_where_higher_row_blocks_would_fit(wt, N, K, M):
+    """Launches for which the regular entry could take row blocks of 64 rows, or larger stages: they split k, and the cuts are those of the static entry."""
+    import torch
+
+    c = capi()
+    W, _, inv, X = O.make_inputs(wt, N, K, M, seed=N + M, scaled=True)
+    dW, dX = to_dev(W), to_dev(X)
+    want, got = (torch.zeros(M * N, dtype=torch.int16, device="cuda") for _ in range(2))
+    assert c.gemm_wq_bf16(wt, dW, None, inv, dX, want, N, M, K, flags=c.FLAG_NO_STREAM | c.FLAG_NO_NATIVE) == 0 and c.check_error("regular") == 0
+    assert c.gemm_wq_bf16_static(wt, dW, None, inv, dX, got, N, M, K, flags=c.FLAG_CHECKED) == 0
+    assert torch.equal(got, want)
+    first = 64
+    _, y32 = O.linear_wq_bf16(wt, W.reshape(N, K)[:first].copy(), None, inv, X, first, M, K)
+    assert_close(O.bf16_bits_to_f32(from_dev_u16(got)).reshape(M, N)[:, :first], y32, (wt, N, K, M))
+
+
 def test_static_scratch_entry_unchecked_and_alpha_beta():
     import torch
 
