@@ -158,6 +158,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WP_THREADS, 1)
     }
     else if (warp == 1)
     {
+        pdl_wait();    // the first stage needs the activations: the limit on the waits below does not count the kernels before this one
         if (lane == 0 && rank != 0)
         {
             // =========================== rank 1: forward "stage full" to the leader ===========================
@@ -447,6 +448,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WP_THREADS, 1)
     }
     else if (warp == 1)
     {
+        pdl_wait();    // the first stage needs the activations: the limit on the waits below does not count the kernels before this one
         if (lane == 0 && rank != 0)
         {
             // =========================== rank 1: forward "stage full" to the leader ===========================

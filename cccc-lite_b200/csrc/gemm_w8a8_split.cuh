@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(WS_THREADS, BN == 64 ? 2 : 1)
             for (unsigned int kb = kb_begin; kb < kb_end; kb++)
             {
                 const unsigned int i = kb - kb_begin, s = i % NS;
+                if (i == (unsigned int)NS) { pdl_wait(); }    // from here on the ring waits for products: see the MMA warp
                 if (i >= (unsigned int)NS && (*abort_flag != 0 || !mbar_wait_bounded(empty + s, ((i / NS) - 1u) & 1u)))
                 {
                     ok = false;
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(WS_THREADS, BN == 64 ? 2 : 1)
     else if (warp == 2)
     {
         // =========================== MMA warp ===========================
+        pdl_wait();    // the first stage needs the activations: the limit on the waits below does not count the kernels before this one
         bool ok = true;
         const uint32_t idesc = umma_idesc_f8(false, false, SK_BM, (tile_tokens + 15u) & ~15u);
         for (unsigned int l = 0; l < own && ok; l++)
