@@ -29,19 +29,24 @@ static inline bool w8a8_split_early(unsigned int M, unsigned int K) { return M >
 //     160 44.8 / 57.0,  224 52.6 / 59.5,  448 97.7 / 114.1;
 //   129 tokens, by tiles (two per 128 features):  16 23.2 / 13.1,  64 23.7 / 19.1,  128 25.5 / 28.3,  160 27.2 / 42.2,  448 53.0 / 103.9;
 //   256 tokens:  64 28.1 / 19.7,  128 30.3 / 28.9,  160 31.8 / 51.9.  (K = 12288 to 28672: the same sides, few tiles gain more.)
-// Hence above 128 tokens as long as every tile gets two slices, which then run at once.  Up to 128 tokens the line lies behind what
-// would be the best one, at five quarters of a wave instead of one: the outputs of a feature keep their bits whatever matrix they are
-// part of at up to 20480 features, which the tests hold.
-// Shorter k: up to 128 tokens, where the tiles leave more than half of the SMs idle (dynamic scale, K = 4096, pairs / slices at 65 / 100 / 128
-// tokens: 1024 features 15.9 / 11.1, 15.3 / 12.6, 15.7 / 13.5; 4096 15.0 / 13.6, 15.8 / 13.4, 16.9 / 14.1; 6144 15.4 / 15.7, 16.1 / 17.2, 17.4 / 18.0;
-// 8192 16.2 / 16.7, 17.6 / 16.8, 18.5 / 17.7; 12288 18.9 / 19.6, 19.7 / 21.6, 20.2 / 22.5).  The line is one for all of a layer's q, k and v, which then
-// stay one launch.  Above 128 tokens 4096 features gain (20.8 / 17.8 at 256) less than q, k and v together lose (19.3 / 21.6 at 200), and at K = 2048
-// the pairs are ahead (4096 features at 128 11.8 / 13.5).  Fewer than eight tiles, a thousand features, keep the pairs.
+// Hence above 128 tokens as long as every tile gets two slices, which then run at once; up to 128 tokens to five quarters of a wave, which is behind
+// what would be the best line, one wave.
+// Shorter k: up to 128 tokens, where the tiles leave more than half of the SMs idle.  Dynamic scale, K = 4096, pairs / slices at 65 / 80 / 100 / 128 tokens:
+//   256 features 15.5 / 11.5, 15.5 / 11.1, 16.4 / 12.8, 16.0 / 13.0;  1024 14.7 / 11.0, 15.0 / 11.5, 16.1 / 12.6, 16.6 / 13.6;
+//   4096 15.2 / 13.7, 15.5 / 14.0, 15.8 / 13.4, 17.0 / 14.2;  6144 15.7 / 15.7, 16.1 / 16.0, 16.3 / 17.4, 17.5 / 18.3;
+//   7168 15.9 / 16.5, 16.4 / 17.0, 18.1 / 17.7, 18.5 / 18.5;  8448 16.4 / 15.7, 17.5 / 16.0, 18.6 / 17.1, 19.1 / 17.9;  12288 18.9 / 19.6 at 65, 20.2 / 22.5 at 128.
+// Between 4608 and 7168 features the pairs are up to 6 % ahead.  The line does not lie there because it would part a layer's q from its k and v, which then are two
+// launches (q + k + v of 4096 + 512 + 512 features 23.1 at 65 tokens and 25.2 at 128; on pairs 15.5 and 17.2, in slices 15.2 and 17.9), and because a layer gains:
+// the four calls of a Qwen3-8B layer 80.4 / 79.3, 81.4 / 79.9, 84.5 / 80.9, 88.5 / 85.0, of a Llama-3.1-8B layer 83.2 / 81.5, 85.2 / 83.5, 87.9 / 84.4, 92.1 / 89.0.
+// Above 128 tokens 4096 features gain (20.8 / 17.8 at 256) less than q, k and v together lose (19.3 / 21.6 at 200), and at K = 2048 the pairs are ahead (4096
+// features at 128 11.8 / 13.5).  A single tile keeps the pairs, which the tests hold; no layer has one beside a wider member but for a single kv head of 128.
+// A feature's bits are the same in every matrix that takes the same kernel: on this line's side, up to 128 tokens, in all of 129 to 8448 features with K from 4096 to
+// 8191 and of up to 20480 with K from 8192 (the tests hold both); with K below 4096, and from 24 to 64 tokens, in all.
 static inline bool w8a8_split_preferred(unsigned int M, unsigned int K, unsigned int N, int sm_count)
 {
     if (M <= 64) { return true; }
     const unsigned long long tiles = (unsigned long long)((N + 127) / 128) * ((M + 127) / 128), sms = (unsigned)sm_count;
-    if (K < 8192) { return K >= 4096 && M <= 128 && tiles >= 8 && 20 * tiles <= 9 * sms; }
+    if (K < 8192) { return K >= 4096 && M <= 128 && tiles >= 2 && 20 * tiles <= 9 * sms; }
     if (M > 256) { return false; }
     return M <= 128 ? 4 * tiles <= 5 * sms : 20 * tiles <= 9 * sms;
 }

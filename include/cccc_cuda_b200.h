@@ -138,7 +138,9 @@ C_EXPORT int cuda_gemm_wq_bf16_group(int w_type, unsigned int count, const cuda_
  * cuda_gemm_wq_bf16).  Both operands go into tcgen05.mma kind::f8f6f4 unchanged: up to 23 tokens in a kernel that
  * streams the weights once over all SMs, above that with k slices as clusters (flags bits 8-10 = 4 force that form for
  * tests) or on CTA pairs (cta_group::2; 256- or 512-feature tiles, or a persistent form whose epilogue overlaps the next
- * tile; bits 8-9 = 1 / 2 / 3 force one of them, 0 lets the shape decide).  Needs K % 128 == 0, ldw % 16 == 0, ldx % 8 == 0, 16-byte aligned W and X, at most 65535 tokens
+ * tile; bits 8-9 = 1 / 2 / 3 force one of them, 0 lets the shape decide).  The order of the sums is the kernel's: above 64 tokens a
+ * feature's last bits can differ between a matrix of few features, which the k slices take where K >= 4096, and one of many (CTA pairs).
+ * Needs K % 128 == 0, ldw % 16 == 0, ldx % 8 == 0, 16-byte aligned W and X, at most 65535 tokens
  * and M_tokens * K quantised bytes within the 64 MB workspace; anything else returns -1 (the caller keeps its own
  * path).  Shares the device's workspace with cuda_gemm_wq_bf16: same ordering rule. */
 C_EXPORT int cuda_gemm_w8a8_bf16(const void* W, float w_inv_scale, const void* X, float act_scale, void* Y, unsigned int N_out,

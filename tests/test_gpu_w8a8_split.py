@@ -77,6 +77,45 @@ def test_the_bits_do_not_depend_on_the_grid(K, M):
     assert torch.equal(items[0]["Y"], alone)
 
 
+# k slices: all matrices within the line (129 to 8448 features with K from 4096 on, up to 128 tokens); CTA pairs in all their forms where k is shorter, or the tokens are more
+@pytest.mark.parametrize("M,K,features", [(65, 4096, (129, 1000, 4096, 6144, 8448)), (100, 4096, (256, 1024, 4096, 8448)), (128, 5120, (512, 5120, 8448)), (100, 2048, (128, 6144, 20480)),
+                                          (129, 4096, (128, 4096, 24576))])
+def test_the_bits_do_not_depend_on_the_matrix(M, K, features):
+    import torch
+
+    c = capi()
+    (W,), X = on_device([max(features)], K, M, 3)
+    first = min(features)
+
+    def linear(n):
+        y = torch.zeros(M, n, dtype=torch.float32, device="cuda")
+        assert c.gemm_w8a8_bf16(W, 0.01, X, 0.0, y, n, M, K, flags=5) == 0 and c.check_error("matrix") == 0
+        return y
+
+    alone = linear(first)
+    for n in features:
+        assert torch.equal(linear(n)[:, :first], alone), n
+    Ns = (features[-1], first, features[1])
+    items = [dict(W=W[:n], S=None, inv=0.01, N=n, Y=torch.zeros(M, n, dtype=torch.float32, device="cuda")) for n in Ns]
+    assert c.gemm_w8a8_bf16_group(c.make_group(items, K), X, 0.0, M, K, flags=5) == 0 and c.check_error("group") == 0
+    for it in items:
+        assert torch.equal(it["Y"][:, :first], alone)
+
+
+# q, k and v of a model, or of a rank's share of one: one quantisation (two kernels with the scale found) and one linear
+@pytest.mark.parametrize("Ns,K", [((4096, 1024, 1024), 4096), ((4096, 512, 512), 4096), ((2048, 256, 256), 4096), ((5120, 1024, 1024), 5120), ((8192, 256, 256), 5120)])
+@pytest.mark.parametrize("M", [65, 128])
+def test_q_k_and_v_are_one_launch(Ns, K, M):
+    import torch
+
+    c = capi()
+    Ws, X = on_device(Ns, K, M, 4)
+    items = [dict(W=W, S=None, inv=0.01, N=N, Y=torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")) for W, N in zip(Ws, Ns)]
+    before = c.launch_count()
+    assert c.gemm_w8a8_bf16_group(c.make_group(items, K), X, 0.0, M, K) == 0 and c.check_error("group") == 0
+    assert c.launch_count() - before == 3
+
+
 @pytest.mark.parametrize("M", [20, 64])
 def test_the_largest_magnitude_is_found_wherever_it_lies(M):
     """One scale for the tensor: every block of the search has to count."""
@@ -142,9 +181,9 @@ def test_the_line_above_64_tokens(M, K, beyond):
     assert torch.equal(out[0], out[1 if beyond else 4])
 
 
-@pytest.mark.parametrize("M,K,tiles,slices", [(65, 4096, 8, True), (65, 4096, 7, False), (128, 8064, 66, True), (128, 4096, 67, False), (129, 4096, 32, False), (100, 3968, 32, False)])
+@pytest.mark.parametrize("M,K,tiles,slices", [(65, 4096, 2, True), (65, 4096, 1, False), (128, 8064, 66, True), (128, 4096, 67, False), (129, 4096, 32, False), (100, 3968, 32, False)])
 def test_the_line_of_shorter_k(M, K, tiles, slices):
-    """As above, for k below 8192: 8 tiles of features to nine twentieths of the SMs (66 of 148), up to 128 tokens."""
+    """As above, for k below 8192: two tiles of features to nine twentieths of the SMs (66 of 148), up to 128 tokens."""
     import torch
 
     c, sms = capi(), torch.cuda.get_device_properties(0).multi_processor_count
