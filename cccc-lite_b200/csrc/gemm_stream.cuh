@@ -449,18 +449,22 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
     else { __syncthreads(); }
 
     // ---- sum the slices in slice order; CTA `rank` finishes tokens rank, rank + S, ... ----
-    // A warp finishes a token's 128 features at a time, four per lane: the partial tiles are read and Y is written in whole rows.
-    // One feature per lane, as before, is a 64-byte store per 32 features and token, of which an SM gets one done in 25 ns: a tile of
-    // 32 / 100 tokens spent 3.3 / 9.2 us here, now 1.3 / 2.6; E4M3 24576 x 4096 at 32 / 64 / 128 tokens 32.9 / 37.4 / 47.8 -> 31.5 / 33.1 /
-    // 37.7 us, 6144 x 4096 11.2 / 13.3 / 17.7 -> 10.5 / 11.6 / 14.3.
+    // A warp finishes a token's 128 features at a time, four per lane.  Where four elements of Y lie side by side and may be accessed at once, they
+    // are the lane's: the partial tiles are read and Y is written in whole rows.  (One feature per lane is a 64-byte store per 32 features and
+    // token, of which an SM gets one done in 25 ns: a tile of 32 / 100 tokens spent 3.3 / 9.2 us here, now 1.3 / 2.6; E4M3 24576 x 4096 at 32 / 64 /
+    // 128 tokens 32.9 / 37.4 / 47.8 -> 31.5 / 33.1 / 37.7 us, 6144 x 4096 11.2 / 13.3 / 17.7 -> 10.5 / 11.6 / 14.3.)  Elsewhere a lane has every 32nd
+    // feature, so that the accesses of a warp, one element each, lie side by side (32767 features at 64 / 128 tokens, four side by side / every 32nd:
+    // 35.8 / 34.7, 42.0 / 40.1 us, with an old Y 39.9 / 37.9, 50.5 / 46.1) - but not with eight slices, where reading the others' tiles one element at a time
+    // costs more than it saves (4097 features at 64 tokens 10.6 / 11.2).
     if (warp < SK_DQ_WARPS && *abort_flag == 0)
     {
-        const unsigned int n = n0 + 4 * lane;
         const unsigned int y_size = p.out_f32 == 1u ? 4u : 2u;
-        // four elements of Y at once where they lie side by side
-        const bool whole = g.ldy_n == 1 && n + 4 <= g.N && (reinterpret_cast<uintptr_t>(g.Y) & (4 * y_size - 1)) == 0 && g.ldy_m % 4 == 0;
-        auto finish = [&](unsigned int t, const float (&sum)[4]) {
-            if (n >= g.N) { return; }
+        const bool aligned = g.ldy_n == 1 && (reinterpret_cast<uintptr_t>(g.Y) & (4 * y_size - 1)) == 0 && g.ldy_m % 4 == 0;
+        auto finish = [&](auto fours, unsigned int t, const float (&sum)[4]) {
+            constexpr bool FOURS = decltype(fours)::value;
+            constexpr unsigned int STEP = FOURS ? 1 : 32;
+            const unsigned int n = n0 + (FOURS ? 4 * lane : lane);
+            const bool whole = FOURS && aligned && n + 4 <= g.N;
             const long long yi = (long long)(m0 + t) * g.ldy_m + (long long)n * g.ldy_n;
             float old[4] = { 0.f, 0.f, 0.f, 0.f }, o[4];
             if (g.beta != 0.f)
@@ -481,7 +485,8 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
 #pragma unroll
                     for (int q = 0; q < 4; q++)
                     {
-                        if (n + q < g.N) { old[q] = p.out_f32 == 1u ? reinterpret_cast<const float*>(g.Y)[yi + q * g.ldy_n] : bf16_bits_to_float(g.Y[yi + q * g.ldy_n]); }
+                        const long long at = yi + (long long)(q * STEP) * g.ldy_n;
+                        if (n + q * STEP < g.N) { old[q] = p.out_f32 == 1u ? reinterpret_cast<const float*>(g.Y)[at] : bf16_bits_to_float(g.Y[at]); }
                     }
                 }
             }
@@ -498,22 +503,28 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
 #pragma unroll
                 for (int q = 0; q < 4; q++)
                 {
-                    if (n + q >= g.N) { continue; }
-                    if (p.out_f32 == 1u) { reinterpret_cast<float*>(g.Y)[yi + q * g.ldy_n] = o[q]; }
-                    else { g.Y[yi + q * g.ldy_n] = __bfloat16_as_ushort(__float2bfloat16_rn(o[q])); }
+                    const long long at = yi + (long long)(q * STEP) * g.ldy_n;
+                    if (n + q * STEP >= g.N) { continue; }
+                    if (p.out_f32 == 1u) { reinterpret_cast<float*>(g.Y)[at] = o[q]; }
+                    else { g.Y[at] = __bfloat16_as_ushort(__float2bfloat16_rn(o[q])); }
                 }
             }
         };
-        auto add = [&](auto slices) {
+        auto add = [&](auto slices, auto fours) {
             constexpr int SL = decltype(slices)::value;
-            const float4* peer[SL];
+            constexpr bool FOURS = decltype(fours)::value;
+            const float* peer[SL];
 #pragma unroll
-            for (int r = 0; r < SL; r++) { peer[r] = reinterpret_cast<const float4*>(SL > 1 ? cluster.map_shared_rank(part, r) : part) + lane; }
+            for (int r = 0; r < SL; r++) { peer[r] = (SL > 1 ? cluster.map_shared_rank(part, r) : part) + (FOURS ? 4 * lane : lane); }
             for (unsigned int t = rank + SL * warp; t < tile_tokens; t += SL * SK_DQ_WARPS)
             {
                 float4 v[SL];
 #pragma unroll
-                for (int r = 0; r < SL; r++) { v[r] = peer[r][t * (SK_BM / 4)]; }
+                for (int r = 0; r < SL; r++)
+                {
+                    const float* row = peer[r] + t * SK_BM;
+                    v[r] = FOURS ? *reinterpret_cast<const float4*>(row) : make_float4(row[0], row[32], row[64], row[96]);
+                }
                 float sum[4] = { 0.f, 0.f, 0.f, 0.f };
 #pragma unroll
                 for (int r = 0; r < SL; r++)
@@ -523,13 +534,17 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
                     sum[2] += v[r].z;
                     sum[3] += v[r].w;
                 }
-                finish(t, sum);
+                finish(fours, t, sum);
             }
         };
-        if (S == 1) { add(std::integral_constant<int, 1>()); }
-        else if (S == 2) { add(std::integral_constant<int, 2>()); }
-        else if (S == 4) { add(std::integral_constant<int, 4>()); }
-        else { add(std::integral_constant<int, 8>()); }
+        auto add_slices = [&](auto fours) {
+            if (S == 1) { add(std::integral_constant<int, 1>(), fours); }
+            else if (S == 2) { add(std::integral_constant<int, 2>(), fours); }
+            else { add(std::integral_constant<int, 4>(), fours); }
+        };
+        if (S > 4) { add(std::integral_constant<int, 8>(), std::true_type{}); }
+        else if (aligned) { add_slices(std::true_type{}); }
+        else { add_slices(std::false_type{}); }
     }
     // nobody leaves while a peer may still read its partial tile
     if (S > 1) { cluster.sync(); }

@@ -77,6 +77,46 @@ def test_stream_alpha_beta_strides_and_output_modes(wt):
     assert_close(O.bf16_bits_to_f32(Yr).reshape(M, N), want, ("residual", wt))
 
 
+# one, two, four and eight k slices; features that end inside a lane's four, tokens of every tile size
+@pytest.mark.parametrize("wt", WTS)
+@pytest.mark.parametrize("N,K,M", [(203, 256, 20), (4, 512, 9), (131, 1024, 100), (77, 16384, 24), (1002, 4096, 128), (129, 2048, 50)])
+@pytest.mark.parametrize("mode", [0, 4, 8])
+@pytest.mark.parametrize("beta", [0.0, 1.5])
+def test_rows_on_and_off_8_and_16_bytes_have_the_same_bits(wt, N, K, M, mode, beta):
+    """Four elements of Y at once where its rows allow it, else one by one, in rows and in columns: the same bits, the oracle's values, and nothing
+    beside the rows is written."""
+    import torch
+
+    c = capi()
+    W, blk, inv, X = O.make_inputs(wt, N, K, M, seed=N, scaled=True)
+    dW, dX, dB = to_dev(W), to_dev(X), to_dev(blk) if blk is not None else None
+    Y0 = np.random.default_rng(M).standard_normal((M, N)).astype(np.float32)
+    Y0 = Y0 if mode == 4 else O.bf16_bits_to_f32(O.f32_to_bf16_bits(Y0)).reshape(M, N)
+    dtype, canary = (torch.float32, 7.0) if mode == 4 else (torch.bfloat16, 3.0)
+    fours = (N + 3) // 4 * 4 + 4
+    got = []
+    for ld, off, column in ((fours, 0, False), (fours, 4, False), (fours + 1, 0, False), (fours, 1, False), (fours, 2, False), (M + 3, 0, True)):
+        rows, cols = (N, M) if column else (M, N)
+        buf = torch.full((off + rows * ld,), canary, dtype=dtype, device="cuda")
+        y = buf[off:].view(rows, ld)
+        y[:, :cols] = torch.from_numpy(Y0.T.copy() if column else Y0).to("cuda", dtype)
+        assert c.gemm_wq_bf16(wt, dW, dB, inv, dX, buf[off:], N, M, K, ldy_m=1 if column else ld, ldy_n=ld if column else 1, alpha=0.75, beta=beta,
+                              flags=STREAM | mode) == 0 and c.check_error("rows") == 0
+        assert (y[:, cols:] == canary).all() and (buf[:off] == canary).all()
+        got.append((y[:, :cols].T if column else y[:, :cols]).clone())
+    assert all(torch.equal(g, got[0]) for g in got[1:])
+    _, y32 = O.linear_wq_bf16(wt, W, blk, inv, X, N, M, K, alpha=0.75)
+    y = got[0].float().cpu().numpy()
+    if mode == 8 and beta != 0.0:
+        # a product next to the middle of two BF16 numbers may round to either: they lie 2^-7 of it apart at most; the result is rounded by half of that
+        prod = O.bf16_bits_to_f32(O.f32_to_bf16_bits(y32.astype(np.float32))).reshape(M, N)
+        want = prod + beta * Y0
+        assert (np.abs(y - want) <= 2.0 ** -7 * np.abs(prod) + 2.0 ** -8 * np.abs(want)).all()
+        assert np.linalg.norm(y - want) <= 2.0 ** -8 * np.linalg.norm(want)
+    else:
+        assert_close(y, y32.reshape(M, N) + beta * Y0, (wt, N, K, M, mode))
+
+
 @pytest.mark.parametrize("wt", [O.FP8_E5M2, O.FP8_E4M3])
 @pytest.mark.parametrize("inv", [1.0, 0.25, 0.37])
 @pytest.mark.parametrize("M", [1, 16, 40, 128])
