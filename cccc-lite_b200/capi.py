@@ -8,6 +8,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+from .torch_stream import current_stream
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libcccc-cuda-b200.so")
 
@@ -310,15 +312,7 @@ class FusedRowLinear:
 
 
 def _stream(stream):
-    """The raw stream: torch's current one for None.  Asked for directly where torch has been initialised: the object that
-    torch.cuda.current_stream() makes takes 3.2 us, a third of a call."""
-    if stream is None:
-        import torch
-
-        if not torch.cuda.is_initialized():
-            return torch.cuda.current_stream().cuda_stream
-        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
-    return stream
+    return current_stream() if stream is None else stream
 
 
 def rms_norm_bf16(X, Y, scale, rows: int, inner: int, eps: float = 1e-6, residual=None, sum_out=None, stream=None, flags: int = 0) -> int:
