@@ -7,8 +7,8 @@
 // microseconds, the chain from the previous kernel's end to the results: each chunk is requested a turn ahead into the registers of
 // the chunk just used, the first ones of a dense member before the previous kernel of the stream has finished, a task's first ones
 // while the sums of the task before it are made; what the results are added to is fetched before the products.  The warps' partial
-// sums meet in shared memory.  At 8 rows, with two turns of two chunks, one CTA per task and no such prefetch, before: 2048 x 2048
-// 4.2 us, 5120 x 2048 8.2, 6144 x 2048 8.7 (gated 12.7), 2048 x 6144 9.5, 32768 x 2048 27.4; now 3.0, 7.3, 7.3 (11.1), 6.2, 25.1.
+// sums meet in shared memory.  At 8 rows, with two turns of two chunks, one CTA per task and no such prefetch, before: 2048 x 2048 3.9
+// us, 5120 x 2048 8.4, 2048 x 6144 9.3, 32768 x 2048 27.5, gated 6144 x 2048 13.2; now 3.1, 7.4, 6.4, 24.6, 11.1.
 #include "decoder_common.cuh"
 #include "../gemv_decode.cuh"
 #include "linear.cuh"
@@ -35,7 +35,7 @@ __device__ __forceinline__ void ldg_stream(const void* p, uint4& a, uint4& b)
 // What one CTA does at a time: C rows (from n0) of a CTA's share of the features of one group.
 struct StreamTask
 {
-    unsigned int block, member, slot, fc;    // fc: first feature of the CTA
+    unsigned int block, member, fc;    // fc: first feature of the CTA
     unsigned int group, row0, count, n0;
 };
 
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(32 * LS_WARPS, OCC) linear_stream_kernel(const
     constexpr int R = 16 * RT, C = 8 * NT, NW = LS_WARPS, T = 32 * NW;
     constexpr int RED = NW * C * (R + 1);
     constexpr bool TWO = RED * 8 <= 24 * 1024;    // two places for the partial sums: one barrier per task instead of two
-    constexpr int XD = U < 2 || (NT == 2 && U * RT > 2) ? 1 : 2;    // chunks of X in registers
+    constexpr int XD = U < 2 || (NT == 2 && U * RT > 2) || (NT == 4 && OCC == 2) ? 1 : 2;    // chunks of X in registers
     __shared__ float red_all[(TWO ? 2 : 1) * RED];
     const unsigned int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const unsigned int wk = warp % WK, wf = warp / WK;
@@ -66,7 +66,6 @@ __global__ void __launch_bounds__(32 * LS_WARPS, OCC) linear_stream_kernel(const
             const unsigned int b = block - m.block0, fb = b % m.fblocks, slot = b / m.fblocks;
             k.block = block;
             k.member = mi;
-            k.slot = slot;
             k.fc = fb * (activation_gated(m.activation) ? R / 2 : R) * (NW / WK);
             k.group = m.blocks > 1 ? slot : 0u;
             k.row0 = 0;
@@ -166,11 +165,13 @@ __global__ void __launch_bounds__(32 * LS_WARPS, OCC) linear_stream_kernel(const
         };
 #pragma unroll
         for (int d = 0; d < XD; d++) { load_x(d, wk + d * WK); }
-        // what the results are added to, fetched while the products are made
+        // What the results are added to, fetched while the products are made; not in the forms of gated launches, which have no register
+        // left and as good as never add.
+        constexpr bool EARLY = RT == 1 || NT == 4;
         const unsigned int cols = min((unsigned int)C, k.count - k.n0);
         const unsigned int F = gated ? R / 2 : R, all = F * (NW / WK);    // output features of a warp, of the CTA
         float old = 0.f;
-        const bool adds = m.accumulate != 0 && threadIdx.x < cols * all && k.fc + threadIdx.x % all < m.N;
+        const bool adds = EARLY && m.accumulate != 0 && threadIdx.x < cols * all && k.fc + threadIdx.x % all < m.N;
         if (adds) { old = ((const float*)m.Y)[(size_t)(k.row0 + k.n0 + threadIdx.x / all) * m.ldy + ycol + k.fc + threadIdx.x % all]; }
         // the task after this one
         StreamTask nk = k;
@@ -355,37 +356,75 @@ static int launch_stream_wk(LinearLaunch& L, unsigned int sm_count, unsigned int
     return launch_kernel("linear_stream", linear_stream_kernel<NT, RT, U, WK, OCC>, dim3(grid), dim3(32 * LS_WARPS), 0, st, pdl, L);
 }
 
-// Which form a launch takes (one linear in a CUDA graph of distinct weights, microseconds at 8 / 16 / 32 rows):
-//   * CTAs that take task after task, or one for each task?  Taking the next task hides its first loads behind this one's sums, a CTA
-//     of its own fits itself to what an SM gets done.  Up to 8 rows dense tasks gain nothing (5120 x 2048: 7.3 either way, at 1 row
-//     7.3 against 6.0; 32768 x 2048: 28.4 against 25.1), gated ones up to four rounds do (6144 x 2048: 11.1 against 12.0; 12288 x 4096
-//     either way 33.4); more rows do at any number (32768 x 2048: 28.7 / 45.8 against 30.1 / 51.3).
-//   * Chunks in flight: a whole k of 2048 (four per warp) up to 8 rows, two where k is longer (4096 x 12288: 20.5 with four, 18.1;
-//     151936 x 4096: 218 with four, 202.5) and up to 16 rows, where registers are short (4096 x 4096: 9.7, 8.0).
-//   * One CTA per SM with twice the chunks in flight where the tasks are fewer than the SMs and k is long: 2048 x 6144 9.5, 6.2.
-template <int NT, int RT, int U>
+// Which form a launch takes (one linear in a CUDA graph of distinct weights, us; "few": a launch has no more tasks than there are SMs).
+//   * Two warps over k up to 1024, eight beyond: the bits follow this alone.
+//   * Few tasks: one CTA per SM with twice the chunks in flight, or four times (8 rows, one CTA / two: 2048 x 768 2.8 / 3.9, 8192 x 1024 4.8 / 5.9, gated 4096 x 512
+//     3.4 / 4.4, 2048 x 6144 6.3 / 7.2; 16 rows: 8192 x 1024 7.0 / 7.6, gated 1024 x 4096 8.4 / 10.8).  Not where k is short enough to be under way whole with two: 512 x
+//     8192 at 8 rows 3.4 / 3.3.
+//   * More tasks, up to 8 rows, two warps over k: four chunks where a warp's chunks are whole fours, else two (32768 x 1024 14.3 / 14.9, 32768 x 768 12.0 / 11.8, the
+//     down projections of 16 experts, k 768, 13.0 / 12.0).  Eight warps: a whole k of 2048 (four per warp), two chunks where k is longer (4096 x 12288 20.5 with
+//     four, 18.1; 151936 x 4096 218, 202.5).
+//   * CTAs that take task after task (up to so many rounds), or one for each task?  Taking the next task hides its first loads behind this one's sums, a CTA of its own
+//     fits itself to what an SM gets done.  Up to 8 rows two warps over k gain in the second round (32768 x 1024: 14.0 against 14.8) and lose beyond (experts, 1024
+//     tasks, k 1024: 26.1 against 24.8), dense tasks of eight warps gain nothing (5120 x 2048 at 1 row 7.3 against 6.0; 32768 x 2048 28.4 against 25.1), gated ones of eight
+//     warps do up to four rounds (6144 x 2048 11.1 against 12.0), of two warps they lose (64 experts of 512, k 1024, at 32 tokens: 28.4 against 24.3).  More rows gain
+//     at any number (32768 x 2048: 28.7 / 45.8 at 16 / 32 rows against 30.1 / 51.3).
+//   * Registers: gated 9 to 16 rows hold one chunk on two CTAs per SM (two chunks spill: 12288 x 4096 at 9 / 16 rows 39.4 / 40.1 with one, 42.2 / 43.1 with two); 17 to 32 rows of
+//     two warps that are not gated hold 16 features a warp on two CTAs (32 features on one: 32768 x 1024 at 32 rows 24.8 / 29.1, 2048 x 512, few, 6.0 / 10.2).
+template <int NT, int RT>
 static int launch_stream(LinearLaunch& L, cudaStream_t st, bool pdl)
 {
     const DecoderDevice* dev = decoder_device();
     if (!dev) { return 1; }
-    const unsigned int sms = (unsigned int)dev->sm_count, waves = NT > 1 ? 0xFFFFFFFFu : RT == 2 ? 4u : 1u;
-    unsigned int longest = 0, blocks = 0;
+    constexpr unsigned int EVERY = 0xFFFFFFFFu;
+    const unsigned int sms = (unsigned int)dev->sm_count;
+    unsigned int longest = 0;
+    for (unsigned int j = 0; j < L.count; j++) { longest = L.m[j].K > longest ? L.m[j].K : longest; }
+    // eight warps over few chunks would leave some without any; the members of a launch take one form
+    const bool two = longest <= 1024;
+    if constexpr (NT == 4 && RT == 1)
+    {
+        if (!two) { return launch_stream<4, 2>(L, st, pdl); }
+    }
+    unsigned int tasks = 0;
     for (unsigned int j = 0; j < L.count; j++)
     {
         const LinearMember& m = L.m[j];
-        longest = m.K > longest ? m.K : longest;
-        const unsigned int F = activation_gated(m.activation) ? 8 * RT : 16 * RT;
-        blocks += (m.N + F - 1) / F * m.slots;
+        const unsigned int F = (activation_gated(m.activation) ? 8 * RT : 16 * RT) * (two ? LS_WARPS / 2 : 1);
+        tasks += (m.N + F - 1) / F * m.slots;
     }
-    // eight warps over few chunks would leave some without any; the members of a launch take one form
-    constexpr int OCC = NT == 4 ? 1 : 2;
-    if (longest <= 1024) { return launch_stream_wk<NT, RT, U, 2, OCC>(L, sms, waves, st, pdl); }
-    if constexpr (NT == 1)
+    const bool few = tasks <= sms;
+    if constexpr (NT == 1 && RT == 1)
     {
-        if (blocks <= sms && longest >= 4096) { return launch_stream_wk<NT, RT, 2 * U, 8, 1>(L, sms, waves, st, pdl); }
-        if (RT == 1 && longest > 2048) { return launch_stream_wk<NT, RT, 2, 8, OCC>(L, sms, waves, st, pdl); }
+        if (two)
+        {
+            const unsigned int own = ((longest + 63) / 64 + 1) / 2;    // chunks of a warp
+            if (few && own > 4) { return launch_stream_wk<1, 1, 8, 2, 1>(L, sms, 1, st, pdl); }
+            return own <= 4 || own % 4 == 0 ? launch_stream_wk<1, 1, 4, 2, 2>(L, sms, 2, st, pdl) : launch_stream_wk<1, 1, 2, 2, 2>(L, sms, 2, st, pdl);
+        }
+        if (few && longest >= 4096) { return launch_stream_wk<1, 1, 8, 8, 1>(L, sms, 1, st, pdl); }
+        return longest > 2048 ? launch_stream_wk<1, 1, 2, 8, 2>(L, sms, 1, st, pdl) : launch_stream_wk<1, 1, 4, 8, 2>(L, sms, 1, st, pdl);
     }
-    return launch_stream_wk<NT, RT, U, 8, OCC>(L, sms, waves, st, pdl);
+    else if constexpr (NT == 1)
+    {
+        if (two) { return few ? launch_stream_wk<1, 2, 4, 2, 1>(L, sms, 1, st, pdl) : launch_stream_wk<1, 2, 2, 2, 2>(L, sms, 1, st, pdl); }
+        return few && longest >= 4096 ? launch_stream_wk<1, 2, 4, 8, 1>(L, sms, 1, st, pdl) : launch_stream_wk<1, 2, 2, 8, 2>(L, sms, 4, st, pdl);
+    }
+    else if constexpr (NT == 2 && RT == 1)
+    {
+        if (two && few) { return launch_stream_wk<2, 1, 4, 2, 1>(L, sms, EVERY, st, pdl); }
+        return two ? launch_stream_wk<2, 1, 2, 2, 2>(L, sms, EVERY, st, pdl) : launch_stream_wk<2, 1, 2, 8, 2>(L, sms, EVERY, st, pdl);
+    }
+    else if constexpr (NT == 2)
+    {
+        if (few) { return two ? launch_stream_wk<2, 2, 4, 2, 1>(L, sms, EVERY, st, pdl) : launch_stream_wk<2, 2, 4, 8, 1>(L, sms, EVERY, st, pdl); }
+        return two ? launch_stream_wk<2, 2, 1, 2, 2>(L, sms, EVERY, st, pdl) : launch_stream_wk<2, 2, 1, 8, 2>(L, sms, EVERY, st, pdl);
+    }
+    else if constexpr (RT == 1)
+    {
+        return few ? launch_stream_wk<4, 1, 4, 2, 1>(L, sms, EVERY, st, pdl) : launch_stream_wk<4, 1, 2, 2, 2>(L, sms, EVERY, st, pdl);
+    }
+    else { return two ? launch_stream_wk<4, 2, 2, 2, 1>(L, sms, EVERY, st, pdl) : launch_stream_wk<4, 2, 2, 8, 1>(L, sms, EVERY, st, pdl); }
 }
 
 }    // namespace b200
@@ -498,9 +537,9 @@ C_EXPORT int cuda_b200_linear_rows(int dtype, unsigned int count, const cuda_b20
             }
             if (part.count == 0) { continue; }
             int rc;
-            if (width == 8) { rc = gated ? launch_stream<1, 2, 2>(part, st, pdl) : launch_stream<1, 1, 4>(part, st, pdl); }
-            else if (width == 16) { rc = gated ? launch_stream<2, 2, 2>(part, st, pdl) : launch_stream<2, 1, 2>(part, st, pdl); }
-            else { rc = launch_stream<4, 2, 2>(part, st, pdl); }
+            if (width == 8) { rc = gated ? launch_stream<1, 2>(part, st, pdl) : launch_stream<1, 1>(part, st, pdl); }
+            else if (width == 16) { rc = gated ? launch_stream<2, 2>(part, st, pdl) : launch_stream<2, 1>(part, st, pdl); }
+            else { rc = gated ? launch_stream<4, 2>(part, st, pdl) : launch_stream<4, 1>(part, st, pdl); }
             if (rc) { return rc; }
         }
         return 0;

@@ -265,6 +265,39 @@ def test_streaming_tasks_one_behind_the_other(D, rows, members):
         assert np.all(host(Y)[:, N:] == -3.0)
 
 
+@pytest.mark.parametrize("rows", [1, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("act", [0, 2])
+@pytest.mark.parametrize("K", [200, 512, 640, 768, 1024, 1100, 2048, 4160])
+def test_a_features_bits_follow_the_warps_over_k_alone(D, rows, act, K):
+    """Fewer tasks than SMs, more, and more than the GPU holds at once; all rows as the rows of one group: another form each, the same bits."""
+    import torch
+
+    Ns = (40, 9500, 20000) if K <= 1024 else (40, 2400, 5000)
+    most, first, ld = Ns[-1], Ns[0], pad64(K)
+    g = torch.Generator(device="cuda").manual_seed(K + rows)
+    W = torch.zeros(2 * most, ld, dtype=torch.bfloat16, device="cuda")
+    W[:, :K] = torch.randn(2 * most, K, device="cuda", generator=g) * K ** -0.5
+    X = torch.zeros(rows, ld, dtype=torch.bfloat16, device="cuda")
+    X[:, :K] = torch.randn(rows, K, device="cuda", generator=g)
+    offset, active = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([0, rows], [0]))
+
+    def linear(N, **group):
+        Y = torch.zeros(rows, N, device="cuda")
+        a = D.fill(D.Linear, W=W, X=X, Y=Y, rows=rows, N=N, K=K, ldw=ld, ldx=ld, ldy=N, up_row=most, activation=act, accumulate=1, alpha=1.0, **group)
+        assert D.linear(BF16, [a], kernel=1) == 0 and D.check() == 0
+        return Y
+
+    z = X.double() @ W.double().T
+    want = (torch.nn.functional.silu(z[:, :most]) * z[:, most:] if act == 2 else z[:, :most]).cpu().numpy()
+    alone = linear(first)
+    for N in Ns:
+        Y = linear(N)
+        # a warp's products of 16 k add up one behind the other: at most K / 16 / 2 (or 8) roundings of 2^-23
+        close(host(Y), want[:, :N], FLOAT, N, 10 + K / 16 / (2 if K <= 1024 else 8) * 2 ** -23 / TOL[FLOAT])
+        assert torch.equal(Y[:, :first], alone), N
+    assert torch.equal(linear(first, group_offset=offset, active=active, groups=1, group_rows=2 * most, group_max=rows, active_cap=1), alone)
+
+
 def test_descriptors_that_are_not_taken(D):
     X = padded(np.ones((2, 64)), BF16)
     base = dict(W=X, X=X, Y=X, rows=2, N=2, K=64, ldw=64, ldx=64, ldy=64, alpha=1.0)
