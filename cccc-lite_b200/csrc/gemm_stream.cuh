@@ -465,6 +465,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
             constexpr unsigned int STEP = FOURS ? 1 : 32;
             const unsigned int n = n0 + (FOURS ? 4 * lane : lane);
             const bool whole = FOURS && aligned && n + 4 <= g.N;
+            if (n >= g.N) { return; }
             const long long yi = (long long)(m0 + t) * g.ldy_m + (long long)n * g.ldy_n;
             float old[4] = { 0.f, 0.f, 0.f, 0.f }, o[4];
             if (g.beta != 0.f)
