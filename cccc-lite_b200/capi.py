@@ -8,7 +8,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from .torch_stream import current_stream
+from .torch_stream import raw_stream as _stream
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libcccc-cuda-b200.so")
@@ -309,10 +309,6 @@ class FusedRowLinear:
                                                  K if ldw is None else ldw, K if ldx is None else ldx,
                                                  N if ldy_m is None else ldy_m, ldy_n, alpha, self.recv_ptrs, self.flag_ptrs,
                                                  _ptr(self.counters), self.n_max, self.rank, self.world, stream, flags)
-
-
-def _stream(stream):
-    return current_stream() if stream is None else stream
 
 
 def rms_norm_bf16(X, Y, scale, rows: int, inner: int, eps: float = 1e-6, residual=None, sum_out=None, stream=None, flags: int = 0) -> int:

@@ -5,7 +5,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from .torch_stream import current_stream
+from .torch_stream import raw_stream
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libcccc-b200-decoder.so")
@@ -93,19 +93,19 @@ def fill(cls, **kw):
 
 
 def embed(dtype, ids, table, ld_table, X, ldx, n, width, vocab, scale, flags=0):
-    return lib().cuda_b200_embed_f32(dtype, _ptr(ids), _ptr(table), ld_table, _ptr(X), ldx, n, width, vocab, scale, current_stream(), flags)
+    return lib().cuda_b200_embed_f32(dtype, _ptr(ids), _ptr(table), ld_table, _ptr(X), ldx, n, width, vocab, scale, raw_stream(), flags)
 
 
 def norm(dtype, desc, flags=0):
-    return lib().cuda_b200_norm_rows(dtype, C.byref(desc), current_stream(), flags)
+    return lib().cuda_b200_norm_rows(dtype, C.byref(desc), raw_stream(), flags)
 
 
 def linear(dtype, descs, flags=0, kernel=0):
-    return lib().cuda_b200_linear_rows(dtype, len(descs), (Linear * len(descs))(*descs), current_stream(), flags, kernel)
+    return lib().cuda_b200_linear_rows(dtype, len(descs), (Linear * len(descs))(*descs), raw_stream(), flags, kernel)
 
 
 def attention(dtype, desc, batch, flags=0, kernel=0):
-    return lib().cuda_b200_attention_rows(dtype, C.byref(desc), C.byref(batch), current_stream(), flags, kernel)
+    return lib().cuda_b200_attention_rows(dtype, C.byref(desc), C.byref(batch), raw_stream(), flags, kernel)
 
 
 def attention_work_bytes(vdim):
@@ -113,20 +113,20 @@ def attention_work_bytes(vdim):
 
 
 def rotary_table(table, rows, dims, base):
-    return lib().cuda_b200_rotary_table(_ptr(table), rows, dims, base, current_stream())
+    return lib().cuda_b200_rotary_table(_ptr(table), rows, dims, base, raw_stream())
 
 
 def latent_down(dtype, desc, batch, flags=0):
-    return lib().cuda_b200_latent_down(dtype, C.byref(desc), C.byref(batch), current_stream(), flags)
+    return lib().cuda_b200_latent_down(dtype, C.byref(desc), C.byref(batch), raw_stream(), flags)
 
 
 def latent_query(dtype, src, ld_src, src_step, src_off, dst, ld_dst, dst_step, dst_off, heads, rot_dim, rotary, T_max, batch, flags=0):
     return lib().cuda_b200_latent_query(dtype, _ptr(src), ld_src, src_step, src_off, _ptr(dst), ld_dst, dst_step, dst_off, heads, rot_dim, _ptr(rotary), T_max,
-                                        C.byref(batch), current_stream(), flags)
+                                        C.byref(batch), raw_stream(), flags)
 
 
 def latent_expand(dtype, desc, batch, flags=0):
-    return lib().cuda_b200_latent_expand(dtype, C.byref(desc), C.byref(batch), current_stream(), flags)
+    return lib().cuda_b200_latent_expand(dtype, C.byref(desc), C.byref(batch), raw_stream(), flags)
 
 
 def mlstm_state_floats(dim, vdim):
@@ -138,19 +138,19 @@ def mlstm_work_floats(tokens, entries, heads, dim, vdim):
 
 
 def mlstm(dtype, desc, batch, flags=0, kernel=0):
-    return lib().cuda_b200_mlstm_rows(dtype, C.byref(desc), C.byref(batch), current_stream(), flags, kernel)
+    return lib().cuda_b200_mlstm_rows(dtype, C.byref(desc), C.byref(batch), raw_stream(), flags, kernel)
 
 
 def route(desc, flags=0):
-    return lib().cuda_b200_route_rows(C.byref(desc), current_stream(), flags)
+    return lib().cuda_b200_route_rows(C.byref(desc), raw_stream(), flags)
 
 
 def gather(dtype, X, ldx, row_token, out, ldo, n, width, flags=0):
-    return lib().cuda_b200_gather_rows(dtype, _ptr(X), ldx, _ptr(row_token), _ptr(out), ldo, n, width, current_stream(), flags)
+    return lib().cuda_b200_gather_rows(dtype, _ptr(X), ldx, _ptr(row_token), _ptr(out), ldo, n, width, raw_stream(), flags)
 
 
 def argmax(logits, rows, cols, ld, idx, val, flags=0):
-    return lib().cuda_b200_argmax_f32(_ptr(logits), rows, cols, ld, _ptr(idx), _ptr(val), current_stream(), flags)
+    return lib().cuda_b200_argmax_f32(_ptr(logits), rows, cols, ld, _ptr(idx), _ptr(val), raw_stream(), flags)
 
 
 def check(label="decoder"):

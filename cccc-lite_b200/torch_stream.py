@@ -1,10 +1,12 @@
-"""The stream that a call from Python goes to where none is given: torch's current one."""
+"""The stream that a call from Python goes to."""
 from __future__ import annotations
 
 
-def current_stream() -> int:
-    """torch's current stream as a raw cudaStream_t.  Asked for directly where torch has been initialised and has the two calls that its
-    own stream object is made of: that object takes 3.2 us, a third of a call."""
+def raw_stream(stream=None):
+    """The raw cudaStream_t: the given one, or torch's current one for None.  That is asked for directly where torch has been initialised and has the two
+    calls that its own stream object is made of: the object takes 3.2 us, a third of a call."""
+    if stream is not None:
+        return stream
     import torch
 
     if torch.cuda.is_initialized():

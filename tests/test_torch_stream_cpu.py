@@ -8,7 +8,7 @@ from __graft_entry__ import load_package
 
 @pytest.mark.parametrize("missing", [(), ("_cuda_getCurrentRawStream",), ("_cuda_getDevice",)])
 @pytest.mark.parametrize("initialised", [False, True])
-def test_current_stream(monkeypatch, missing, initialised):
+def test_the_stream_of_a_call_without_one(monkeypatch, missing, initialised):
     import torch
 
     load_package()
@@ -20,6 +20,6 @@ def test_current_stream(monkeypatch, missing, initialised):
     for name in missing:
         monkeypatch.delattr(torch._C, name)
     want = 1003 if initialised and not missing else 77
-    assert sys.modules[pkg + "torch_stream"].current_stream() == want
+    assert sys.modules[pkg + "torch_stream"].raw_stream() == want
     capi = sys.modules[pkg + "capi"]
     assert capi._stream(None) == want and capi._stream(0) == 0 and capi._stream(5) == 5
