@@ -40,8 +40,8 @@ static inline bool w8a8_split_early(unsigned int M, unsigned int K) { return M >
 // the four calls of a Qwen3-8B layer 80.4 / 79.3, 81.4 / 79.9, 84.5 / 80.9, 88.5 / 85.0, of a Llama-3.1-8B layer 83.2 / 81.5, 85.2 / 83.5, 87.9 / 84.4, 92.1 / 89.0.
 // Above 128 tokens 4096 features gain (20.8 / 17.8 at 256) less than q, k and v together lose (19.3 / 21.6 at 200), and at K = 2048 the pairs are ahead (4096
 // features at 128 11.8 / 13.5).  A single tile keeps the pairs, which the tests hold; no layer has one beside a wider member but for a single kv head of 128.
-// A feature's bits are the same in every matrix that takes the same kernel: on this line's side, up to 128 tokens, in all of 129 to 8448 features with K from 4096 to
-// 8191 and of up to 20480 with K from 8192 (the tests hold both); with K below 4096, and from 24 to 64 tokens, in all.
+// A feature's bits are the same in every matrix that takes the same kernel: from 24 to 64 tokens in all; to 128 tokens in all of 129 to 8448 features with K from 4096 to
+// 8191 and of up to 20480 with K from 8192 (the tests hold both); to 256 in all of up to 4224 with K from 8192; otherwise (K below 4096, or more tokens) in all.
 static inline bool w8a8_split_preferred(unsigned int M, unsigned int K, unsigned int N, int sm_count)
 {
     if (M <= 64) { return true; }
