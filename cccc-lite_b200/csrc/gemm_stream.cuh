@@ -454,8 +454,9 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
     // token, of which an SM gets one done in 25 ns: a tile of 32 / 100 tokens spent 3.3 / 9.2 us here, now 1.3 / 2.6; E4M3 24576 x 4096 at 32 / 64 /
     // 128 tokens 32.9 / 37.4 / 47.8 -> 31.5 / 33.1 / 37.7 us, 6144 x 4096 11.2 / 13.3 / 17.7 -> 10.5 / 11.6 / 14.3.)  Elsewhere a lane has every 32nd
     // feature, so that the accesses of a warp, one element each, lie side by side (32767 features at 64 / 128 tokens, four side by side / every 32nd:
-    // 35.8 / 34.7, 42.0 / 40.1 us, with an old Y 39.9 / 37.9, 50.5 / 46.1) - but not with eight slices, where reading the others' tiles one element at a time
-    // costs more than it saves (4097 features at 64 tokens 10.6 / 11.2).
+    // 35.7 / 34.5, 41.5 / 39.4 us, with an old Y 39.7 / 37.4, 49.4 / 45.3; with eight slices, whose tiles are then read one element at a time, 4097 features
+    // 10.6 / 11.0, 14.7 / 15.0, 11.4 / 11.1, 14.8 / 14.7).  In the host's memory, where the head of a decode step writes, pieces of two bytes in eight take a bus
+    // transaction each: 32767 features at 16 tokens, call to end, 392 / 56 us, 4097 with eight slices 65 / 27, 151935 1683 / 179.
     if (warp < SK_DQ_WARPS && *abort_flag == 0)
     {
         const unsigned int y_size = p.out_f32 == 1u ? 4u : 2u;
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
             constexpr bool FOURS = decltype(fours)::value;
             constexpr unsigned int STEP = FOURS ? 1 : 32;
             const unsigned int n = n0 + (FOURS ? 4 * lane : lane);
-            const bool whole = FOURS && aligned && n + 4 <= g.N;
+            const bool whole = FOURS && n + 4 <= g.N;
             if (n >= g.N) { return; }
             const long long yi = (long long)(m0 + t) * g.ldy_m + (long long)n * g.ldy_n;
             float old[4] = { 0.f, 0.f, 0.f, 0.f }, o[4];
@@ -541,10 +542,10 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_wq_stream_kernel(const __g
         auto add_slices = [&](auto fours) {
             if (S == 1) { add(std::integral_constant<int, 1>(), fours); }
             else if (S == 2) { add(std::integral_constant<int, 2>(), fours); }
-            else { add(std::integral_constant<int, 4>(), fours); }
+            else if (S == 4) { add(std::integral_constant<int, 4>(), fours); }
+            else { add(std::integral_constant<int, 8>(), fours); }
         };
-        if (S > 4) { add(std::integral_constant<int, 8>(), std::true_type{}); }
-        else if (aligned) { add_slices(std::true_type{}); }
+        if (aligned) { add_slices(std::true_type{}); }
         else { add_slices(std::false_type{}); }
     }
     // nobody leaves while a peer may still read its partial tile
